@@ -99,7 +99,7 @@ void free_all(Handle& h) {
   void* ptrs[] = {m.own, m.nei, m.Sf, m.magSf, m.w, m.nodc, m.dOwn, m.dNei, m.dCC, m.nf, m.bnf, m.C, m.V,
                   m.bcell, m.bpatch, m.bSf, m.bmagSf, m.bdOwn, m.bdc, m.patches, m.cptr, m.cface, m.bptr,
                   m.bface, m.slot_base, m.scol, m.sface, m.nlow, m.nslot, m.fl_cells, m.rl_cells, m.fl_lptr,
-                  m.rl_lptr, m.sweep_pad, m.sweep_ticket, h.W, h.W0, h.W00, h.Wprev, h.prim, h.pB, h.TB, h.UB, h.phiB, h.pseudoCo, h.rPDT,
+                  m.rl_lptr, m.sweep_pad, m.sweep_ticket, m.sw_fwd, m.sw_rev, h.W, h.W0, h.W00, h.Wprev, h.prim, h.pB, h.TB, h.UB, h.phiB, h.pseudoCo, h.rPDT,
                   h.ddtCoeff, h.q, h.bq, h.clin, h.grad, h.fflux, h.frec, h.flam, h.bjac, h.src, h.vcell,
                   h.fvisc, h.vsf2, h.vjac, m.dc, m.Dhb, m.mrfU, m.mrfOm, m.mrfBU, m.mrfBIn, m.plagMode, m.plagP, m.bpartner, m.bw, m.bdelta, m.bdNei,
                   m.bnodc, m.cyc_face, m.cyc_row, m.cyc_ptr, h.cblk, h.vjslotbuf, h.vjcellbuf, h.cfrec, h.tW, h.tprim, h.tq, h.tgrad, h.tflux, h.tvc, h.tfv, h.tv,
@@ -216,6 +216,17 @@ void ensure_workspace(Handle& h) {
     h.kv = dalloc<char>(kstride(h) * eb * m);
     h.kvDirs = m;
   }
+}
+
+// rows in level order with every level padded to whole sweep tickets (-1), so
+// that the rows of one ticket never depend on one another
+std::vector<int> ticket_order(const std::vector<int>& cells, const std::vector<int>& ptr) {
+  std::vector<int> out;
+  for (size_t l = 0; l + 1 < ptr.size(); ++l) {
+    out.insert(out.end(), cells.begin() + ptr[l], cells.begin() + ptr[l + 1]);
+    while (out.size() % SWEEP_TICKET) out.push_back(-1);
+  }
+  return out;
 }
 
 void build_mesh(Handle& h, const ics_mesh_desc* d) {
@@ -458,8 +469,18 @@ void build_mesh(Handle& h, const ics_mesh_desc* d) {
   m.fl_cells = upload(fcells);
   m.rl_cells = upload(rcells);
   m.fl_lptr = upload(m.fl_ptr);
-  // outputs of the sync-free sweeps (the schedules with many levels only)
-  if (m.nfl > 2 && (long)N >= 2048L * m.nfl) m.sweep_pad = dalloc<double>(16ull * N);
+  // the sync-free sweeps: every schedule of more than two levels.  Measured
+  // against one CTA that walks the levels (us per forward sweep, FP64 / FP32):
+  // 12^3 RCM box 48 / 47 against 176 / 58, 24^3 97 / 96 against 556 / 131,
+  // 61^3 276 / 268 against 7069 / 1010.
+  if (m.nfl > 2) {
+    m.sweep_pad = dalloc<double>(16ull * N);
+    const std::vector<int> sf = ticket_order(fcells, m.fl_ptr), sr = ticket_order(rcells, m.rl_ptr);
+    m.nsw_fwd = (int)(sf.size() / SWEEP_TICKET);
+    m.nsw_rev = (int)(sr.size() / SWEEP_TICKET);
+    m.sw_fwd = upload(sf);
+    m.sw_rev = upload(sr);
+  }
   m.sweep_ticket = dalloc<unsigned int>(2);
   m.rl_lptr = upload(m.rl_ptr);
 }
@@ -1254,14 +1275,17 @@ int ics_test_sweep_timeout(ics_handle hh, int32_t skip_row, int32_t spin_limit) 
     }
     if (skip_row < 0 || skip_row >= N) return ICS_ERR_ARG;
     if (!h.m.sweep_pad) h.m.sweep_pad = dalloc<double>(16ull * N);  // schedules with few levels
-    // the forward level order without skip_row
-    std::vector<int> order(N);
-    ICS_CUDA(cudaMemcpy(order.data(), h.m.fl_cells, N * sizeof(int), cudaMemcpyDeviceToHost));
-    order.erase(std::remove(order.begin(), order.end(), (int)skip_row), order.end());
-    if ((int)order.size() != N - 1) return ICS_ERR_ARG;
-    ICS_CUDA(cudaMemcpy(h.ibuf, order.data(), (N - 1) * sizeof(int), cudaMemcpyHostToDevice));
+    // the forward tickets with skip_row left out
+    std::vector<int> cells(N);
+    ICS_CUDA(cudaMemcpy(cells.data(), h.m.fl_cells, N * sizeof(int), cudaMemcpyDeviceToHost));
+    std::vector<int> order = ticket_order(cells, h.m.fl_ptr);
+    for (int& c : order)
+      if (c == skip_row) c = -1;
+    int* dev = upload(order);
     ICS_CUDA(cudaMemsetAsync(&h.ks->status, 0, sizeof(int), h.stream));
-    sweep_probe(h, h.ibuf, N - 1, spin_limit);
+    sweep_probe(h, dev, (int)(order.size() / SWEEP_TICKET), spin_limit);
+    ICS_CUDA(cudaStreamSynchronize(h.stream));
+    ICS_CUDA(cudaFree(dev));
     int st = 0;
     ICS_CUDA(cudaMemcpyAsync(&st, &h.ks->status, sizeof(int), cudaMemcpyDeviceToHost, h.stream));
     ICS_CUDA(cudaStreamSynchronize(h.stream));

@@ -36,6 +36,7 @@ constexpr double VGREAT = 1e300;
 enum { Q_RHO = 0, Q_P = 1, Q_UX = 2, Q_UY = 3, Q_UZ = 4, Q_E = 5, Q_H = 6, Q_C = 7, NQ = 8 };
 
 constexpr int SLICE = 32;
+constexpr int SWEEP_TICKET = 32;  // rows per ticket of the sync-free LU-SGS sweeps
 constexpr int REDUCE_BLOCKS = 1216;  // 8 x 152 SMs
 constexpr int MAX_DIRS = 64;
 constexpr int MAX_INST = ICS_MAX_INSTANCES;  // Harmonic Balance instances
@@ -106,6 +107,11 @@ struct DevMesh {
   int* rl_lptr = nullptr;
   void* sweep_pad = nullptr;         // [2][8N] FP64-sized outputs of the sync-free sweeps
   unsigned int* sweep_ticket = nullptr;  // [2] row tickets of the sync-free sweeps
+  // rows of the sync-free sweeps in level order, every level padded with -1
+  // to whole tickets of 32 rows (nullptr: other schedules)
+  int* sw_fwd = nullptr;
+  int* sw_rev = nullptr;
+  int nsw_fwd = 0, nsw_rev = 0;      // tickets
   bool fuse_last = false;            // last forward level == first reverse level (same rows)
   // Harmonic Balance: nInst stacked instances of Nc cells (instance-major),
   // coupled through the spectral operator Dhb [nInst][nInst]
@@ -450,7 +456,7 @@ void autotune_residual(Handle& h, std::vector<std::pair<std::string, double>>& l
 // fields with a reconstruction gradient (bit k = q field k) and the MUSCL limiter kind
 unsigned grad_mask(const Handle& h, int* limited);
 void to_vec(Handle& h, const double* src, void* dst);   // FP64 -> Krylov type
-void sweep_probe(Handle& h, const int* order, int count, int spin_limit);
+void sweep_probe(Handle& h, const int* order, int tickets, int spin_limit);
 void from_vec(Handle& h, const void* src, double* dst); // Krylov type -> FP64
 
 inline int prec(const Handle& h) { return h.cfg.c.precision; }

@@ -530,50 +530,32 @@ __global__ void __launch_bounds__(128) k_lusgs_level(DevMesh m, const TB* __rest
     lusgs_fwd_row<TB, TV, true>(m, blk, rD, r, c);
 }
 
-// one CTA walks every level (small meshes / many tiny levels)
-template <typename TB, typename TV, bool FWD>
-__global__ void __launch_bounds__(1024) k_lusgs_block(DevMesh m, const TB* __restrict__ blk,
-                                                      const TB* __restrict__ rD, TV* __restrict__ r,
-                                                      const int* __restrict__ cells, const int* __restrict__ lptr,
-                                                      int nlev) {
-  for (int l = 0; l < nlev; ++l) {
-    const int a = lptr[l], b = lptr[l + 1];
-    for (int i = a + threadIdx.x; i < b; i += blockDim.x) {
-      const int c = cells[i];
-      if (FWD)
-        lusgs_fwd_row<TB, TV>(m, blk, rD, r, c);
-      else
-        lusgs_rev_row<TB, TV>(m, blk, rD, r, c);
-    }
-    __syncthreads();
-  }
-}
-
 // ----------------------------------------------- sync-free LU-SGS sweeps
 // One launch per sweep for schedules with many levels (RCM / natural
-// numbering): blocks draw consecutive tickets in level order (order[]), so a
-// row only ever waits for rows with smaller tickets, whose blocks started
-// earlier and are resident or done -- no deadlock.  The sweep writes its rows
-// into a padded output array (8 words per row, 32 B for FP32) that starts
-// filled with a sentinel (all bits set: a NaN with the sign bit, which GPU
-// arithmetic does not produce from finite operands -- a result that matched
-// it, from a NaN already in the input, would make its dependents give up
-// at the bound and report, never hang), and a row's result
-// words are their own done flags: a row polls its neighbours' five words
-// with relaxed loads until none is the sentinel.  One L2 round trip per
-// poll brings both the readiness and the values, the writer needs no fence,
-// and the polls of all prefetched neighbours are issued together.  The
-// arithmetic per row is that of lusgs_fwd_row / lusgs_rev_row, so the result
-// equals the level-by-level sweep bit for bit.  A wait that exceeds the
-// bound sets status bit 8, publishes zeros (so that its dependents do not
-// wait in turn) and returns; waiting rows that see bit 8 give up too (the
-// host reports ICS_ERR_TIMEOUT).
+// numbering).  A resident set of warps draws consecutive tickets; ticket t
+// holds rows order[32 t .. 32 t + 31], the levels one after the other and
+// each padded to whole tickets (-1), so a row only ever waits for rows of
+// smaller tickets -- drawn earlier by warps that are resident or done and
+// that never wait for a later one -- and never for a lane of its own warp:
+// no deadlock.  The sweep writes its rows into a padded output array (8 words
+// per row, 32 B for FP32) that starts filled with a sentinel (all bits set: a
+// NaN with the sign bit, which GPU arithmetic does not produce from finite
+// operands and which a row never publishes),
+// and a row's result words are their own done flags: a row polls its
+// neighbours' five words with relaxed loads until none is the sentinel.  One
+// L2 round trip per poll brings both the readiness and the values, the writer
+// needs no fence, and the polls of all prefetched neighbours are issued
+// together.  The arithmetic per row is that of lusgs_fwd_row / lusgs_rev_row,
+// so the result equals the level-by-level sweep bit for bit.  A wait that
+// exceeds the bound sets status bit 8, publishes zeros (so that its
+// dependents do not wait in turn) and goes on; waiting rows that see bit 8
+// give up too (the host reports ICS_ERR_TIMEOUT).
 constexpr int SWEEP_SPIN_LIMIT = 1 << 22;
 constexpr int SWEEP_PAD = 8;  // words per row of the sweep outputs
-// rows per block: a level's rows are consecutive tickets, so small blocks
-// spread each level over more SMs (FP64 sweeps 4% faster than with 128-row
-// blocks on a 285-level RCM box; FP32 unchanged)
-constexpr int SWEEP_THREADS = 32;
+constexpr int SWEEP_THREADS = 32;  // one warp per block
+// rows a warp takes at once (sweep_row16 / sweep_row)
+template <typename TB, typename TV>
+constexpr int sweep_rows = sizeof(TB) == 8 && sizeof(TV) == 8 ? 2 : SWEEP_TICKET;
 
 __device__ __forceinline__ int ld_relaxed_int(const int* p) {
   int v;
@@ -607,26 +589,120 @@ __device__ __forceinline__ bool sweep_word_set(float v) { return __float_as_uint
 __device__ __forceinline__ bool sweep_word_set(double v) {
   return (unsigned long long)__double_as_longlong(v) != ~0ull;
 }
+// a result that is the sentinel itself (a NaN of that payload in the input)
+// is published as the canonical NaN, so that its dependents do not wait
+__device__ __forceinline__ float sweep_word(float v) { return sweep_word_set(v) ? v : __uint_as_float(0x7fffffffu); }
+__device__ __forceinline__ double sweep_word(double v) {
+  return sweep_word_set(v) ? v : __longlong_as_double(0x7fffffffffffffffLL);
+}
 template <typename TV>
 __device__ __forceinline__ bool sweep_ready(const TV* v) {
   return sweep_word_set(v[0]) && sweep_word_set(v[1]) && sweep_word_set(v[2]) && sweep_word_set(v[3]) &&
          sweep_word_set(v[4]);
 }
 
+// FP64 rows, 16 lanes each (two rows per warp): lane (p, i) = (lane / 5, lane
+// % 5) of a row handles component i of its p-th neighbour of three, so the
+// three neighbours are polled, scaled and multiplied at once.  GB300 issues a
+// warp's FP64 instruction over about 70 cycles of its scheduler whatever
+// lanes are active, so a row costs its count of instructions: 10 here against
+// 105 with one row per lane.  The sums keep the order of lusgs_fwd_row /
+// lusgs_rev_row.
+template <typename TB, bool FWD>
+__device__ __forceinline__ void sweep_row16(const DevMesh& m, const TB* __restrict__ blk, const TB* __restrict__ rD,
+                                            const double* in, double* out, double* r, int c, int* status,
+                                            int spin_limit) {
+  const unsigned half = 0xffffu << (threadIdx.x & 16);
+  const int l16 = threadIdx.x & 15;
+  const int p = l16 / 5, i = l16 - 5 * p;  // lane 15: idle (p == 3)
+  const bool row = c >= 0;
+  int sb = 0, nl = 0, nn = 0, ns = 0, lane = 0;
+  double acc = 0.0, rc = 0.0;
+  if (row) {
+    const int s = c >> 5;
+    lane = c & 31;
+    sb = m.slot_base[s];
+    nl = m.nlow[c];
+    ns = m.nslot[c];
+    nn = FWD ? nl : ns - nl;
+    if (p == 0) acc = FWD ? __ldcg(in + 5 * (size_t)c + i) : __ldcg(in + SWEEP_PAD * (size_t)c + i);
+    if (!FWD) rc = double(rD[c]);
+  }
+  for (int q0 = 0; __any_sync(half, q0 < nn); q0 += 3) {
+    const int q = q0 + p;
+    const bool on = p < 3 && q < nn;
+    double B[5], rj = 1.0;
+    int col = 0, t = 0;
+    if (on) {
+      t = FWD ? q : ns - 1 - q;
+      col = m.scol[(sb + t) * 32 + lane];
+      const double* bp = (const double*)blk + ((size_t)(sb + t) * 25 + 5 * i) * 32 + lane;
+#pragma unroll
+      for (int j = 0; j < 5; ++j) B[j] = bp[j * 32];
+      if (FWD) rj = double(rD[col]);
+    }
+    // poll this lane's word; the lanes of a half-warp go on together
+    double v = 0.0;
+    bool ready = !on;
+    int it = 0;
+    while (true) {
+      if (!ready) {
+        asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(out + SWEEP_PAD * (size_t)col + i) : "memory");
+        ready = sweep_word_set(v);
+      }
+      if (__all_sync(half, ready)) break;
+      ++it;
+      bool stop = it > spin_limit;
+      if (stop && l16 == 0) atomicOr(status, 8);
+      if ((it & 63) == 0) stop = stop || (ld_relaxed_int(status) & 8);
+      if (__any_sync(half, stop)) {
+        if (p == 0) {
+          const double z = 0.0;
+          asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(out + SWEEP_PAD * (size_t)c + i), "d"(z) : "memory");
+        }
+        return;
+      }
+    }
+    const double d = FWD ? rj * v : v;
+    double y = 0.0;
+#pragma unroll
+    for (int j = 0; j < 5; ++j) {
+      const double dj = __shfl_sync(half, d, 5 * p + j, 16);
+      if (on) y += B[j] * dj;
+    }
+    if (m.vjslot) {
+      // the non-LF viscous part needs the neighbour's five words in one lane
+      double x5[5], y5[5] = {0, 0, 0, 0, 0};
+#pragma unroll
+      for (int j = 0; j < 5; ++j) x5[j] = __shfl_sync(half, d, 5 * p + j, 16);
+      if (on) {
+        vj_sub<TB>(m, sb + t, lane, col, x5, y5);
+#pragma unroll
+        for (int j = 0; j < 5; ++j)
+          if (j == i) y += y5[j];
+      }
+    }
+    const double y1 = __shfl_sync(half, y, 5 + i, 16), y2 = __shfl_sync(half, y, (10 + i) & 15, 16);
+    acc -= y;
+    if (q0 + 1 < nn) acc -= y1;
+    if (q0 + 2 < nn) acc -= y2;
+  }
+  if (row && p == 0) {
+    if (!FWD) {
+      acc = rc * acc;
+      r[5 * (size_t)c + i] = acc;
+    }
+    acc = sweep_word(acc);
+    asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(out + SWEEP_PAD * (size_t)c + i), "d"(acc) : "memory");
+  }
+}
+
 // FWD: in = the right-hand side r (5 words per row), out = the forward
 // result; !FWD: in = the forward result (padded), out = the reverse result,
 // also written to r (5 words per row).  `out` holds the sentinel on entry.
 template <typename TB, typename TV, bool FWD>
-__global__ void __launch_bounds__(SWEEP_THREADS) k_lusgs_sweep(DevMesh m, const TB* __restrict__ blk,
-                                                     const TB* __restrict__ rD, const TV* in, TV* out, TV* r,
-                                                     const int* __restrict__ order, int count, unsigned int* ticket,
-                                                     int* status, int spin_limit) {
-  __shared__ int base;
-  if (threadIdx.x == 0) base = (int)atomicAdd(ticket, blockDim.x);
-  __syncthreads();
-  const int i = base + threadIdx.x;
-  if (i >= count) return;
-  const int c = order[i];
+__device__ __forceinline__ void sweep_row(const DevMesh& m, const TB* __restrict__ blk, const TB* __restrict__ rD,
+                                          const TV* in, TV* out, TV* r, int c, int* status, int spin_limit) {
   const int s = c >> 5, lane = c & 31;
   const int sb = m.slot_base[s];
   const int nl = m.nlow[c], ns = m.nslot[c];
@@ -661,7 +737,6 @@ __global__ void __launch_bounds__(SWEEP_THREADS) k_lusgs_sweep(DevMesh m, const 
     if (p < nn) pending |= 1u << p;
   {
     int it = 0;
-    unsigned ns_ = 32;
     while (true) {
 #pragma unroll
       for (int p = 0; p < PF; ++p)
@@ -677,8 +752,6 @@ __global__ void __launch_bounds__(SWEEP_THREADS) k_lusgs_sweep(DevMesh m, const 
         st_relaxed5(mine, z);
         return;
       }
-      __nanosleep(ns_);
-      if (ns_ < 256) ns_ <<= 1;
     }
   }
 #pragma unroll
@@ -699,7 +772,6 @@ __global__ void __launch_bounds__(SWEEP_THREADS) k_lusgs_sweep(DevMesh m, const 
     const int col = m.scol[(sb + t) * 32 + lane];
     TV rj5[5];
     int it = 0;
-    unsigned ns_ = 32;
     while (true) {
       ld_relaxed5(out + (size_t)SWEEP_PAD * col, rj5);
       if (sweep_ready(rj5)) break;
@@ -710,8 +782,6 @@ __global__ void __launch_bounds__(SWEEP_THREADS) k_lusgs_sweep(DevMesh m, const 
         st_relaxed5(mine, z);
         return;
       }
-      __nanosleep(ns_);
-      if (ns_ < 256) ns_ <<= 1;
     }
     const TV rj = FWD ? TV(rD[col]) : TV(1);
     TV dj[5], y[5];
@@ -731,7 +801,32 @@ __global__ void __launch_bounds__(SWEEP_THREADS) k_lusgs_sweep(DevMesh m, const 
 #pragma unroll
     for (int k = 0; k < 5; ++k) r[5 * c + k] = acc[k];
   }
+#pragma unroll
+  for (int k = 0; k < 5; ++k) acc[k] = sweep_word(acc[k]);
   st_relaxed5(mine, acc);
+}
+
+template <typename TB, typename TV, bool FWD>
+__global__ void __launch_bounds__(SWEEP_THREADS) k_lusgs_sweep(DevMesh m, const TB* __restrict__ blk,
+                                                     const TB* __restrict__ rD, const TV* in, TV* out, TV* r,
+                                                     const int* __restrict__ order, int tickets,
+                                                     unsigned int* ticket, int* status, int spin_limit) {
+  constexpr int ROWS = sweep_rows<TB, TV>;
+  const int total = tickets * (SWEEP_TICKET / ROWS);
+  while (true) {
+    int t = 0;
+    if (threadIdx.x == 0) t = (int)atomicAdd(ticket, 1u);
+    t = __shfl_sync(0xffffffffu, t, 0);
+    if (t >= total) return;
+    if constexpr (ROWS == 2) {
+      const int c = order[t * 2 + (threadIdx.x >> 4)];
+      sweep_row16<TB, FWD>(m, blk, rD, in, out, r, c, status, spin_limit);
+    } else {
+      const int c = order[t * SWEEP_TICKET + threadIdx.x];
+      if (c >= 0) sweep_row<TB, TV, FWD>(m, blk, rD, in, out, r, c, status, spin_limit);
+    }
+    __syncwarp();
+  }
 }
 
 template <typename TB, typename TV>
@@ -1052,26 +1147,24 @@ static void rev_level(Handle& h, const TB* blk, const TB* rD, TV* r, const int* 
                                        h.m, blk, rD, r, cells, start, cnt));
 }
 
+// Resident warps of a sync-free sweep: about four levels' worth, so that the
+// loads of the next levels' rows are in flight while a level is polled, and no
+// more pollers than that.  Measured on a 227k-cell RCM box (181 levels, ROWS
+// per warp 2 in FP64, 32 in FP32): one / two / four / eight levels 537 / 340 /
+// 276 / 278 us per FP64 sweep; FP32 268 us whatever the grid.
+static int sweep_grid(const DevMesh& m, int tickets, int rows) {
+  const long warps = (long)tickets * (SWEEP_TICKET / rows);
+  const long g = std::min(std::max(4 * warps / m.nfl, 152L), 152L * 32);
+  return (int)std::min(g, warps);
+}
+
 template <typename TB, typename TV>
 static void lusgs_t(Handle& h, TV* r, const TB* blkIn = nullptr, const TB* rDIn = nullptr) {
   const DevMesh& m = h.m;
   const TB* blk = blkIn ? blkIn : (const TB*)h.blk;
   const TB* rD = rDIn ? rDIn : (const TB*)h.rD;
-  // forward sweep, then reverse sweep; many small levels run in one CTA
-  if ((long)m.N < 2048L * m.nfl) {
-    ICS_LAUNCH(h, ICS_K_LUSGS_FWD, k_lusgs_block<TB, TV, true><<<1, 1024, 0, h.stream>>>(m, blk, rD, r, m.fl_cells, m.fl_lptr, m.nfl));
-    if ((long)m.N < 2048L * m.nrl) {
-      ICS_LAUNCH(h, ICS_K_LUSGS_REV,
-                 k_lusgs_block<TB, TV, false><<<1, 1024, 0, h.stream>>>(m, blk, rD, r, m.rl_cells, m.rl_lptr, m.nrl));
-      return;
-    }
-  }
-  // Level launches.  Forward level 0 has no lower neighbours (r' = r): skipped.
-  // When the last forward level holds exactly the rows of the first reverse
-  // level (rows without upper neighbours, e.g. the last colour), the two are
-  // fused: r' = r - L d*, then delta = rD r' in the same pass.
-  // many levels on a large mesh: one sync-free launch per sweep
-  if (m.nfl > 2 && (long)m.N >= 2048L * m.nfl) {
+  // many levels: one sync-free launch per sweep
+  if (m.sw_fwd) {
     cudaStream_t st = h.stream;
     int* status = &h.ks->status;
     TV* fwd = (TV*)m.sweep_pad;
@@ -1079,53 +1172,49 @@ static void lusgs_t(Handle& h, TV* r, const TB* blkIn = nullptr, const TB* rDIn 
     const size_t padBytes = (size_t)SWEEP_PAD * m.N * sizeof(TV);
     ICS_CUDA(cudaMemsetAsync(fwd, 0xff, 2 * padBytes, st));  // the sentinel in both outputs
     ICS_CUDA(cudaMemsetAsync(m.sweep_ticket, 0, 2 * sizeof(unsigned int), st));
-    ICS_LAUNCH(h, ICS_K_LUSGS_FWD, k_lusgs_sweep<TB, TV, true><<<grid_for(m.N, SWEEP_THREADS), SWEEP_THREADS, 0, st>>>(
-                                       m, blk, rD, r, fwd, nullptr, m.fl_cells, m.N, m.sweep_ticket, status,
+    const int grid = sweep_grid(m, m.nsw_fwd, sweep_rows<TB, TV>);
+    ICS_LAUNCH(h, ICS_K_LUSGS_FWD, k_lusgs_sweep<TB, TV, true><<<grid, SWEEP_THREADS, 0, st>>>(
+                                       m, blk, rD, r, fwd, nullptr, m.sw_fwd, m.nsw_fwd, m.sweep_ticket, status,
                                        SWEEP_SPIN_LIMIT));
-    ICS_LAUNCH(h, ICS_K_LUSGS_REV, k_lusgs_sweep<TB, TV, false><<<grid_for(m.N, SWEEP_THREADS), SWEEP_THREADS, 0, st>>>(
-                                       m, blk, rD, fwd, rev, r, m.rl_cells, m.N, m.sweep_ticket + 1, status,
+    ICS_LAUNCH(h, ICS_K_LUSGS_REV, k_lusgs_sweep<TB, TV, false><<<grid, SWEEP_THREADS, 0, st>>>(
+                                       m, blk, rD, fwd, rev, r, m.sw_rev, m.nsw_rev, m.sweep_ticket + 1, status,
                                        SWEEP_SPIN_LIMIT));
     return;
   }
-  const bool blockFwd = (long)m.N < 2048L * m.nfl;
-  const bool fuse = !blockFwd && m.fuse_last;
-  if (!blockFwd) {
-    for (int l = 0; l < m.nfl; ++l) {
-      const bool last = l == m.nfl - 1;
-      if (l == 0 && !(fuse && last)) continue;
-      const int a = m.fl_ptr[l], cnt = m.fl_ptr[l + 1] - a;
-      const bool contig = m.fl_cstart[l] >= 0;
-      const int* cells = contig ? nullptr : m.fl_cells;
-      const int start = contig ? m.fl_cstart[l] : a;
-      if (fuse && last)
-        ICS_LAUNCH(h, ICS_K_LUSGS_FWD, k_lusgs_level<TB, TV, 2><<<grid_for(cnt, 128), 128, 0, h.stream>>>(
-                                           m, blk, rD, r, cells, start, cnt));
-      else
-        ICS_LAUNCH(h, ICS_K_LUSGS_FWD, k_lusgs_level<TB, TV, 0><<<grid_for(cnt, 128), 128, 0, h.stream>>>(
-                                           m, blk, rD, r, cells, start, cnt));
-    }
+  // One or two levels (colour-blocked numberings): a launch per level.
+  // Forward level 0 has no lower neighbours (r' = r): skipped.  When the last
+  // forward level holds exactly the rows of the first reverse level (rows
+  // without upper neighbours, e.g. the last colour), the two are fused:
+  // r' = r - L d*, then delta = rD r' in the same pass.
+  for (int l = 0; l < m.nfl; ++l) {
+    const bool last = l == m.nfl - 1;
+    if (l == 0 && !(m.fuse_last && last)) continue;
+    const int a = m.fl_ptr[l], cnt = m.fl_ptr[l + 1] - a;
+    const bool contig = m.fl_cstart[l] >= 0;
+    const int* cells = contig ? nullptr : m.fl_cells;
+    const int start = contig ? m.fl_cstart[l] : a;
+    if (m.fuse_last && last)
+      ICS_LAUNCH(h, ICS_K_LUSGS_FWD, k_lusgs_level<TB, TV, 2><<<grid_for(cnt, 128), 128, 0, h.stream>>>(
+                                         m, blk, rD, r, cells, start, cnt));
+    else
+      ICS_LAUNCH(h, ICS_K_LUSGS_FWD, k_lusgs_level<TB, TV, 0><<<grid_for(cnt, 128), 128, 0, h.stream>>>(
+                                         m, blk, rD, r, cells, start, cnt));
   }
-  if ((long)m.N < 2048L * m.nrl) {
-    ICS_LAUNCH(h, ICS_K_LUSGS_REV,
-               k_lusgs_block<TB, TV, false><<<1, 1024, 0, h.stream>>>(m, blk, rD, r, m.rl_cells, m.rl_lptr, m.nrl));
-  } else {
-    for (int l = fuse ? 1 : 0; l < m.nrl; ++l) {
-      const int a = m.rl_ptr[l], cnt = m.rl_ptr[l + 1] - a;
-      const bool contig = m.rl_cstart[l] >= 0;
-      rev_level<TB, TV>(h, blk, rD, r, contig ? nullptr : m.rl_cells, contig ? m.rl_cstart[l] : a, cnt);
-    }
+  for (int l = m.fuse_last ? 1 : 0; l < m.nrl; ++l) {
+    const int a = m.rl_ptr[l], cnt = m.rl_ptr[l + 1] - a;
+    const bool contig = m.rl_cstart[l] >= 0;
+    rev_level<TB, TV>(h, blk, rD, r, contig ? nullptr : m.rl_cells, contig ? m.rl_cstart[l] : a, cnt);
   }
 }
 
 // w = M^-1 A x with M the LU-SGS preconditioner; true when the fused
-// three-pass form applies (two levels, the second without upper neighbours,
-// level launches rather than the single-CTA walk)
+// three-pass form applies (two levels, the second without upper neighbours)
 template <typename TB, typename TV>
 static bool fused_op_available(const Handle& h) {
   const DevMesh& m = h.m;
   // (the fused passes carry no cyclic couplings: those meshes take spmv_t)
   return h.tuneFused && h.cfg.c.preconditioner == ICS_PC_LUSGS && m.nfl == 2 && m.nrl == 2 && m.fuse_last &&
-         (long)m.N >= 2048L * m.nfl && m.ncyc == 0;
+         m.ncyc == 0;
 }
 
 // vout != nullptr: x is unnormalised; v = x / beta is stored in vout and
@@ -1186,20 +1275,20 @@ static void precondition_t(Handle& h, TV* r) {
     ICS_LAUNCH(h, ICS_K_JACOBI, k_jacobi_apply<TB, TV><<<grid_for(h.m.N, 128), 128, 0, h.stream>>>(h.m.N, (const TB*)h.dginv, r));
 }
 
-// One sync-free forward sweep over `order` (count rows) with a given wait
+// One sync-free forward sweep over `order` (whole tickets) with a given wait
 // bound; used to exercise the bounded waits (a row left out of the order
 // never writes its result, so its dependents must give up and report).
 template <typename TB, typename TV>
-static void sweep_probe_t(Handle& h, const int* order, int count, int spin_limit) {
+static void sweep_probe_t(Handle& h, const int* order, int tickets, int spin_limit) {
   const DevMesh& m = h.m;
   cudaStream_t st = h.stream;
   TV* fwd = (TV*)m.sweep_pad;
   ICS_CUDA(cudaMemsetAsync(fwd, 0xff, (size_t)SWEEP_PAD * m.N * sizeof(TV), st));
   ICS_CUDA(cudaMemsetAsync(m.sweep_ticket, 0, 2 * sizeof(unsigned int), st));
   ICS_CUDA(cudaMemsetAsync(h.kw, 0, 5ull * m.N * sizeof(TV), st));
-  ICS_LAUNCH(h, ICS_K_LUSGS_FWD, k_lusgs_sweep<TB, TV, true><<<grid_for(count, SWEEP_THREADS), SWEEP_THREADS, 0, st>>>(
+  ICS_LAUNCH(h, ICS_K_LUSGS_FWD, k_lusgs_sweep<TB, TV, true><<<sweep_grid(m, tickets, sweep_rows<TB, TV>), SWEEP_THREADS, 0, st>>>(
                                      m, (const TB*)h.blk, (const TB*)h.rD, (const TV*)h.kw, fwd, nullptr, order,
-                                     count, m.sweep_ticket, &h.ks->status, spin_limit));
+                                     tickets, m.sweep_ticket, &h.ks->status, spin_limit));
   ICS_CUDA(cudaGetLastError());
 }
 
@@ -1221,11 +1310,11 @@ bool fused_operator(Handle& h, const void* x, void* w, void* vout) {
   return fused_op_t<double, double>(h, (const double*)x, (double*)w, (double*)vout);
 }
 
-void sweep_probe(Handle& h, const int* order, int count, int spin_limit) {
+void sweep_probe(Handle& h, const int* order, int tickets, int spin_limit) {
   if (prec(h) == ICS_PREC_MIXED)
-    sweep_probe_t<float, float>(h, order, count, spin_limit);
+    sweep_probe_t<float, float>(h, order, tickets, spin_limit);
   else
-    sweep_probe_t<double, double>(h, order, count, spin_limit);
+    sweep_probe_t<double, double>(h, order, tickets, spin_limit);
 }
 
 void spmv(Handle& h, const void* x, void* y) {
