@@ -11,9 +11,8 @@
 //      forward kernels of the residual, k_fields and k_grad);
 //   2. k_adj_face (internal faces): F_bar = u_nei - u_own, then the adjoints
 //      of the two reconstructed face states, F_bar . dF/dq_L and
-//      F_bar . dF/dq_R, with the flux's local partial derivatives taken by
-//      forward-mode dual numbers through the same flux function the residual
-//      uses (16 inputs, 5 outputs; one pass per input);
+//      F_bar . dF/dq_R, by walking the flux function backwards
+//      (flux_adjoint.cuh);
 //   3. k_adj_lim (cells): the reconstruction's transpose (the upwind value
 //      and the gradient extrapolation d . g of every face of the cell), then
 //      the transpose of the cellLimited limiter, recomputing the cell's Gauss
@@ -24,8 +23,8 @@
 //   4. k_adj_cell (cells): the Gauss gradient's transpose (each face value
 //      w q_own + (1 - w) q_nei feeds both cells' gradients), the recorded
 //      bound contributions of the neighbours, and the transpose of the
-//      pointwise map W -> q (five dual-number passes of the cell map), plus
-//      the diagonal physical ddt, MRF rotation and Harmonic Balance terms.
+//      pointwise map W -> q (cell_adjoint), plus the diagonal physical ddt,
+//      MRF rotation and Harmonic Balance terms.
 //
 // Every branch (limiter selection, flux region) is decided on the values as
 // the forward pass decides it, so this is the transpose of ics_jvp's linear
@@ -35,37 +34,87 @@
 // kernel transposes it there and hands on the adjoint of the gradient's
 // projection.  Not provided (the entry point returns ICS_ERR_ARG): viscous
 // terms and cyclic patches.
+#include "flux_adjoint.cuh"
 #include "residual.cuh"
 
 namespace ics {
 
-// Pointwise map W -> q of one cell: the primitives of k_derive (U = rhoU /
-// rho, e = rhoE / rho - |U|^2 / 2, T = e / Cv, p = rho R T) then the fields
-// of k_fields (E, H, sound speed or AUSM+up's c*), in the same arithmetic.
-template <typename Real>
-__device__ __forceinline__ void cell_q(const Real W[5], const ResParams& P, Real q[NQ]) {
-  const Real rho = W[0];
-  const Real U[3] = {W[1] / rho, W[2] / rho, W[3] / rho};
-  const Real e = W[4] / rho - 0.5 * dot3(U, U);
-  const Real T = e / P.Cv;
-  const Real p = rho / (1.0 / (P.R * T));
-  const Real E = P.Cv * T + 0.5 * (U[0] * U[0] + U[1] * U[1] + U[2] * U[2]);
-  const Real H = fmax(E, SMALL) + fmax(p / rho, SMALL);
-  const Real psi = 1.0 / (P.R * T);
-  const Real cl = sqrt(P.gamma / psi);
-  q[Q_RHO] = rho;
-  q[Q_P] = p;
-  q[Q_UX] = U[0];
-  q[Q_UY] = U[1];
-  q[Q_UZ] = U[2];
-  q[Q_E] = E;
-  q[Q_H] = H;
-  q[Q_C] = P.scheme == ICS_FLUX_AUSMPLUSUP ? sqrt(P.cstarFac * H) : fmax(cl, VSMALL);
+// Transpose of the pointwise map W -> q of one cell (the primitives of
+// k_derive: U = rhoU / rho, e = rhoE / rho - |U|^2 / 2, T = e / Cv, p = rho R T;
+// then the fields of k_fields: E, H, sound speed or AUSM+up's c*): the adjoint
+// r of W from the adjoint qb of q, walked backwards through those expressions.
+// (Five dual-number passes of that map and a division by V per face and field
+// made k_adj_cell 2.65 ms on 465k cells; with this and the 1/V folded into
+// k_adj_lim's output it takes 0.54 ms.)
+__device__ __forceinline__ void cell_adjoint(const double W[5], const ResParams& P, const double qb[NQ], double r[5]) {
+  const double rho = W[0], ir = 1.0 / rho;
+  const double U[3] = {W[1] * ir, W[2] * ir, W[3] * ir};
+  const double e = W[4] * ir - 0.5 * dot3(U, U);
+  const double T = e / P.Cv;
+  const double p = rho * P.R * T;
+  const double E = P.Cv * T + 0.5 * dot3(U, U);
+  double Hb = qb[Q_H], Tb = 0.0, pb = qb[Q_P], rb = qb[Q_RHO];
+  if (P.scheme == ICS_FLUX_AUSMPLUSUP) {
+    const double H = fmax(E, SMALL) + fmax(p * ir, SMALL);
+    const double c = sqrt(P.cstarFac * H);
+    if (c > 0.0) Hb += qb[Q_C] * 0.5 * P.cstarFac / c;
+  } else {
+    const double c = sqrt(P.gamma * P.R * T);
+    if (c >= VSMALL) Tb = qb[Q_C] * 0.5 * P.gamma * P.R / c;
+  }
+  const double Eb = qb[Q_E] + (E >= SMALL ? Hb : 0.0);
+  if (p * ir >= SMALL) {
+    pb += Hb * ir;
+    rb -= Hb * p * ir * ir;
+  }
+  Tb += P.Cv * Eb + pb * rho * P.R;
+  rb += pb * P.R * T;
+  const double eb = Tb / P.Cv;
+  double ub = 0.0;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const double Ub = qb[Q_UX + k] + (Eb - eb) * U[k];
+    r[1 + k] = Ub * ir;
+    ub += Ub * U[k];
+  }
+  r[4] = eb * ir;
+  r[0] = rb - (ub + eb * W[4] * ir) * ir;
+}
+
+// The flux adjoint of one face by forward-mode dual numbers, one pass per
+// input: the Roe flux in a moving frame, and HLLC faces whose wave switches
+// overlap (flux_adjoint.cuh has the others).
+__device__ __noinline__ void face_adjoint_dual(const ResParams& P, const double* qs, const double* n, const double* S,
+                                               double magS, double um, const double* Fb, double* qb) {
+#pragma unroll 1
+  for (int j = 0; j < 2 * NQ; ++j) {
+    if (P.scheme == ICS_FLUX_ROE && (j % NQ) == Q_C) {
+      qb[j] = 0.0;
+      continue;
+    }
+    Dual x[2 * NQ];
+#pragma unroll
+    for (int i = 0; i < 2 * NQ; ++i) x[i] = Dual(qs[i], i == j ? 1.0 : 0.0);
+    FStateT<Dual> L{x[Q_RHO], x[Q_P], {x[Q_UX], x[Q_UY], x[Q_UZ]}, x[Q_E], x[Q_H], x[Q_C]};
+    FStateT<Dual> R{x[NQ + Q_RHO], x[NQ + Q_P], {x[NQ + Q_UX], x[NQ + Q_UY], x[NQ + Q_UZ]},
+                    x[NQ + Q_E],   x[NQ + Q_H], x[NQ + Q_C]};
+    Dual out[5];
+    if (P.scheme == ICS_FLUX_HLLC)
+      flux_hllc(L, R, n, magS, P.gamma, um, out);
+    else
+      flux_roe(L, R, n, magS, P.gamma, P.entropyFix, um, out);
+    double a = 0.0;
+#pragma unroll
+    for (int i = 0; i < 5; ++i) a += Fb[i] * out[i].d;
+    qb[j] = a;
+  }
 }
 
 // adjoint of the reconstructed face states: aF[j][F], j < NQ the owner-side
 // (left) field j, j >= NQ the neighbour-side (right) field j - NQ
-template <bool MRF>
+// SCHEME: ICS_FLUX_*; MRF: a moving frame's face velocity; TVD: some field is
+// reconstructed by a limitedScheme.  Bound by the FP64 pipe.
+template <int SCHEME, bool MRF, bool TVD>
 __global__ void __launch_bounds__(128) k_adj_face(DevMesh m, ResParams P, const double* __restrict__ q,
                                                   const double* __restrict__ grad, const double* __restrict__ u,
                                                   double* __restrict__ aF, double* __restrict__ aS) {
@@ -76,7 +125,7 @@ __global__ void __launch_bounds__(128) k_adj_face(DevMesh m, ResParams P, const 
   double qs[2 * NQ];
 #pragma unroll
   for (int k = 0; k < NQ; ++k) {
-    if (P.scheme == ICS_FLUX_ROE && k == Q_C) {
+    if (SCHEME == ICS_FLUX_ROE && k == Q_C) {
       qs[k] = qs[NQ + k] = 0.0;
       continue;
     }
@@ -92,42 +141,40 @@ __global__ void __launch_bounds__(128) k_adj_face(DevMesh m, ResParams P, const 
   const double S[3] = {m.Sf[f], m.Sf[F + f], m.Sf[2 * F + f]};
   const double magS = m.magSf[f];
   const double um = MRF ? m.mrfU[f] : 0.0;
-  double qb[2 * NQ];
-#pragma unroll 1
-  for (int j = 0; j < 2 * NQ; ++j) {
-    if (P.scheme == ICS_FLUX_ROE && (j % NQ) == Q_C) {
-      qb[j] = 0.0;
-      continue;
-    }
-    Dual x[2 * NQ];
+  const FState L{qs[Q_RHO], qs[Q_P], {qs[Q_UX], qs[Q_UY], qs[Q_UZ]}, qs[Q_E], qs[Q_H], qs[Q_C]};
+  const FState R{qs[NQ + Q_RHO], qs[NQ + Q_P], {qs[NQ + Q_UX], qs[NQ + Q_UY], qs[NQ + Q_UZ]},
+                 qs[NQ + Q_E],   qs[NQ + Q_H], qs[NQ + Q_C]};
+  FState Lb, Rb;
+  bool done = true;
+  if constexpr (SCHEME == ICS_FLUX_AUSMPLUSUP)
+    flux_ausm_adjoint(L, R, S, magS, P.lowMach, um, Fb, Lb, Rb);
+  else if constexpr (SCHEME == ICS_FLUX_HLLC)
+    done = flux_hllc_adjoint(L, R, n, magS, P.gamma, um, Fb, Lb, Rb);
+  else if (!MRF || um == 0.0)
+    flux_roe_adjoint(L, R, n, magS, P.gamma, P.entropyFix, Fb, Lb, Rb);
+  else
+    done = false;
+  double qb[2 * NQ] = {Lb.rho, Lb.p, Lb.U[0], Lb.U[1], Lb.U[2], Lb.E, Lb.H, Lb.c,
+                       Rb.rho, Rb.p, Rb.U[0], Rb.U[1], Rb.U[2], Rb.E, Rb.H, Rb.c};
+  if (SCHEME != ICS_FLUX_AUSMPLUSUP && !done) {
+    double qc[2 * NQ], tmp[2 * NQ];
 #pragma unroll
-    for (int i = 0; i < 2 * NQ; ++i) x[i] = Dual(qs[i], i == j ? 1.0 : 0.0);
-    FStateT<Dual> L{x[Q_RHO], x[Q_P], {x[Q_UX], x[Q_UY], x[Q_UZ]}, x[Q_E], x[Q_H], x[Q_C]};
-    FStateT<Dual> R{x[NQ + Q_RHO], x[NQ + Q_P], {x[NQ + Q_UX], x[NQ + Q_UY], x[NQ + Q_UZ]},
-                    x[NQ + Q_E],   x[NQ + Q_H], x[NQ + Q_C]};
-    Dual out[5];
-    if (P.scheme == ICS_FLUX_AUSMPLUSUP)
-      flux_ausm(L, R, S, magS, P.lowMach, um, out);
-    else if (P.scheme == ICS_FLUX_HLLC)
-      flux_hllc(L, R, n, magS, P.gamma, um, out);
-    else
-      flux_roe(L, R, n, magS, P.gamma, P.entropyFix, um, out);
-    double a = 0.0;
+    for (int i = 0; i < 2 * NQ; ++i) qc[i] = qs[i];
+    face_adjoint_dual(P, qc, n, S, magS, um, Fb, tmp);
 #pragma unroll
-    for (int i = 0; i < 5; ++i) a += Fb[i] * out[i].d;
-    qb[j] = a;
+    for (int i = 0; i < 2 * NQ; ++i) qb[i] = tmp[i];
   }
   // the reconstructions' transpose: adjoints reaching the owner's and the
   // neighbour's value (aF[k], aF[NQ + k]); for the TVD limitedSchemes, whose
   // face value depends on both cells and on the upwind cell's gradient
   // projected on C_nei - C_own, also the adjoints of those projections of
   // the left and right values (aS[k], aS[NQ + k])
-#pragma unroll 1
+#pragma unroll
   for (int k = 0; k < NQ; ++k) {
     const int sch = recon_of(P, k);
-    double ao = qb[k], an = qb[NQ + k], sl = 0.0, sr = 0.0;
-    const bool used = !(P.scheme == ICS_FLUX_ROE && k == Q_C);  // Roe reconstructs no sound speed
-    if (used && (sch == ICS_RECON_VANLEER || sch == ICS_RECON_MINMOD)) {
+    double ao = qb[k], an = qb[NQ + k];
+    const bool used = !(SCHEME == ICS_FLUX_ROE && k == Q_C);  // Roe reconstructs no sound speed
+    if (TVD && used && (sch == ICS_RECON_VANLEER || sch == ICS_RECON_MINMOD)) {
       const double qo = q[k * N + o], qn = q[k * N + nb];
       const double d0 = m.dCC[f], d1 = m.dCC[F + f], d2 = m.dCC[2 * F + f];
       const double gl = d0 * grad[(3 * k) * N + o] + d1 * grad[(3 * k + 1) * N + o] + d2 * grad[(3 * k + 2) * N + o];
@@ -143,20 +190,18 @@ __global__ void __launch_bounds__(128) k_adj_face(DevMesh m, ResParams P, const 
       }
       ao = qb[k] * dl[0] + qb[NQ + k] * dr[0];
       an = qb[k] * dl[1] + qb[NQ + k] * dr[1];
-      sl = qb[k] * dl[2];
-      sr = qb[NQ + k] * dr[2];
+      aS[(size_t)k * F + f] = qb[k] * dl[2];
+      aS[(size_t)(NQ + k) * F + f] = qb[NQ + k] * dr[2];
     }
     aF[(size_t)k * F + f] = ao;
     aF[(size_t)(NQ + k) * F + f] = an;
-    aS[(size_t)k * F + f] = sl;
-    aS[(size_t)(NQ + k) * F + f] = sr;
   }
 }
 
 // Per cell and field: the transpose of the reconstruction (upwind value and
 // gradient extrapolation on every face of the cell) and of the cellLimited
 // limiter.  Outputs: aQ[k][N] the adjoint reaching q_k of the cell directly,
-// aG[3k+d][N] the adjoint of its unlimited Gauss gradient, and per bound
+// aG[3k+d][N] the adjoint of its unlimited Gauss gradient over V, and per bound
 // (max: slot k, min: slot NQ + k) the neighbour cell that attained it
 // (aSrc, -1 for none) and the adjoint it receives (aVal).
 template <int LIMITED>
@@ -170,6 +215,7 @@ __global__ void __launch_bounds__(128) k_adj_lim(DevMesh m, unsigned mask, unsig
   const int N = m.N, F = m.F, B = m.B;
   const int e0 = m.cptr[c], e1 = m.cptr[c + 1];
   const int b0 = m.bptr[c], b1 = m.bptr[c + 1];
+  const double rV = 1.0 / m.V[c];
 #pragma unroll 1
   for (int k = 0; k < NQ; ++k) {
     const bool hasGrad = (mask >> k) & 1;
@@ -238,7 +284,6 @@ __global__ void __launch_bounds__(128) k_adj_lim(DevMesh m, unsigned mask, unsig
           srcMin = -1;
         }
       }
-      const double rV = 1.0 / m.V[c];
       G[0] = G[0] * rV;
       G[1] = G[1] * rV;
       G[2] = G[2] * rV;
@@ -303,14 +348,14 @@ __global__ void __launch_bounds__(128) k_adj_lim(DevMesh m, unsigned mask, unsig
       double lim = 1.0, lr = 1.0, dra = 0.0, drb = 0.0;
       if (anyFace && sel != 0) {
         if (LIMITED == 2) {
-          const double num = ra * ra + 2 * ra * rb, den = ra * ra + ra * rb + 2 * rb * rb;
-          lr = num / den;
-          dra = ((2 * ra + 2 * rb) * den - num * (2 * ra + rb)) / (den * den);
-          drb = (2 * ra * den - num * (ra + 4 * rb)) / (den * den);
+          const double num = ra * ra + 2 * ra * rb, iden = 1.0 / (ra * ra + ra * rb + 2 * rb * rb);
+          lr = num * iden;
+          dra = ((2 * ra + 2 * rb) - lr * (2 * ra + rb)) * iden;
+          drb = (2 * ra - lr * (ra + 4 * rb)) * iden;
         } else {
-          lr = ra / rb;
           dra = 1.0 / rb;
-          drb = -ra / (rb * rb);
+          lr = ra / rb;
+          drb = -lr * dra;
         }
         lim = fmin(1.0, lr);
       }
@@ -348,9 +393,10 @@ __global__ void __launch_bounds__(128) k_adj_lim(DevMesh m, unsigned mask, unsig
       }
     }
     aQ[(size_t)k * N + c] = qd;
-    aG[(size_t)(3 * k) * N + c] = hasGrad ? gb[0] : 0.0;
-    aG[(size_t)(3 * k + 1) * N + c] = hasGrad ? gb[1] : 0.0;
-    aG[(size_t)(3 * k + 2) * N + c] = hasGrad ? gb[2] : 0.0;
+    // the Gauss sum's 1/V here, once per cell, rather than per face in k_adj_cell
+    aG[(size_t)(3 * k) * N + c] = hasGrad ? gb[0] * rV : 0.0;
+    aG[(size_t)(3 * k + 1) * N + c] = hasGrad ? gb[1] * rV : 0.0;
+    aG[(size_t)(3 * k + 2) * N + c] = hasGrad ? gb[2] * rV : 0.0;
     aSrc[(size_t)k * N + c] = sMax;
     aVal[(size_t)k * N + c] = vMax;
     aSrc[(size_t)(NQ + k) * N + c] = sMin;
@@ -382,11 +428,9 @@ __global__ void __launch_bounds__(128) k_adj_cell(DevMesh m, ResParams P, unsign
         const int f = isOwn ? code : ~code;
         const int o = m.own[f], nb = m.nei[f];
         const double S0 = m.Sf[f], S1 = m.Sf[F + f], S2 = m.Sf[2 * F + f];
-        const double go = S0 * aG[(size_t)(3 * k) * N + o] + S1 * aG[(size_t)(3 * k + 1) * N + o] +
-                          S2 * aG[(size_t)(3 * k + 2) * N + o];
-        const double gn = S0 * aG[(size_t)(3 * k) * N + nb] + S1 * aG[(size_t)(3 * k + 1) * N + nb] +
-                          S2 * aG[(size_t)(3 * k + 2) * N + nb];
-        const double sfBar = go / m.V[o] - gn / m.V[nb];
+        const double sfBar = S0 * (aG[(size_t)(3 * k) * N + o] - aG[(size_t)(3 * k) * N + nb]) +
+                             S1 * (aG[(size_t)(3 * k + 1) * N + o] - aG[(size_t)(3 * k + 1) * N + nb]) +
+                             S2 * (aG[(size_t)(3 * k + 2) * N + o] - aG[(size_t)(3 * k + 2) * N + nb]);
         const double wf = m.w[f];
         acc += (isOwn ? wf : 1.0 - wf) * sfBar;
         if (limited) {
@@ -399,18 +443,8 @@ __global__ void __launch_bounds__(128) k_adj_cell(DevMesh m, ResParams P, unsign
     qb[k] = acc;
   }
   double r[5];
-#pragma unroll 1
-  for (int j = 0; j < 5; ++j) {
-    Dual Wd[5];
-#pragma unroll
-    for (int i = 0; i < 5; ++i) Wd[i] = Dual(W[5 * c + i], i == j ? 1.0 : 0.0);
-    Dual qd[NQ];
-    cell_q(Wd, P, qd);
-    double a = 0.0;
-#pragma unroll
-    for (int k = 0; k < NQ; ++k) a += qb[k] * qd[k].d;
-    r[j] = a;
-  }
+  const double Wc[5] = {W[5 * c], W[5 * c + 1], W[5 * c + 2], W[5 * c + 3], W[5 * c + 4]};
+  cell_adjoint(Wc, P, qb, r);
   const double Vc = m.V[c];
 #pragma unroll
   for (int k = 0; k < 5; ++k) r[k] -= dgPhys * Vc * u[5 * c + k];
@@ -469,12 +503,29 @@ void launch_residual_vjp(Handle& h, const double* u, double* out) {
     if (sch == ICS_RECON_VANLEER || sch == ICS_RECON_MINMOD) tvd |= 1u << k;
   }
   if (h.m.F > 0) {
-    if (h.m.mrfU)
-      ICS_LAUNCH(h, ICS_K_ADJOINT, (k_adj_face<true><<<grid_for(h.m.F, 128), 128, 0, h.stream>>>(
-                                       h.m, P, h.q, h.grad, u, h.aF, h.aS)));
+    auto face = [&](auto scheme, auto mrf, auto anyTvd) {
+      ICS_LAUNCH(h, ICS_K_ADJOINT,
+                 (k_adj_face<scheme(), mrf(), anyTvd()><<<grid_for(h.m.F, 128), 128, 0, h.stream>>>(
+                     h.m, P, h.q, h.grad, u, h.aF, h.aS)));
+    };
+    auto byTvd = [&](auto scheme, auto mrf) {
+      if (tvd)
+        face(scheme, mrf, std::true_type{});
+      else
+        face(scheme, mrf, std::false_type{});
+    };
+    auto byMrf = [&](auto scheme) {
+      if (h.m.mrfU)
+        byTvd(scheme, std::true_type{});
+      else
+        byTvd(scheme, std::false_type{});
+    };
+    if (P.scheme == ICS_FLUX_AUSMPLUSUP)
+      byMrf(std::integral_constant<int, ICS_FLUX_AUSMPLUSUP>{});
+    else if (P.scheme == ICS_FLUX_HLLC)
+      byMrf(std::integral_constant<int, ICS_FLUX_HLLC>{});
     else
-      ICS_LAUNCH(h, ICS_K_ADJOINT, (k_adj_face<false><<<grid_for(h.m.F, 128), 128, 0, h.stream>>>(
-                                       h.m, P, h.q, h.grad, u, h.aF, h.aS)));
+      byMrf(std::integral_constant<int, ICS_FLUX_ROE>{});
   }
   const int N = h.m.N;
   if (limited == 2)

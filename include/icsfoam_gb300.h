@@ -404,8 +404,8 @@ int ics_vjp(ics_handle h, const double* u, double* JTu, int32_t device);
 /* The same vector-Jacobian product by reverse mode, storing no Jacobian:
  * the face and cell maps of the residual are transposed in reverse order and
  * the fields, Gauss gradients and cellLimited limiters are recomputed from
- * the state in the backward pass (the flux's local partial derivatives by
- * dual numbers through the same flux function).  Equal to ics_vjp up to
+ * the state in the backward pass (the flux functions walked backwards).
+ * Equal to ics_vjp up to
  * round-off, and the exact transpose of ics_jvp's map.  Covers the inviscid
  * residual with every reconstruction (upwind, the TVD limitedSchemes,
  * linearUpwind with cellLimited gradients), all three flux schemes, the
