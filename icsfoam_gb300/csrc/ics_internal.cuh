@@ -336,7 +336,20 @@ struct Handle {
   double* xblk = nullptr;  // [nnz][25]
   long long xnnz = 0;
   int xncol = 0;
-  bool haveExact = false;
+  // whether xblk holds the exact Jacobian at the current state, and how many
+  // ics_vjp calls at this state the reverse chain has served instead; a
+  // change of state (haveExact = false) restarts the count
+  struct ExactState {
+    bool have = false;
+    int served = 0;
+    ExactState& operator=(bool b) {
+      have = b;
+      served = 0;
+      return *this;
+    }
+    operator bool() const { return have; }
+  };
+  ExactState haveExact;
   // passive scalar transport: s, rhoS (+ old levels) [N], boundary s [B],
   // per-patch BC (fixed flag, value), face terms and the 1x1-block matrix
   bool scalarOn = false;

@@ -393,13 +393,16 @@ int ics_jvp(ics_handle h, const double* v, double* Jv, int32_t device);
  * colours (products = 5 x colours).  Valid until the state, the boundary
  * values or the configuration change.                                        */
 int ics_assemble_exact_jacobian(ics_handle h, int64_t* nnz_blocks, int32_t* n_colours);
-/* The assembled exact Jacobian in CSR form (host arrays): row_ptr
+/* The assembled exact Jacobian in CSR form (host arrays; assembled here when
+ * only ics_vjp was called at this state): row_ptr
  * [n_cells+1], cols [nnz] increasing within a row, blocks [nnz][5][5] with
  * blocks[j][i][k] = d(R V)_i of the row cell / d(W_k) of cols[j].  Any
  * pointer may be NULL.  ICS_ERR_STATE when not assembled at this state.    */
 int ics_get_exact_jacobian(ics_handle h, int32_t* row_ptr, int32_t* cols, double* blocks);
-/* Vector-Jacobian product JTu = (d(R V)/dW)^T u with the exact Jacobian,
- * assembled first when the state changed.  Pointers as in ics_jvp.         */
+/* Vector-Jacobian product JTu = (d(R V)/dW)^T u with the exact Jacobian: the
+ * assembled one when it is there, else, where ics_vjp_recompute covers the
+ * case, its reverse chain (equal up to round-off) for the first sixteen calls
+ * at a state, and an assembly after those.  Pointers as in ics_jvp.         */
 int ics_vjp(ics_handle h, const double* u, double* JTu, int32_t device);
 /* The same vector-Jacobian product by reverse mode, storing no Jacobian:
  * the face and cell maps of the residual are transposed in reverse order and

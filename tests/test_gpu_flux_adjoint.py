@@ -42,3 +42,23 @@ def test_flux_adjoints_in_a_moving_frame(gpu_binding, flux):
     h = open_case(gpu_binding, w)
     h.set_mrf(MRF.frame_fields(w.mesh, *w.mrf), 0)
     _transpose(h, h.get_state()["W"])
+
+
+def test_vjp_before_and_after_the_exact_jacobian(gpu_binding):
+    """ics_vjp serves a new state's first calls by the reverse chain: they equal
+    the products with the assembled Jacobian (1e-10 of the largest entry, the
+    bound of the two routes), and the Jacobian is there when it is asked for."""
+    w = perturb(cases.bump_channel(9, 5, 3, ordering_mode="colour"))
+    h = open_case(gpu_binding, w)
+    u = np.random.default_rng(6).standard_normal((w.mesh.n_cells, 5))
+    first = h.vjp(u)
+    ptr, cols, blocks = h.get_exact_jacobian()
+    rows = np.repeat(np.arange(w.mesh.n_cells), np.diff(ptr))
+    dense = np.zeros((w.mesh.n_cells, 5))
+    np.add.at(dense, cols, np.einsum("jik,ji->jk", blocks, u[rows]))
+    scale = np.abs(dense).max(axis=0)
+    assert (np.abs(first - dense) <= 1e-10 * scale).all()
+    h.set_conservative(h.get_state()["W"])  # a new state: the count starts again
+    calls = [h.vjp(u) for _ in range(18)]   # beyond the calls the reverse chain serves
+    assert all((np.abs(c - dense) <= 1e-10 * scale).all() for c in calls)
+    assert np.array_equal(calls[16], calls[17])
