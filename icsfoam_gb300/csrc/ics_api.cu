@@ -99,7 +99,7 @@ void free_all(Handle& h) {
   void* ptrs[] = {m.own, m.nei, m.Sf, m.magSf, m.w, m.nodc, m.dOwn, m.dNei, m.dCC, m.nf, m.bnf, m.C, m.V,
                   m.bcell, m.bpatch, m.bSf, m.bmagSf, m.bdOwn, m.bdc, m.patches, m.cptr, m.cface, m.bptr,
                   m.bface, m.slot_base, m.scol, m.sface, m.nlow, m.nslot, m.fl_cells, m.rl_cells, m.fl_lptr,
-                  m.rl_lptr, m.sweep_pad, m.sweep_ticket, m.sw_fwd, m.sw_rev, h.W, h.W0, h.W00, h.Wprev, h.prim, h.pB, h.TB, h.UB, h.phiB, h.pseudoCo, h.rPDT,
+                  m.rl_lptr, m.sweep_pad, m.sweep_ticket, m.sw_fwd, m.sw_rev, m.chain, h.W, h.W0, h.W00, h.Wprev, h.prim, h.pB, h.TB, h.UB, h.phiB, h.pseudoCo, h.rPDT,
                   h.ddtCoeff, h.q, h.bq, h.clin, h.grad, h.fflux, h.frec, h.flam, h.bjac, h.src, h.vcell,
                   h.fvisc, h.vsf2, h.vjac, m.dc, m.Dhb, m.mrfU, m.mrfOm, m.mrfBU, m.mrfBIn, m.plagMode, m.plagP, m.bpartner, m.bw, m.bdelta, m.bdNei,
                   m.bnodc, m.cyc_face, m.cyc_row, m.cyc_ptr, h.cblk, h.vjslotbuf, h.vjcellbuf, h.cfrec, h.tW, h.tprim, h.tq, h.tgrad, h.tflux, h.tvc, h.tfv, h.tv,
@@ -480,6 +480,12 @@ void build_mesh(Handle& h, const ics_mesh_desc* d) {
     m.nsw_rev = (int)(sr.size() / SWEEP_TICKET);
     m.sw_fwd = upload(sf);
     m.sw_rev = upload(sr);
+    // one unbroken chain: every row couples to the one before and the one
+    // after, and to no other (a break would let a non-finite value of one
+    // part reach the next through the zero products across it)
+    bool chain = F == N - 1;
+    for (int f = 0; f < F && chain; ++f) chain = d->neighbour[f] == d->owner[f] + 1;
+    if (chain) m.chain = dalloc<double>(chain_table_words(N));
   }
   m.sweep_ticket = dalloc<unsigned int>(2);
   m.rl_lptr = upload(m.rl_ptr);

@@ -112,6 +112,8 @@ struct DevMesh {
   int* sw_fwd = nullptr;
   int* sw_rev = nullptr;
   int nsw_fwd = 0, nsw_rev = 0;      // tickets
+  // LU-SGS of a chain (k_chain.cu): its products per matrix; nullptr elsewhere
+  double* chain = nullptr;
   bool fuse_last = false;            // last forward level == first reverse level (same rows)
   // Harmonic Balance: nInst stacked instances of Nc cells (instance-major),
   // coupled through the spectral operator Dhb [nInst][nInst]
@@ -455,6 +457,12 @@ void free_cases(Handle& h);
 int gmres_cases(Handle& h, std::vector<int>& caseStatus);
 void case_l2(Handle& h);
 void case_upload_ser(Handle& h);
+
+// LU-SGS of a chain (k_chain.cu; h.m.chain set): the tables of the assembled
+// matrix, and r <- both sweeps of r
+size_t chain_table_words(int N);
+void chain_setup(Handle& h);
+void chain_sweeps(Handle& h, void* r);
 
 // linear algebra: precision-dispatched (mixed = FP32 blocks and vectors)
 void spmv(Handle& h, const void* x, void* y);

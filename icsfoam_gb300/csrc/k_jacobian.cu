@@ -602,6 +602,7 @@ void launch_jacobian(Handle& h) {
                                                                            status));
   }
   ICS_CUDA(cudaGetLastError());
+  if (h.m.chain) chain_setup(h);
   h.jacPrecision = prec(h);
 }
 

@@ -1163,6 +1163,10 @@ static void lusgs_t(Handle& h, TV* r, const TB* blkIn = nullptr, const TB* rDIn 
   const DevMesh& m = h.m;
   const TB* blk = blkIn ? blkIn : (const TB*)h.blk;
   const TB* rD = rDIn ? rDIn : (const TB*)h.rD;
+  if (m.chain && !blkIn) {
+    chain_sweeps(h, r);
+    return;
+  }
   // many levels: one sync-free launch per sweep
   if (m.sw_fwd) {
     cudaStream_t st = h.stream;

@@ -27,6 +27,12 @@ SHAPES = {
     "levels_33": lambda: cases.bump_channel(33, 33, 1, ordering_mode="natural", second_order=False),
     "box_rcm_5": lambda: cases.random_box(5, ordering_mode="rcm"),
     "box_rcm_11": lambda: cases.random_box(11, ordering_mode="rcm"),
+    # chains: fewer rows than chunks, one row per chunk, a short last chunk
+    "chain_3": lambda: cases.shock_tube(3),
+    "chain_37": lambda: cases.shock_tube(37),
+    "chain_128": lambda: cases.shock_tube(128),
+    "chain_129": lambda: cases.shock_tube(129),
+    "chain_1000": lambda: cases.shock_tube(1000),
     # two colours on a few cells: level launches and the fused operator
     "two_colours_2x2x1": lambda: cases.bump_channel(2, 2, 1, ordering_mode="colour", second_order=False),
     "two_colours_9x5x3": lambda: cases.bump_channel(9, 5, 3, ordering_mode="colour", second_order=False),
