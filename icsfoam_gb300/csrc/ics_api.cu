@@ -107,7 +107,7 @@ void free_all(Handle& h) {
                   h.ss, h.ssB, h.srhoS, h.srhoS0, h.srhoS00, h.sgrad, h.sgradL, h.sface, h.sblk, h.sdg, h.srD,
                   h.ssrc, h.sFixed, h.sValue,
                   h.blk, h.dg,
-                  h.dginv, h.rD, h.kv, h.kw, h.kx, h.kb, h.kt, h.dW, h.partials, h.counter, h.ks, h.scratch,
+                  h.dginv, h.rD, h.kv, h.kw, h.kx, h.kb, h.kt, h.dW, h.partials, h.counter, h.ks, h.colSlots, h.scratch,
                   h.ibuf};
   drop_graphs(h);
   free_exact(h);
@@ -203,7 +203,7 @@ void ensure_workspace(Handle& h) {
     h.dg = dalloc<char>((size_t)h.m.nslices * 25 * 32 * eb);
     h.dginv = dalloc<char>((size_t)h.m.nslices * 25 * 32 * eb);
     h.rD = dalloc<char>((size_t)h.m.N * eb);
-    h.kw = dalloc<char>(n5 * eb);
+    h.kw = dalloc<char>(kstride(h) * eb);  // whole 16-byte chunks
     h.kx = dalloc<char>(n5 * eb);
     h.kb = dalloc<char>(n5 * eb);
     h.kt = dalloc<char>(n5 * eb);
@@ -522,6 +522,7 @@ void alloc_state(Handle& h) {
   h.partials = dalloc<double>((size_t)REDUCE_BLOCKS * 16);
   h.counter = dalloc<unsigned int>(MAX_INST + 4);
   h.ks = dalloc<KrylovScalars>(1);
+  h.colSlots = dalloc<double>(column_slot_words());
   ICS_CUDA(cudaMallocHost(&h.ksHost, sizeof(KrylovScalars)));
   h.scratch = dalloc<double>(5ull * N + 8);
   h.ibuf = dalloc<int>((size_t)N + 8);
@@ -807,6 +808,7 @@ int ics_create(const ics_mesh_desc* mesh, const ics_config* cfg, ics_handle* out
   h.m.limWiden = 1.0 / cfg->limiter_coeff - 1.0;
   st = guard(hh, [&](Handle& hd) {
     ICS_CUDA(cudaGetDevice(&hd.device));
+    ICS_CUDA(cudaDeviceGetAttribute(&hd.sms, cudaDevAttrMultiProcessorCount, hd.device));
     ICS_CUDA(cudaStreamCreateWithFlags(&hd.stream, cudaStreamNonBlocking));
     build_mesh(hd, mesh);
     alloc_state(hd);

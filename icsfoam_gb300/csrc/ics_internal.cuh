@@ -45,7 +45,7 @@ constexpr int MAX_INST = ICS_MAX_INSTANCES;  // Harmonic Balance instances
 struct KrylovScalars {
   double H[MAX_DIRS * MAX_DIRS];
   double c[MAX_DIRS], s[MAX_DIRS], bh[MAX_DIRS + 1], y[MAX_DIRS];
-  double beta;            // norm used to scale the next Krylov vector
+  double nrm2[MAX_DIRS];  // |w|^2 after the Gram-Schmidt of each direction
   double red[16];         // reduction results
   double avg[5 * MAX_INST];  // per-instance field averages of W
   double nfr[8 * MAX_INST];  // per instance: norm-factor sums (rho, rhoE, rhoU), |b| per equation
@@ -295,6 +295,8 @@ struct Handle {
   unsigned int* counter = nullptr;
   KrylovScalars* ks = nullptr;  // device
   KrylovScalars* ksHost = nullptr;  // pinned mirror
+  double* colSlots = nullptr;   // partial sums of the Gram-Schmidt columns (k_column.cu)
+  int sms = 0;                  // multiprocessors of the device
   // host-side residual bookkeeping (setCoAndDeltaT.H, pseudotimeControl):
   // linear-solver initial residuals per instance and equation, [5*J + k]
   bool initResValid = false, prevResValid = false;
@@ -458,6 +460,13 @@ int gmres_cases(Handle& h, std::vector<int>& caseStatus);
 void case_l2(Handle& h);
 void case_upload_ser(Handle& h);
 
+// Gram-Schmidt columns of the GMRES cycles (k_column.cu): words of the blocks'
+// slots, their reset before a solve of m directions, and column dir (-1: the
+// cycle start) of vectors of n elements, basis stride vs
+size_t column_slot_words();
+void column_reset(Handle& h, int m);
+void krylov_column(Handle& h, bool fp32, long n, void* w, void* V, long vs, int dir, int m);
+
 // LU-SGS of a chain (k_chain.cu; h.m.chain set): the tables of the assembled
 // matrix, and r <- both sweeps of r
 size_t chain_table_words(int N);
@@ -481,8 +490,9 @@ void sweep_probe(Handle& h, const int* order, int tickets, int spin_limit);
 void from_vec(Handle& h, const void* src, double* dst); // Krylov type -> FP64
 
 inline int prec(const Handle& h) { return h.cfg.c.precision; }
-// w = M^-1 A (x / beta) with v = x / beta stored in vout, by the fused LU-SGS
-// operator passes; false (nothing launched) where they do not apply
+// w = M^-1 A x by the fused LU-SGS operator passes, x scaled by the reciprocal
+// norm of each row's stacked case and stored in vout when that is given; false
+// (nothing launched) where they do not apply
 bool fused_operator(Handle& h, const void* x, void* w, void* vout);
 // element stride between consecutive Krylov basis vectors (5N rounded up to 64)
 inline size_t kstride(const Handle& h) { return ((5ull * h.m.N + 63) / 64) * 64; }

@@ -20,6 +20,7 @@
 #include "blocks.cuh"
 #include "hb.cuh"
 #include "ics_internal.cuh"
+#include "krylov.cuh"
 
 namespace ics {
 
@@ -83,46 +84,6 @@ __device__ __forceinline__ bool reduce_finish(double (&v)[NV], double* __restric
 }
 
 constexpr int RB = 256;  // threads per reduction block
-
-// MGS steps stream 3 Krylov vectors of which two are L2-resident, so they are
-// bound by latency and the reduction tail rather than by HBM: 4 blocks per SM
-// (608 on 152 SMs) measured 11% faster than 8 per SM (sweep of 304-1216);
-// the default of Handle::tuneMgsBlocks, which the autotuner may change.
-constexpr int MGS_CHUNKS = 2;
-
-// 16-byte vector of the Krylov element type
-template <typename TV>
-struct V16;
-template <>
-struct V16<float> {
-  using T = float4;
-  static constexpr int n = 4;
-  __device__ static float get(const T& v, int k) { return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w; }
-};
-template <>
-struct V16<double> {
-  using T = double2;
-  static constexpr int n = 2;
-  __device__ static double get(const T& v, int k) { return k == 0 ? v.x : v.y; }
-};
-
-__device__ __forceinline__ void axpy16(float4& x, float h, const float4& p) {
-  x.x -= h * p.x;
-  x.y -= h * p.y;
-  x.z -= h * p.z;
-  x.w -= h * p.w;
-}
-__device__ __forceinline__ void axpy16(double2& x, double h, const double2& p) {
-  x.x -= h * p.x;
-  x.y -= h * p.y;
-}
-// Per-thread dot accumulation stays in the Krylov element type (a thread
-// sums a few dozen products); FP64 conversions on GB300 run on the slow
-// FP64 pipe, so the FP32 path converts once per thread, not per product.
-__device__ __forceinline__ float dot16(const float4& a, const float4& b) {
-  return a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w;
-}
-__device__ __forceinline__ double dot16(const double2& a, const double2& b) { return a.x * b.x + a.y * b.y; }
 
 // ------------------------------------------------------------------- spmv
 template <typename TB, typename TV>
@@ -215,38 +176,31 @@ __global__ void __launch_bounds__(128) k_cyc_mv(DevMesh m, const TB* __restrict_
 //                          w_c = rD_c r'   (forward + fused first reverse)
 //   pass 3 (level-0 rows): the reverse sweep, as k_lusgs_level MODE 1.
 // Same arithmetic as the separate kernels up to the order of the sums.
-// SCALED: x is the unnormalised Krylov vector; the kernels use x * (1/beta)
-// (the next basis vector) and store it in vout for their own rows, which
-// removes the separate normalisation pass.  One reciprocal per thread: a
+// SCALED (stacked cases): x is the unnormalised Krylov vector; the kernels use
+// x * (1/beta) (the next basis vector) and store it in vout for their own rows,
+// which removes the separate normalisation pass.  One reciprocal per thread: a
 // division per gathered element would make the FP64 path ALU-bound.
 template <bool SCALED, typename TV>
 __device__ __forceinline__ TV ldx(const TV* __restrict__ x, size_t i, TV rbeta) {
   return SCALED ? x[i] * rbeta : x[i];
 }
+// the reciprocal norm of row c's stacked case
 template <typename TV>
-__device__ __forceinline__ TV krylov_rbeta(const KrylovScalars* ks) {
-  return ks && ks->status == 0 ? TV(1.0 / ks->beta) : TV(1);
-}
-// the reciprocal norm of row c's system: its stacked case's, else the handle's
-template <typename TV>
-__device__ __forceinline__ TV row_rbeta(const DevMesh& m, int c, const KrylovScalars* ks) {
-  if (m.caseBeta) {
-    const int k = m.caseOf[c];
-    return m.caseActive[k] && m.caseStatus[k] == 0 ? TV(1.0 / m.caseBeta[k]) : TV(1);
-  }
-  return krylov_rbeta<TV>(ks);
+__device__ __forceinline__ TV row_rbeta(const DevMesh& m, int c) {
+  const int k = m.caseOf[c];
+  return m.caseActive[k] && m.caseStatus[k] == 0 ? TV(1.0 / m.caseBeta[k]) : TV(1);
 }
 
 template <typename TB, typename TV, int MINB = 1, int UNR = 1, bool SCALED = false>
 __global__ void __launch_bounds__(128, MINB) k_op_level0(DevMesh m, const TB* __restrict__ blk, const TB* __restrict__ dg,
                                                    const TV* __restrict__ x, TV* __restrict__ w,
                                                    const int* __restrict__ cells, int start, int count,
-                                                   const KrylovScalars* __restrict__ ks, TV* __restrict__ vout) {
+                                                   TV* __restrict__ vout) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   const int c = cells ? cells[start + i] : start + i;
   const int s = c >> 5, lane = c & 31;
-  const TV beta = SCALED ? row_rbeta<TV>(m, c, ks) : TV(1);  // reciprocal
+  const TV beta = SCALED ? row_rbeta<TV>(m, c) : TV(1);  // reciprocal
   TV xc[5], acc[5];
 #pragma unroll
   for (int k = 0; k < 5; ++k) xc[k] = ldx<SCALED>(x, 5 * (size_t)c + k, beta);
@@ -309,13 +263,12 @@ template <typename TB, typename TV, int MINB = 1, int UNR = 1, bool SCALED = fal
 __global__ void __launch_bounds__(128, MINB) k_op_level1(DevMesh m, const TB* __restrict__ blk, const TB* __restrict__ dg,
                                                    const TB* __restrict__ rD, const TV* __restrict__ x,
                                                    TV* __restrict__ w, const int* __restrict__ cells, int start,
-                                                   int count, const KrylovScalars* __restrict__ ks,
-                                                   TV* __restrict__ vout) {
+                                                   int count, TV* __restrict__ vout) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   const int c = cells ? cells[start + i] : start + i;
   const int s = c >> 5, lane = c & 31;
-  const TV beta = SCALED ? row_rbeta<TV>(m, c, ks) : TV(1);  // reciprocal
+  const TV beta = SCALED ? row_rbeta<TV>(m, c) : TV(1);  // reciprocal
   TV xc[5], acc[5], fw[5];
 #pragma unroll
   for (int k = 0; k < 5; ++k) {
@@ -855,121 +808,6 @@ __global__ void k_cast(long n, const TS* __restrict__ a, TD* __restrict__ b) {
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) b[i] = TD(a[i]);
 }
 
-// start of a cycle: beta = sqrt(sum), bh = (beta, 0...)
-__device__ __forceinline__ void dev_beta0(KrylovScalars* ks, int m) {
-  const double beta = sqrt(ks->red[0]);
-  ks->beta = beta;
-  for (int i = 0; i <= m; ++i) ks->bh[i] = 0.0;
-  ks->bh[0] = beta;
-  if (!(beta > 0.0)) ks->status = isfinite(beta) ? 2 : 4;
-}
-
-__device__ __forceinline__ void givens(double h, double beta, double& c, double& s) {
-  if (beta == 0) {
-    c = 1;
-    s = 0;
-  } else if (fabs(beta) > fabs(h)) {
-    const double tau = -h / beta;
-    s = 1.0 / sqrt(1.0 + tau * tau);
-    c = s * tau;
-  } else {
-    const double tau = -beta / h;
-    c = 1.0 / sqrt(1.0 + tau * tau);
-    s = c * tau;
-  }
-}
-
-// after MGS of direction i: H[j][i] for j <= i are in H, red[1] holds |w|^2;
-// rotate column i with the previous Givens rotations and make a new one
-// (gmres.C:1013-1027, rotation gmres.C:44-69)
-__device__ __forceinline__ void dev_hess(KrylovScalars* ks, int i, int m) {
-  if (ks->status) return;
-  double* H = ks->H;
-  const double beta = sqrt(ks->red[1]);
-  for (int j = 0; j < i; ++j) {
-    const double Hji = H[j * m + i];
-    H[j * m + i] = ks->c[j] * Hji - ks->s[j] * H[(j + 1) * m + i];
-    H[(j + 1) * m + i] = ks->s[j] * Hji + ks->c[j] * H[(j + 1) * m + i];
-  }
-  givens(H[i * m + i], beta, ks->c[i], ks->s[i]);
-  const double bhi = ks->bh[i];
-  ks->bh[i] = ks->c[i] * bhi - ks->s[i] * ks->bh[i + 1];
-  ks->bh[i + 1] = ks->s[i] * bhi + ks->c[i] * ks->bh[i + 1];
-  H[i * m + i] = ks->c[i] * H[i * m + i] - ks->s[i] * beta;
-  ks->beta = beta;
-}
-
-// w -= hprev * vprev (when vprev), then sum w.vnext (or w.w) -> out.
-// post = 1: the finishing thread also starts the cycle (dev_beta0);
-// post = 2: it also performs the Hessenberg update of direction i.
-template <typename TV>
-__global__ void __launch_bounds__(RB, 4) k_mgs(long n, TV* __restrict__ w, const TV* __restrict__ vprev,
-                                            const double* __restrict__ hprev, const TV* __restrict__ vnext,
-                                            const int* __restrict__ status, double* __restrict__ partials,
-                                            unsigned int* __restrict__ counter, double* __restrict__ out,
-                                            KrylovScalars* __restrict__ ks, int post, int dir, int m) {
-  double acc[1] = {0.0};
-  if (*status == 0) {
-    const TV h = vprev ? TV(*hprev) : TV(0);
-    using VT = typename V16<TV>::T;
-    constexpr int L = V16<TV>::n;
-    const long nv = n / L;  // 16-byte chunks (vectors start 256-byte aligned)
-    VT* w4 = reinterpret_cast<VT*>(w);
-    const VT* p4 = reinterpret_cast<const VT*>(vprev);
-    const VT* o4 = reinterpret_cast<const VT*>(vnext);
-    const long stride = (long)gridDim.x * blockDim.x;
-    TV tacc = TV(0);
-    // MGS_CHUNKS 16-byte chunks per thread and iteration, every load issued
-    // before the first use: the compiler's unrolled loop kept one chunk in
-    // flight at 32 registers (ncu: long-scoreboard stalls, 50% warps active);
-    // two chunks at <= 64 registers measured 6% faster per step
-    long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    for (; i + (MGS_CHUNKS - 1) * stride < nv; i += MGS_CHUNKS * stride) {
-      VT x[MGS_CHUNKS], pv[MGS_CHUNKS], ov[MGS_CHUNKS];
-#pragma unroll
-      for (int u = 0; u < MGS_CHUNKS; ++u) {
-        x[u] = w4[i + u * stride];
-        if (vprev) pv[u] = p4[i + u * stride];
-        if (vnext) ov[u] = o4[i + u * stride];
-      }
-#pragma unroll
-      for (int u = 0; u < MGS_CHUNKS; ++u) {
-        if (vprev) {
-          axpy16(x[u], h, pv[u]);
-          w4[i + u * stride] = x[u];
-        }
-        tacc += dot16(x[u], vnext ? ov[u] : x[u]);
-      }
-    }
-    for (; i < nv; i += stride) {
-      VT x = w4[i];
-      if (vprev) {
-        axpy16(x, h, p4[i]);
-        w4[i] = x;
-      }
-      tacc += dot16(x, vnext ? o4[i] : x);
-    }
-    for (long i = nv * L + blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += stride) {
-      TV x = w[i];
-      if (vprev) {
-        x = x - h * vprev[i];
-        w[i] = x;
-      }
-      const TV o = vnext ? vnext[i] : x;
-      tacc += x * o;
-    }
-    acc[0] = double(tacc);
-  }
-  if (reduce_finish<1>(acc, partials, counter, out)) {
-    if (post == 1)
-      dev_beta0(ks, m);
-    else if (post == 2)
-      dev_hess(ks, dir, m);
-  }
-}
-
-__device__ __forceinline__ float4 div16(float4 x, float b) { return make_float4(x.x / b, x.y / b, x.z / b, x.w / b); }
-__device__ __forceinline__ double2 div16(double2 x, double b) { return make_double2(x.x / b, x.y / b); }
 __device__ __forceinline__ void addmul16(float4& a, float y, const float4& v) {
   a.x += y * v.x;
   a.y += y * v.y;
@@ -981,24 +819,10 @@ __device__ __forceinline__ void addmul16(double2& a, double y, const double2& v)
   a.y += y * v.y;
 }
 
-// v = w / beta (gmres.C: sV = sTmp/beta)
-template <typename TV>
-__global__ void k_scale(long n, const TV* __restrict__ w, TV* __restrict__ v, const KrylovScalars* __restrict__ ks) {
-  if (ks->status) return;
-  const TV beta = TV(ks->beta);
-  using VT = typename V16<TV>::T;
-  constexpr int L = V16<TV>::n;
-  const long nv = n / L;
-  const long stride = (long)gridDim.x * blockDim.x;
-  const VT* w4 = reinterpret_cast<const VT*>(w);
-  VT* v4 = reinterpret_cast<VT*>(v);
-#pragma unroll 4
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < nv; i += stride) v4[i] = div16(w4[i], beta);
-  for (long i = nv * L + blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += stride) v[i] = w[i] / beta;
-}
-
+// the last direction's Givens rotation, then H y = bh
 __global__ void k_backsub(KrylovScalars* ks, int m) {
   if (ks->status) return;
+  dev_hess(ks, m - 1, m);
   for (int i = m - 1; i >= 0; --i) {
     double sum = ks->bh[i];
     for (int j = i + 1; j < m; ++j) sum -= ks->H[i * m + j] * ks->y[j];
@@ -1221,8 +1045,8 @@ static bool fused_op_available(const Handle& h) {
          m.ncyc == 0;
 }
 
-// vout != nullptr: x is unnormalised; v = x / beta is stored in vout and
-// w = M^-1 A v (w must then differ from x)
+// vout != nullptr (stacked cases): x is unnormalised; v = x / beta is stored in
+// vout and w = M^-1 A v (w must then differ from x)
 template <typename TB, typename TV>
 static bool fused_op_t(Handle& h, const TV* x, TV* w, TV* vout = nullptr) {
   const DevMesh& m = h.m;
@@ -1247,22 +1071,21 @@ static bool fused_op_t(Handle& h, const TV* x, TV* w, TV* vout = nullptr) {
   // in flight or the compiler's register choice (72-80), and 10 or 12 blocks
   // (51 / 40 registers, the latter spilling) were not faster; FP64 would spill
   constexpr int OPB = sizeof(TB) == 4 ? 8 : 1;
-  const KrylovScalars* ks = h.ks;
   if (n0) {
     if (vout)
       ICS_LAUNCH(h, ICS_K_OP0, k_op_level0<TB, TV, OPB, 1, true><<<grid_for(n0, 128), 128, 0, h.stream>>>(
-                                   m, blk, dg, x, w, c0, s0, n0, ks, vout));
+                                   m, blk, dg, x, w, c0, s0, n0, vout));
     else
       ICS_LAUNCH(h, ICS_K_OP0, k_op_level0<TB, TV, OPB, 1><<<grid_for(n0, 128), 128, 0, h.stream>>>(
-                                   m, blk, dg, x, w, c0, s0, n0, nullptr, nullptr));
+                                   m, blk, dg, x, w, c0, s0, n0, nullptr));
   }
   if (n1) {
     if (vout)
       ICS_LAUNCH(h, ICS_K_OP1, k_op_level1<TB, TV, OPB, 1, true><<<grid_for(n1, 128), 128, 0, h.stream>>>(
-                                   m, blk, dg, rD, x, w, c1, s1, n1, ks, vout));
+                                   m, blk, dg, rD, x, w, c1, s1, n1, vout));
     else
       ICS_LAUNCH(h, ICS_K_OP1, k_op_level1<TB, TV, OPB, 1><<<grid_for(n1, 128), 128, 0, h.stream>>>(
-                                   m, blk, dg, rD, x, w, c1, s1, n1, nullptr, nullptr));
+                                   m, blk, dg, rD, x, w, c1, s1, n1, nullptr));
   }
   // reverse level 1 = forward level 0 rows
   const int a = m.rl_ptr[1], cnt = m.rl_ptr[2] - a;
@@ -1523,9 +1346,9 @@ static int gmres_t(Handle& h, ResIO& p) {
   TV* w = (TV*)h.kw;
   TV* x = (TV*)h.kx;
   TV* t = (TV*)h.kt;
-  double* red = ks->red;
   std::vector<double> nf;
   norm_factors_t<TB, TV>(h, nf, p);
+  column_reset(h, m);
   // r = b, x = 0
   ICS_CUDA(cudaMemsetAsync(x, 0, n5 * sizeof(TV), st));
   to_vec(h, h.src, w);
@@ -1534,35 +1357,14 @@ static int gmres_t(Handle& h, ResIO& p) {
   // same launch sequence can be captured once and replayed per cycle
   auto cycle = [&]() {
     precondition_t<TB, TV>(h, w);
-    ICS_LAUNCH(h, ICS_K_MGS,
-               k_mgs<TV><<<h.tuneMgsBlocks, RB, 0, st>>>(n5, w, nullptr, nullptr, nullptr, &ks->status, h.partials,
-                                                       h.counter, red, ks, 1, 0, m));
-    // with the fused operator the step's normalisation is folded into it and
-    // the unnormalised vector alternates between two buffers (w, t); the
-    // cycle's residual goes back to w
-    const bool fused = fused_op_available<TB, TV>(h);
-    TV* wb[2] = {w, t};
-    TV* wc = w;
+    krylov_column(h, sizeof(TV) == 4, n5, w, V, vs, -1, m);
     for (int i = 0; i < m; ++i) {
-      TV* vi = V + (size_t)i * vs;
-      if (fused) {
-        fused_op_t<TB, TV>(h, wb[i & 1], wb[(i + 1) & 1], vi);
-        wc = wb[(i + 1) & 1];
-      } else {
-        ICS_LAUNCH(h, ICS_K_VECTOR, k_scale<TV><<<REDUCE_BLOCKS, RB, 0, st>>>(n5, wc, vi, ks));
-        spmv_t<TB, TV>(h, vi, wc);
-        precondition_t<TB, TV>(h, wc);
+      const TV* vi = V + (size_t)i * vs;
+      if (!fused_op_t<TB, TV>(h, vi, w)) {
+        spmv_t<TB, TV>(h, vi, w);
+        precondition_t<TB, TV>(h, w);
       }
-      for (int j = 0; j <= i; ++j) {
-        const TV* vprev = j > 0 ? V + (size_t)(j - 1) * vs : nullptr;
-        const double* hprev = j > 0 ? &ks->H[(j - 1) * m + i] : nullptr;
-        ICS_LAUNCH(h, ICS_K_MGS,
-                   k_mgs<TV><<<h.tuneMgsBlocks, RB, 0, st>>>(n5, wc, vprev, hprev, V + (size_t)j * vs, &ks->status,
-                                                           h.partials, h.counter, &ks->H[j * m + i], ks, 0, i, m));
-      }
-      ICS_LAUNCH(h, ICS_K_MGS,
-                 k_mgs<TV><<<h.tuneMgsBlocks, RB, 0, st>>>(n5, wc, vi, &ks->H[i * m + i], nullptr, &ks->status,
-                                                         h.partials, h.counter, &red[1], ks, 2, i, m));
+      krylov_column(h, sizeof(TV) == 4, n5, w, V, vs, i, m);
     }
     ICS_LAUNCH(h, ICS_K_SCALAR, k_backsub<<<1, 1, 0, st>>>(ks, m));
     ICS_LAUNCH(h, ICS_K_VECTOR, k_xupdate<TV><<<REDUCE_BLOCKS, RB, 0, st>>>(n5, x, V, ks, m, vs));
@@ -1642,13 +1444,12 @@ int gmres_solve(Handle& h, ics_solver_perf* perf, std::vector<double>& initRes) 
 // ------------------------------------------------------------ autotuner
 // Times the Krylov-side launch choices on the handle's assembled system with
 // CUDA events on its stream (median of three runs each, after a warm-up):
-// the MGS step's grid, and the fused LU-SGS operator against SpMV plus
-// separate sweeps.  Sets the fastest; the arithmetic of every choice is the
+// the fused LU-SGS operator against SpMV plus separate sweeps, and the rows
+// per thread of the reverse sweep.  Sets the fastest; the arithmetic of every choice is the
 // same up to the order of the sums.
 template <typename TB, typename TV>
 static void autotune_linalg_t(Handle& h, std::vector<std::pair<std::string, double>>& log) {
   cudaStream_t st = h.stream;
-  const long n5 = 5L * h.m.N;
   TV* V = (TV*)h.kv;
   TV* w = (TV*)h.kw;
   TV* t = (TV*)h.kt;
@@ -1670,32 +1471,9 @@ static void autotune_linalg_t(Handle& h, std::vector<std::pair<std::string, doub
     std::sort(best, best + 5);
     return best[2];
   };
-  // operands: w = b, v_0 = b (a step of the cycle's Gram-Schmidt)
-  to_vec(h, h.src, w);
+  // operand: v_0 = b
   to_vec(h, h.src, V);
-  KrylovScalars* ks = h.ks;
-  const int m = h.cfg.c.n_directions;
-  int bestBlocks = h.tuneMgsBlocks;
-  double bestMs = 1e300;
-  // the cycle's steps: w -= h v_{j-1}, then w . v_j over the m basis vectors
-  // in turn (their working set exceeds L2 as in the cycle; one launch alone
-  // is too short to time); h = 0 keeps w
-  const long vs = (long)kstride(h);
-  for (int j = 1; j < m; ++j) to_vec(h, h.src, V + (size_t)j * vs);
-  ICS_CUDA(cudaMemsetAsync(&ks->red[15], 0, sizeof(double), st));
-  ICS_CUDA(cudaMemsetAsync(&ks->status, 0, sizeof(int), st));
-  for (int blocks : {152, 304, 456, 608}) {
-    const double ms = timed([&]() {
-      for (int j = 0; j < m; ++j)
-        k_mgs<TV><<<blocks, RB, 0, st>>>(n5, w, V + (size_t)((j + m - 1) % m) * vs, &ks->red[15],
-                                          V + (size_t)j * vs, &ks->status, h.partials, h.counter, &ks->red[14], ks,
-                                          0, 0, m);
-    });
-    log.emplace_back("mgs_blocks_" + std::to_string(blocks), ms);
-    if (ms < bestMs) bestMs = ms, bestBlocks = blocks;
-  }
-  h.tuneMgsBlocks = bestBlocks;
-  ICS_CUDA(cudaMemsetAsync(&ks->status, 0, sizeof(int), st));
+  ICS_CUDA(cudaMemsetAsync(&h.ks->status, 0, sizeof(int), st));
   h.tuneFused = 1;
   if (fused_op_available<TB, TV>(h)) {
     const double fused = timed([&]() { fused_op_t<TB, TV>(h, V, w); });
@@ -1941,29 +1719,18 @@ int scalar_gmres(Handle& h, double* dx, ics_solver_perf* perf) {
   const double nf = hv[0] + VSMALL;
   memset(perf, 0, sizeof(*perf));
   perf->init_res[0] = perf->final_res[0] = hv[1] / nf;
+  column_reset(h, m);
   ICS_CUDA(cudaMemsetAsync(dx, 0, N * sizeof(double), st));
   ICS_CUDA(cudaMemcpyAsync(w, h.ssrc, N * sizeof(double), cudaMemcpyDeviceToDevice, st));
   const ics_config& cf = h.cfg.c;
   int status = ICS_OK;
   while (true) {
     s_precondition(h, w);
-    ICS_LAUNCH(h, ICS_K_MGS, k_mgs<double><<<h.tuneMgsBlocks, RB, 0, st>>>(N, w, nullptr, nullptr, nullptr, &ks->status,
-                                                                       h.partials, h.counter, red, ks, 1, 0, m));
+    krylov_column(h, false, N, w, V, vs, -1, m);
     for (int i = 0; i < m; ++i) {
-      double* vi = V + (size_t)i * vs;
-      ICS_LAUNCH(h, ICS_K_VECTOR, k_scale<double><<<REDUCE_BLOCKS, RB, 0, st>>>(N, w, vi, ks));
-      s_spmv(h, vi, w);
+      s_spmv(h, V + (size_t)i * vs, w);
       s_precondition(h, w);
-      for (int j = 0; j <= i; ++j) {
-        const double* vprev = j > 0 ? V + (size_t)(j - 1) * vs : nullptr;
-        const double* hprev = j > 0 ? &ks->H[(j - 1) * m + i] : nullptr;
-        ICS_LAUNCH(h, ICS_K_MGS,
-                   k_mgs<double><<<h.tuneMgsBlocks, RB, 0, st>>>(N, w, vprev, hprev, V + (size_t)j * vs, &ks->status,
-                                                            h.partials, h.counter, &ks->H[j * m + i], ks, 0, i, m));
-      }
-      ICS_LAUNCH(h, ICS_K_MGS, k_mgs<double><<<h.tuneMgsBlocks, RB, 0, st>>>(N, w, vi, &ks->H[i * m + i], nullptr,
-                                                                         &ks->status, h.partials, h.counter, &red[1],
-                                                                         ks, 2, i, m));
+      krylov_column(h, false, N, w, V, vs, i, m);
     }
     ICS_LAUNCH(h, ICS_K_SCALAR, k_backsub<<<1, 1, 0, st>>>(ks, m));
     ICS_LAUNCH(h, ICS_K_VECTOR, k_xupdate<double><<<REDUCE_BLOCKS, RB, 0, st>>>(N, dx, V, ks, m, vs));
