@@ -51,10 +51,16 @@ struct SlotBlock<double> {
       y[i] = a;
     }
   }
-  template <typename TV>
-  __device__ __forceinline__ void mv2(TV g, const TV* xa, TV* ya, const TV* xb, TV* yb) const {
-    mv(g, xa, ya);
-    mv(g, xb, yb);
+  // acc += B x (SIGN 1) or acc -= B x (SIGN -1), one multiply-add per entry:
+  // an addition of its own costs as much of the FP64 pipe as a multiply-add
+  template <int SIGN, typename TV>
+  __device__ __forceinline__ void mac(TV, const TV* x, TV* acc) const {
+#pragma unroll
+    for (int j = 0; j < 5; ++j) {
+      const TV xj = SIGN > 0 ? x[j] : -x[j];
+#pragma unroll
+      for (int i = 0; i < 5; ++i) acc[i] += TV(w[5 * i + j]) * xj;
+    }
   }
   __device__ __forceinline__ double entry(double, int i, int j) const { return w[5 * i + j]; }
 };
@@ -77,12 +83,13 @@ struct SlotBlock<float> {
     Terms<TV> t(g, w);
     t.apply(g, x, y);
   }
-  // ya = B xa, yb = B xb with the per-block terms computed once
-  template <typename TV>
-  __device__ __forceinline__ void mv2(TV g, const TV* xa, TV* ya, const TV* xb, TV* yb) const {
-    Terms<TV> t(g, w);
-    t.apply(g, xa, ya);
-    t.apply(g, xb, yb);
+  // acc += B x (SIGN 1) or acc -= B x (SIGN -1)
+  template <int SIGN, typename TV>
+  __device__ __forceinline__ void mac(TV g, const TV* x, TV* acc) const {
+    TV y[5];
+    mv(g, x, y);
+#pragma unroll
+    for (int i = 0; i < 5; ++i) acc[i] += SIGN > 0 ? y[i] : -y[i];
   }
 
   // entry (i, j) of the convective part (matrix readback)
@@ -144,14 +151,14 @@ struct SlotBlock<float> {
   };
 };
 
-// y -= V x, V = the non-LF viscous laplacians at column cell col of slot
+// y -= SIGN V x, V = the non-LF viscous laplacians at column cell col of slot
 // (only when m.vjslot is set; TB is the block storage type)
-template <typename TB, typename TV>
+template <typename TB, int SIGN = 1, typename TV>
 __device__ __forceinline__ void vj_sub(const DevMesh& m, size_t slot, int lane, int col, const TV* x, TV* y) {
   const TB* vs = (const TB*)m.vjslot + slot * 2 * 32 + lane;
   const TB* vc = (const TB*)m.vjcell;
   const int N = m.N;
-  const TV mg = TV(vs[0]), ag = TV(vs[32]);
+  const TV mg = SIGN * TV(vs[0]), ag = SIGN * TV(vs[32]);
   const TV m0 = TV(vc[col]), m1 = TV(vc[N + col]), m2 = TV(vc[2 * N + col]);
   const TV ir = TV(vc[3 * N + col]), eR = TV(vc[4 * N + col]);
   y[1] -= mg * (m0 * x[0] + ir * x[1]);

@@ -109,15 +109,13 @@ __global__ void __launch_bounds__(128) k_spmv(DevMesh m, const TB* __restrict__ 
 #pragma unroll 1
   for (int t = 0; t < ns; ++t) {
     const int col = m.scol[(base + t) * 32 + lane];
-    TV xj[5], y[5];
+    TV xj[5];
 #pragma unroll
     for (int k = 0; k < 5; ++k) xj[k] = x[5 * col + k];
     SlotBlock<TB> Bk;
     Bk.load(blk, base + t, lane);
-    Bk.mv(g, xj, y);
-    if (m.vjslot) vj_sub<TB>(m, base + t, lane, col, xj, y);
-#pragma unroll
-    for (int i = 0; i < 5; ++i) acc[i] += y[i];
+    Bk.template mac<1>(g, xj, acc);
+    if (m.vjslot) vj_sub<TB>(m, base + t, lane, col, xj, acc);
   }
   if (m.nInst > 1 && hb_in_zone(m, c)) {
     // Harmonic Balance coupling blocks V D_JK I with the other instances
@@ -172,10 +170,15 @@ __global__ void __launch_bounds__(128) k_cyc_mv(DevMesh m, const TB* __restrict_
 // passes instead of SpMV + two sweeps, and the second-level rows read their
 // (lower) blocks once for both the product and the forward sweep:
 //   pass 1 (level-0 rows): w = (A x)_c
-//   pass 2 (level-1 rows): y = (A x)_c; r' = y - sum_lower L (rD w)_j;
+//   pass 2 (level-1 rows): r' = (A x)_c - sum_lower L (rD w)_j, summed as
+//                          D x_c + sum_lower L (x - rD w)_j;
 //                          w_c = rD_c r'   (forward + fused first reverse)
 //   pass 3 (level-0 rows): the reverse sweep, as k_lusgs_level MODE 1.
-// Same arithmetic as the separate kernels up to the order of the sums.
+// Same arithmetic as the separate kernels up to the order of the sums.  In
+// FP64 these passes are bound by the FP64 pipe, so their cost is their count
+// of operations: one product per slot in pass 2 (98k rows: 94 -> 45 us) and
+// products accumulated by multiply-adds (pass 1 52 -> 37, pass 3 45 -> 39 us);
+// the FP32 passes are bound by HBM and did not change.
 // SCALED (stacked cases): x is the unnormalised Krylov vector; the kernels use
 // x * (1/beta) (the next basis vector) and store it in vout for their own rows,
 // which removes the separate normalisation pass.  One reciprocal per thread: a
@@ -229,7 +232,7 @@ __global__ void __launch_bounds__(128, MINB) k_op_level0(DevMesh m, const TB* __
 #pragma unroll UNR
   for (int t = 0; t < ns; ++t) {
     const int col = colA;
-    TV xj[5], y[5];
+    TV xj[5];
 #pragma unroll
     for (int k = 0; k < 5; ++k) xj[k] = xn[k];
     colA = colB;
@@ -239,10 +242,8 @@ __global__ void __launch_bounds__(128, MINB) k_op_level0(DevMesh m, const TB* __
       for (int k = 0; k < 5; ++k) xn[k] = ldx<SCALED>(x, 5 * (size_t)colA + k, beta);
     SlotBlock<TB> Bk;
     Bk.load(blk, base + t, lane);
-    Bk.mv(g, xj, y);
-    if (m.vjslot) vj_sub<TB>(m, base + t, lane, col, xj, y);
-#pragma unroll
-    for (int r = 0; r < 5; ++r) acc[r] += y[r];
+    Bk.template mac<1>(g, xj, acc);
+    if (m.vjslot) vj_sub<TB>(m, base + t, lane, col, xj, acc);
   }
   if (m.nInst > 1 && hb_in_zone(m, c)) {
     const int J = c / m.Nc, cl = c - J * m.Nc;
@@ -269,12 +270,9 @@ __global__ void __launch_bounds__(128, MINB) k_op_level1(DevMesh m, const TB* __
   const int c = cells ? cells[start + i] : start + i;
   const int s = c >> 5, lane = c & 31;
   const TV beta = SCALED ? row_rbeta<TV>(m, c) : TV(1);  // reciprocal
-  TV xc[5], acc[5], fw[5];
+  TV xc[5], acc[5];
 #pragma unroll
-  for (int k = 0; k < 5; ++k) {
-    xc[k] = ldx<SCALED>(x, 5 * (size_t)c + k, beta);
-    fw[k] = TV(0);
-  }
+  for (int k = 0; k < 5; ++k) xc[k] = ldx<SCALED>(x, 5 * (size_t)c + k, beta);
   if (SCALED)
 #pragma unroll
     for (int k = 0; k < 5; ++k) vout[5 * c + k] = xc[k];
@@ -293,24 +291,14 @@ __global__ void __launch_bounds__(128, MINB) k_op_level1(DevMesh m, const TB* __
   for (int t = 0; t < ns; ++t) {
     const int col = m.scol[(base + t) * 32 + lane];
     const TV rj = TV(rD[col]);
-    TV xj[5], dj[5], ya[5], yb[5];
+    // the product's x_j and the sweep's rD w_j meet the same block: one product
+    TV xj[5];
 #pragma unroll
-    for (int k = 0; k < 5; ++k) {
-      xj[k] = ldx<SCALED>(x, 5 * (size_t)col + k, beta);
-      dj[k] = rj * w[5 * col + k];
-    }
+    for (int k = 0; k < 5; ++k) xj[k] = ldx<SCALED>(x, 5 * (size_t)col + k, beta) - rj * w[5 * col + k];
     SlotBlock<TB> Bk;
     Bk.load(blk, base + t, lane);
-    Bk.mv2(g, xj, ya, dj, yb);
-    if (m.vjslot) {
-      vj_sub<TB>(m, base + t, lane, col, xj, ya);
-      vj_sub<TB>(m, base + t, lane, col, dj, yb);
-    }
-#pragma unroll
-    for (int r = 0; r < 5; ++r) {
-      acc[r] += ya[r];
-      fw[r] += yb[r];
-    }
+    Bk.template mac<1>(g, xj, acc);
+    if (m.vjslot) vj_sub<TB>(m, base + t, lane, col, xj, acc);
   }
   if (m.nInst > 1 && hb_in_zone(m, c)) {
     const int J = c / m.Nc, cl = c - J * m.Nc;
@@ -325,7 +313,7 @@ __global__ void __launch_bounds__(128, MINB) k_op_level1(DevMesh m, const TB* __
   }
   const TV rc = TV(rD[c]);
 #pragma unroll
-  for (int k = 0; k < 5; ++k) w[5 * c + k] = rc * (acc[k] - fw[k]);
+  for (int k = 0; k < 5; ++k) w[5 * c + k] = rc * acc[k];
 }
 
 // ------------------------------------------------------------------ LU-SGS
@@ -345,15 +333,13 @@ __device__ __forceinline__ void lusgs_fwd_row(const DevMesh& m, const TB* __rest
   for (int t = 0; t < nl; ++t) {
     const int col = m.scol[(base + t) * 32 + lane];
     const TV rj = TV(rD[col]);
-    TV dj[5], y[5];
+    TV dj[5];
 #pragma unroll
     for (int k = 0; k < 5; ++k) dj[k] = rj * r[5 * col + k];
     SlotBlock<TB> Bk;
     Bk.load(blk, base + t, lane);
-    Bk.mv(g, dj, y);
-    if (m.vjslot) vj_sub<TB>(m, base + t, lane, col, dj, y);
-#pragma unroll
-    for (int i = 0; i < 5; ++i) acc[i] -= y[i];
+    Bk.template mac<-1>(g, dj, acc);
+    if (m.vjslot) vj_sub<TB, -1>(m, base + t, lane, col, dj, acc);
   }
   if (SCALE) {
     const TV rc = TV(rD[c]);
@@ -381,15 +367,13 @@ __device__ __forceinline__ void lusgs_rev_row(const DevMesh& m, const TB* __rest
 #pragma unroll 2
   for (int t = ns - 1; t >= nl; --t) {
     const int col = m.scol[(base + t) * 32 + lane];
-    TV dj[5], y[5];
+    TV dj[5];
 #pragma unroll
     for (int k = 0; k < 5; ++k) dj[k] = r[5 * col + k];
     SlotBlock<TB> Bk;
     Bk.load(blk, base + t, lane);
-    Bk.mv(g, dj, y);
-    if (m.vjslot) vj_sub<TB>(m, base + t, lane, col, dj, y);
-#pragma unroll
-    for (int i = 0; i < 5; ++i) acc[i] -= y[i];
+    Bk.template mac<-1>(g, dj, acc);
+    if (m.vjslot) vj_sub<TB, -1>(m, base + t, lane, col, dj, acc);
   }
   const TV rc = TV(rD[c]);
 #pragma unroll
@@ -420,7 +404,7 @@ __device__ __forceinline__ void lusgs_rev_row2(const DevMesh& m, const TB* __res
     const bool v0 = t0 >= nl0, v1 = t1 >= nl1;
     const int col0 = v0 ? m.scol[(b0 + t0) * 32 + l0] : c0;
     const int col1 = v1 ? m.scol[(b1 + t1) * 32 + l1] : c1;
-    TV d0[5], d1[5], y0[5], y1[5];
+    TV d0[5], d1[5];
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
       d0[k] = r[5 * col0 + k];
@@ -430,16 +414,12 @@ __device__ __forceinline__ void lusgs_rev_row2(const DevMesh& m, const TB* __res
     if (v0) B0.load(blk, b0 + t0, l0);
     if (v1) B1.load(blk, b1 + t1, l1);
     if (v0) {
-      B0.mv(g, d0, y0);
-      if (m.vjslot) vj_sub<TB>(m, b0 + t0, l0, col0, d0, y0);
-#pragma unroll
-      for (int i = 0; i < 5; ++i) a0[i] -= y0[i];
+      B0.template mac<-1>(g, d0, a0);
+      if (m.vjslot) vj_sub<TB, -1>(m, b0 + t0, l0, col0, d0, a0);
     }
     if (v1) {
-      B1.mv(g, d1, y1);
-      if (m.vjslot) vj_sub<TB>(m, b1 + t1, l1, col1, d1, y1);
-#pragma unroll
-      for (int i = 0; i < 5; ++i) a1[i] -= y1[i];
+      B1.template mac<-1>(g, d1, a1);
+      if (m.vjslot) vj_sub<TB, -1>(m, b1 + t1, l1, col1, d1, a1);
     }
   }
   const TV rc0 = TV(rD[c0]), rc1 = TV(rD[c1]);
@@ -498,8 +478,8 @@ __global__ void __launch_bounds__(128) k_lusgs_level(DevMesh m, const TB* __rest
 // neighbours' five words with relaxed loads until none is the sentinel.  One
 // L2 round trip per poll brings both the readiness and the values, the writer
 // needs no fence, and the polls of all prefetched neighbours are issued
-// together.  The arithmetic per row is that of lusgs_fwd_row / lusgs_rev_row,
-// so the result equals the level-by-level sweep bit for bit.  A wait that
+// together.  Per row the neighbours are subtracted in the order of
+// lusgs_fwd_row / lusgs_rev_row.  A wait that
 // exceeds the bound sets status bit 8, publishes zeros (so that its
 // dependents do not wait in turn) and goes on; waiting rows that see bit 8
 // give up too (the host reports ICS_ERR_TIMEOUT).
@@ -1271,15 +1251,13 @@ __global__ void __launch_bounds__(128) k_jacobi_sweep(DevMesh m, const TB* __res
   const TV g = TV(m.gamma);
   for (int t = 0; t < m.nslot[c]; ++t) {
     const int col = m.scol[(base + t) * 32 + lane];
-    TV xj[5], y[5];
+    TV xj[5];
 #pragma unroll
     for (int k = 0; k < 5; ++k) xj[k] = xo[5 * col + k];
     SlotBlock<TB> Bk;
     Bk.load(blk, base + t, lane);
-    Bk.mv(g, xj, y);
-    if (m.vjslot) vj_sub<TB>(m, base + t, lane, col, xj, y);
-#pragma unroll
-    for (int i = 0; i < 5; ++i) acc[i] += y[i];
+    Bk.template mac<1>(g, xj, acc);
+    if (m.vjslot) vj_sub<TB>(m, base + t, lane, col, xj, acc);
   }
   TV r[5];
 #pragma unroll
