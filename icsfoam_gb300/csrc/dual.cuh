@@ -104,6 +104,27 @@ template <typename Real>
 __device__ __forceinline__ Real omin(const Real& a, const Real& b) {
   return okey(a) <= okey(b) ? a : b;
 }
+// the larger of two values >= 0, a NaN second operand ignored as by fmax
+__device__ __forceinline__ double pmax(double a, double b) {
+  const long long ka = __double_as_longlong(a), kb = __double_as_longlong(b);
+  return kb > ka && kb <= 0x7ff0000000000000LL ? b : a;
+}
+// -x when neg: a sign-bit flip, where a product with +-1 would take the FP64 pipe
+__device__ __forceinline__ double flip(double x, bool neg) {
+  return __hiloint2double(__double2hiint(x) ^ (neg ? (int)0x80000000 : 0), __double2loint(x));
+}
+// order of two values >= 0 (either zero the same, a NaN above all)
+__device__ __forceinline__ long long mag(double x) { return __double_as_longlong(x) & 0x7fffffffffffffffLL; }
+__device__ __forceinline__ long long mag(const Dual& x) { return mag(x.v); }
+// -x without the FP64 pipe
+__device__ __forceinline__ double neg(double x) { return flip(x, true); }
+__device__ __forceinline__ Dual neg(const Dual& x) { return -x; }
+// x / b from the reciprocal r = fl(1/b): the product's remainder corrects it
+// to the rounding of a division, in 3 operations of the FP64 pipe against 10
+__device__ __forceinline__ double quot(double x, double b, double r) {
+  const double q = x * r;
+  return fma(fma(-q, b, x), r, q);
+}
 // x > c and x < c for a constant c
 template <typename Real>
 __device__ __forceinline__ bool ogt(const Real& x, double c) {

@@ -583,7 +583,7 @@ int do_residual(Handle& h, double* host_src) {
   if (h.cfg.c.viscous) {
     if (!h.vcell) {
       h.vcell = dalloc<double>(24ull * h.m.N);
-      h.fvisc = dalloc<double>(8ull * (h.m.F + h.m.B));
+      h.fvisc = dalloc<double>(4ull * (h.m.F + h.m.B));
       h.vsf2 = dalloc<double>((size_t)h.m.F + h.m.B);
       h.vjac = dalloc<double>(2ull * (h.m.F + h.m.B));
     }
@@ -1596,7 +1596,7 @@ void ensure_tangent(Handle& h) {
   h.tgrad = dal(3 * NQ * N * D);
   h.tflux = dal(5 * FB * D);
   h.tvc = dal(24 * N * D);
-  h.tfv = dal(8 * FB * D);
+  h.tfv = dal(4 * FB * D);
   h.tv = (double*)dal(10 * N * sizeof(double));
 }
 

@@ -271,7 +271,7 @@ struct Handle {
   double* src = nullptr;    // [N][5] source = R*V
   // viscous terms (allocated when the case is viscous)
   double* vcell = nullptr;  // [24][N] grad U, grad e, tauMC, mu, alphaEff, e
-  double* fvisc = nullptr;  // [8][F+B] lapU, divTau, divSig, lapE face terms
+  double* fvisc = nullptr;  // [4][F+B] viscous face terms (k_viscous.cu)
   double* vsf2 = nullptr;   // [F] LF viscous Jacobian coefficient
   double* vjac = nullptr;   // [2][F+B] non-LF viscous laplacian coefficients: internal and
                             // coupled faces (mu_f|S|) dc, (alpha_f|S|) dc; boundary mu_b, alpha_b
@@ -308,7 +308,7 @@ struct Handle {
   // residual tangent (Jacobian-vector product) workspace of dual numbers
   // (value, derivative), allocated on first use: W, prim [5N], q [NQ N],
   // grad [3 NQ N], face fluxes [5 (F+B)], viscous cell terms [24 N] and
-  // viscous face terms [8 (F+B)]
+  // viscous face terms [4 (F+B)]
   void* tW = nullptr;
   void* tprim = nullptr;
   void* tq = nullptr;

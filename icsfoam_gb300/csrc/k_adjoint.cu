@@ -252,8 +252,7 @@ __global__ void __launch_bounds__(128) k_adj_lim(DevMesh m, unsigned mask, unsig
         const int f = isOwn ? code : ~code;
         const int other = isOwn ? m.nei[f] : m.own[f];
         const double wf = m.w[f];
-        const double sg = isOwn ? 1.0 : -1.0;
-        const double S0 = sg * m.Sf[f], S1 = sg * m.Sf[F + f], S2 = sg * m.Sf[2 * F + f];
+        const double S0 = flip(m.Sf[f], !isOwn), S1 = flip(m.Sf[F + f], !isOwn), S2 = flip(m.Sf[2 * F + f], !isOwn);
         const double qo = q[k * N + other];
         const double qown = isOwn ? qc : qo, qnei = isOwn ? qo : qc;
         const double sf = wf * (qown - qnei) + qnei;

@@ -18,7 +18,7 @@
 namespace ics {
 
 __global__ void k_update(int N, double* __restrict__ W, const double* __restrict__ dW, double* __restrict__ prim,
-                         double R, double Cv, double rhoMin, double eMin, double eMax, int useTMax,
+                         double R, double Cv, double iCv, double rhoMin, double eMin, double eMax, int useTMax,
                          int* __restrict__ bounded) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
@@ -26,8 +26,11 @@ __global__ void k_update(int N, double* __restrict__ W, const double* __restrict
   double rU[3] = {W[5 * i + 1] + dW[5 * i + 1], W[5 * i + 2] + dW[5 * i + 2], W[5 * i + 3] + dW[5 * i + 3]};
   double rE = W[5 * i + 4] + dW[5 * i + 4];
   rho = fmax(rho, rhoMin);
-  double U[3] = {rU[0] / rho, rU[1] / rho, rU[2] / rho};
-  double e = rE / rho - 0.5 * dot3(U, U);
+  // one reciprocal for the four quotients (quot): an FP64 division costs ten
+  // operations of the pipe that bounds this kernel
+  const double ir = 1.0 / rho;
+  double U[3] = {quot(rU[0], rho, ir), quot(rU[1], rho, ir), quot(rU[2], rho, ir)};
+  double e = quot(rE, rho, ir) - 0.5 * dot3(U, U);
   int nb = 0;
   if (e < eMin) {
     e = eMin;
@@ -38,8 +41,8 @@ __global__ void k_update(int N, double* __restrict__ W, const double* __restrict
     nb = 1;
   }
   if (nb) atomicAdd(bounded, 1);
-  const double T = e / Cv;
-  const double p = rho / (1.0 / (R * T));
+  const double T = quot(e, Cv, iCv);
+  const double p = rho * (R * T);
   W[5 * i] = rho;
   W[5 * i + 1] = rho * U[0];
   W[5 * i + 2] = rho * U[1];
@@ -203,33 +206,54 @@ __global__ void k_bc_init(DevMesh m, const double* __restrict__ prim, double R, 
   phiB[b] = (1.0 / (R * T)) * p * dot3(U, S);
 }
 
-// primitives from W (set_conservative); Real = Dual for the tangent
-template <typename Real>
-__global__ void k_derive(int N, const Real* __restrict__ W, Real* __restrict__ prim, double R, double Cv) {
+// primitives from W (set_conservative)
+__global__ void k_derive(int N, const double* __restrict__ W, double* __restrict__ prim, double R, double Cv,
+                         double iCv) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  const Real rho = W[5 * i];
-  const Real U[3] = {W[5 * i + 1] / rho, W[5 * i + 2] / rho, W[5 * i + 3] / rho};
-  const Real e = W[5 * i + 4] / rho - 0.5 * dot3(U, U);
-  const Real T = e / Cv;
-  prim[i] = rho / (1.0 / (R * T));
+  const double rho = W[5 * i], ir = 1.0 / rho;
+  const double U[3] = {quot(W[5 * i + 1], rho, ir), quot(W[5 * i + 2], rho, ir), quot(W[5 * i + 3], rho, ir)};
+  const double e = quot(W[5 * i + 4], rho, ir) - 0.5 * dot3(U, U);
+  const double T = quot(e, Cv, iCv);
+  prim[i] = rho * (R * T);
   prim[N + i] = T;
   prim[2 * N + i] = U[0];
   prim[3 * N + i] = U[1];
   prim[4 * N + i] = U[2];
 }
 
+// Tangent of that map along the derivatives in W.  The values are the stored
+// primitives, those the residual and its reverse product start from, so that
+// all three decide every limiter and flux branch on the same numbers.
+__global__ void k_derive_tangent(int N, const Dual* __restrict__ W, const double* __restrict__ prim,
+                                 Dual* __restrict__ tprim, double R, double iCv) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= N) return;
+  const Dual rho = W[5 * i];
+  const double ir = 1.0 / rho.v;
+  const double p = prim[i], T = prim[N + i];
+  const double U[3] = {prim[2 * N + i], prim[3 * N + i], prim[4 * N + i]};
+  double dU[3];
+  for (int k = 0; k < 3; ++k) dU[k] = (W[5 * i + 1 + k].d - U[k] * rho.d) * ir;
+  const Dual rE = W[5 * i + 4];
+  const double de = (rE.d - rE.v * ir * rho.d) * ir - dot3(U, dU);
+  const double dT = de * iCv;
+  tprim[i] = Dual(p, R * (rho.d * T + rho.v * dT));
+  tprim[N + i] = Dual(T, dT);
+  for (int k = 0; k < 3; ++k) tprim[(2 + k) * N + i] = Dual(U[k], dU[k]);
+}
+
 __global__ void k_bad(int N, const double* __restrict__ W, const double* __restrict__ Wprev, double lb,
                       int* __restrict__ bad) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  const double rp = Wprev[5 * i], rEp = Wprev[5 * i + 4];
-  const double up[3] = {Wprev[5 * i + 1] / rp, Wprev[5 * i + 2] / rp, Wprev[5 * i + 3] / rp};
+  const double rp = Wprev[5 * i], irp = 1.0 / rp;
+  const double up[3] = {quot(Wprev[5 * i + 1], rp, irp), quot(Wprev[5 * i + 2], rp, irp), quot(Wprev[5 * i + 3], rp, irp)};
   const double rhoMin = lb * rp;
-  const double eMin = lb * (rEp / rp - 0.5 * dot3(up, up));
-  const double r = W[5 * i];
-  const double u[3] = {W[5 * i + 1] / r, W[5 * i + 2] / r, W[5 * i + 3] / r};
-  const double eT = W[5 * i + 4] / r - 0.5 * dot3(u, u);
+  const double eMin = lb * (quot(Wprev[5 * i + 4], rp, irp) - 0.5 * dot3(up, up));
+  const double r = W[5 * i], ir = 1.0 / r;
+  const double u[3] = {quot(W[5 * i + 1], r, ir), quot(W[5 * i + 2], r, ir), quot(W[5 * i + 3], r, ir)};
+  const double eT = quot(W[5 * i + 4], r, ir) - 0.5 * dot3(u, u);
   bad[i] = (r < rhoMin || eT < eMin || eT < SMALL) ? 1 : 0;
 }
 
@@ -253,7 +277,7 @@ void launch_update(Handle& h, int* boundedDev) {
   const double eMin = h.cfg.Cv * c.T_min;
   const double eMax = h.cfg.Cv * c.T_max;
   const int useTMax = c.T_max < GREAT ? 1 : 0;
-  ICS_LAUNCH(h, ICS_K_UPDATE, k_update<<<grid_for(h.m.N, 256), 256, 0, h.stream>>>(h.m.N, h.W, h.dW, h.prim, c.R, h.cfg.Cv, c.rho_min, eMin, eMax,
+  ICS_LAUNCH(h, ICS_K_UPDATE, k_update<<<grid_for(h.m.N, 256), 256, 0, h.stream>>>(h.m.N, h.W, h.dW, h.prim, c.R, h.cfg.Cv, 1.0 / h.cfg.Cv, c.rho_min, eMin, eMax,
                                                         useTMax, boundedDev));
   ICS_CUDA(cudaGetLastError());
 }
@@ -293,13 +317,13 @@ void launch_set_primitive(Handle& h) {
 }
 
 void launch_derive_primitive(Handle& h) {
-  ICS_LAUNCH(h, ICS_K_UPDATE, k_derive<<<grid_for(h.m.N, 256), 256, 0, h.stream>>>(h.m.N, h.W, h.prim, h.cfg.c.R, h.cfg.Cv));
+  ICS_LAUNCH(h, ICS_K_UPDATE, k_derive<<<grid_for(h.m.N, 256), 256, 0, h.stream>>>(h.m.N, h.W, h.prim, h.cfg.c.R, h.cfg.Cv, 1.0 / h.cfg.Cv));
   ICS_CUDA(cudaGetLastError());
 }
 
 void launch_derive_tangent(Handle& h, const Dual* W, Dual* prim) {
-  ICS_LAUNCH(h, ICS_K_TANGENT, k_derive<Dual><<<grid_for(h.m.N, 256), 256, 0, h.stream>>>(h.m.N, W, prim, h.cfg.c.R,
-                                                                                          h.cfg.Cv));
+  ICS_LAUNCH(h, ICS_K_TANGENT, k_derive_tangent<<<grid_for(h.m.N, 256), 256, 0, h.stream>>>(h.m.N, W, h.prim, prim,
+                                                                                            h.cfg.c.R, 1.0 / h.cfg.Cv));
   ICS_CUDA(cudaGetLastError());
 }
 

@@ -21,30 +21,30 @@
 namespace ics {
 
 struct ViscParams {
-  double R, Cv, Cp, gamma, mu, Pr, As, Ts;
+  double R, Cv, gamma, mu, As, Ts;
+  double alphaFac;  // alphaEff / mu = Cp / (Cv Pr)
   int sutherland;
 };
 
 template <typename Real>
 __device__ __forceinline__ Real mu_of(const ViscParams& P, const Real& T) {
-  return P.sutherland ? P.As * sqrt(T) / (1.0 + P.Ts / T) : Real(P.mu);
+  return P.sutherland ? P.As * sqrt(T) * T / (T + P.Ts) : Real(P.mu);  // As sqrt(T) / (1 + Ts / T)
 }
 template <typename Real>
 __device__ __forceinline__ Real alpha_of(const ViscParams& P, const Real& mu) {
-  return P.Cp / P.Cv * (mu / P.Pr);
+  return P.alphaFac * mu;
 }
 
 // vc layout [24][N]: 0-8 grad U (3i+j), 9-11 grad e, 12-20 tau (3i+j), 21 mu, 22 alpha, 23 e
 
 template <typename Real = double>
-__global__ void __launch_bounds__(128) k_visc_cell(DevMesh m, ViscParams P, const Real* __restrict__ W,
-                                                   const Real* __restrict__ prim, const double* __restrict__ TB,
+__global__ void __launch_bounds__(128) k_visc_cell(DevMesh m, ViscParams P, const Real* __restrict__ prim, const double* __restrict__ TB,
                                                    const double* __restrict__ UB, Real* __restrict__ vc) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.N) return;
   const int N = m.N, F = m.F, B = m.B;
   Real Uc[3] = {prim[2 * N + c], prim[3 * N + c], prim[4 * N + c]};
-  const Real ec = W[5 * c + 4] / W[5 * c] - 0.5 * dot3(Uc, Uc);
+  const Real ec = P.Cv * prim[N + c];  // e = Cv T
   Real g[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, ge[3] = {0, 0, 0};
   for (int e = m.cptr[c]; e < m.cptr[c + 1]; ++e) {
     const int code = m.cface[e];
@@ -52,17 +52,18 @@ __global__ void __launch_bounds__(128) k_visc_cell(DevMesh m, ViscParams P, cons
     const int f = isOwn ? code : ~code;
     const int other = isOwn ? m.nei[f] : m.own[f];
     const double wf = m.w[f];
-    const double S[3] = {m.Sf[f], m.Sf[F + f], m.Sf[2 * F + f]};
+    // outward area vector
+    const double S[3] = {flip(m.Sf[f], !isOwn), flip(m.Sf[F + f], !isOwn), flip(m.Sf[2 * F + f], !isOwn)};
     const Real Uo[3] = {prim[2 * N + other], prim[3 * N + other], prim[4 * N + other]};
-    const Real eo = W[5 * other + 4] / W[5 * other] - 0.5 * dot3(Uo, Uo);
+    const Real eo = P.Cv * prim[N + other];
     for (int j = 0; j < 3; ++j) {
       const Real a = isOwn ? Uc[j] : Uo[j], b = isOwn ? Uo[j] : Uc[j];
       const Real sf = wf * (a - b) + b;
-      for (int i = 0; i < 3; ++i) g[3 * i + j] = isOwn ? g[3 * i + j] + S[i] * sf : g[3 * i + j] - S[i] * sf;
+      for (int i = 0; i < 3; ++i) g[3 * i + j] = g[3 * i + j] + S[i] * sf;
     }
     const Real a = isOwn ? ec : eo, b = isOwn ? eo : ec;
     const Real sf = wf * (a - b) + b;
-    for (int i = 0; i < 3; ++i) ge[i] = isOwn ? ge[i] + S[i] * sf : ge[i] - S[i] * sf;
+    for (int i = 0; i < 3; ++i) ge[i] = ge[i] + S[i] * sf;
   }
   for (int e = m.bptr[c]; e < m.bptr[c + 1]; ++e) {
     const int b = m.bface[e];
@@ -73,7 +74,7 @@ __global__ void __launch_bounds__(128) k_visc_cell(DevMesh m, ViscParams P, cons
       const double* Rm = m.patches[m.bpatch[b]].R;
       const double wb = m.bw[b];
       const Real Un[3] = {prim[2 * N + pc], prim[3 * N + pc], prim[4 * N + pc]};
-      const Real en = W[5 * pc + 4] / W[5 * pc] - 0.5 * dot3(Un, Un);
+      const Real en = P.Cv * prim[N + pc];
       Real upv[3];
       if (plag_mode(m, b))  // U phase-lagged across an HB phase-lag patch
         plag_vec(m, b, pc, prim + 2 * N, prim + 3 * N, prim + 4 * N, upv);
@@ -94,9 +95,9 @@ __global__ void __launch_bounds__(128) k_visc_cell(DevMesh m, ViscParams P, cons
       for (int i = 0; i < 3; ++i) g[3 * i + j] += S[i] * Ub[j];
     for (int i = 0; i < 3; ++i) ge[i] += S[i] * eb;
   }
-  const double Vc = m.V[c];
-  for (int q = 0; q < 9; ++q) g[q] /= Vc;
-  for (int q = 0; q < 3; ++q) ge[q] /= Vc;
+  const double rV = 1.0 / m.V[c];  // one division for the twelve components
+  for (int q = 0; q < 9; ++q) g[q] = g[q] * rV;
+  for (int q = 0; q < 3; ++q) ge[q] = ge[q] * rV;
   const Real mu = mu_of(P, prim[N + c]);
   const Real tr = g[0] + g[4] + g[8];
   for (int q = 0; q < 9; ++q) vc[q * N + c] = g[q];
@@ -108,7 +109,8 @@ __global__ void __launch_bounds__(128) k_visc_cell(DevMesh m, ViscParams P, cons
   vc[23 * N + c] = ec;
 }
 
-// fv layout [8][F+B]: lapU(3), divTau(3), divSig, lapE
+// fv layout [4][F+B]: laplacian(mu, U) + div(tauMC) (3), div(sigmaDotU . S) +
+// laplacian(alphaEff, e); the cells add the face terms up
 template <typename Real = double>
 __global__ void __launch_bounds__(128) k_visc_face(DevMesh m, const Real* __restrict__ vc,
                                                    const Real* __restrict__ W, const Real* __restrict__ prim,
@@ -139,18 +141,16 @@ __global__ void __launch_bounds__(128) k_visc_face(DevMesh m, const Real* __rest
     snU[j] = nodc * (b - a) + corr;
   }
   const Real ml = muf * ms;
-  for (int j = 0; j < 3; ++j) fv[j * FB + f] = ml * snU[j];
-  for (int j = 0; j < 3; ++j) fv[(3 + j) * FB + f] = S[0] * tf[j] + S[1] * tf[3 + j] + S[2] * tf[6 + j];
+  for (int j = 0; j < 3; ++j) fv[j * FB + f] = ml * snU[j] + S[0] * tf[j] + S[1] * tf[3 + j] + S[2] * tf[6 + j];
   Real sig[3];
   for (int i = 0; i < 3; ++i) {
     Real s = 0;
     for (int j = 0; j < 3; ++j) s += (muf * gUf[3 * i + j] + tf[3 * i + j]) * Uf[j];
     sig[i] = s;
   }
-  fv[6 * FB + f] = dot3(sig, S);
   const Real gef[3] = {lin(9), lin(10), lin(11)};
   const Real snE = nodc * (vc[23 * N + n] - vc[23 * N + o]) + dot3(k, gef);
-  fv[7 * FB + f] = (alf * ms) * snE;
+  fv[3 * FB + f] = dot3(sig, S) + (alf * ms) * snE;
   if constexpr (std::is_same<Real, double>::value) {  // Jacobian coefficient: not part of the tangent
     const double rhof = wf * (W[5 * o] - W[5 * n]) + W[5 * n];
     const double lamv = (muf + alf) / rhof;
@@ -173,7 +173,7 @@ __global__ void k_visc_bface(DevMesh m, ViscParams P, const Real* __restrict__ v
   const int o = m.bcell[b];
   const double ms = m.bmagSf[b];
   const double S[3] = {m.bSf[b], m.bSf[B + b], m.bSf[2 * B + b]};
-  const double n[3] = {S[0] / ms, S[1] / ms, S[2] / ms};
+  const double n[3] = {m.bnf[b], m.bnf[B + b], m.bnf[2 * B + b]};
   const double UB[3] = {UBv[b], UBv[B + b], UBv[2 * B + b]};
   const double muB = mu_of(P, TB[b]);
   const double alB = alpha_of(P, muB);
@@ -193,16 +193,14 @@ __global__ void k_visc_bface(DevMesh m, ViscParams P, const Real* __restrict__ v
   for (int i = 0; i < 3; ++i)
     for (int j = 0; j < 3; ++j) tb[3 * i + j] = muB * (g[3 * j + i] - (i == j ? (2.0 / 3.0) * tr : Real(0.0)));
   const double ml = muB * ms;
-  for (int j = 0; j < 3; ++j) fv[j * FB + F + b] = ml * snU[j];
-  for (int j = 0; j < 3; ++j) fv[(3 + j) * FB + F + b] = S[0] * tb[j] + S[1] * tb[3 + j] + S[2] * tb[6 + j];
+  for (int j = 0; j < 3; ++j) fv[j * FB + F + b] = ml * snU[j] + S[0] * tb[j] + S[1] * tb[3 + j] + S[2] * tb[6 + j];
   Real sig[3];
   for (int i = 0; i < 3; ++i) {
     Real s = 0;
     for (int j = 0; j < 3; ++j) s += (muB * g[3 * i + j] + tb[3 * i + j]) * UB[j];
     sig[i] = s;
   }
-  fv[6 * FB + F + b] = dot3(sig, S);
-  fv[7 * FB + F + b] = (alB * ms) * snE;
+  fv[3 * FB + F + b] = dot3(sig, S) + (alB * ms) * snE;
   if (vj) {  // patch mu and alphaEff for the non-LF boundary terms (viscousFluxScheme.C:57-58)
     vj[F + b] = muB;
     vj[FB + F + b] = alB;
@@ -259,22 +257,20 @@ __global__ void __launch_bounds__(128) k_visc_cface(DevMesh m, const Real* __res
     snU[j] = nodc * (up - uo) + corr;
   }
   const Real ml = muf * ms;
-  for (int j = 0; j < 3; ++j) fv[j * FB + F + b] = ml * snU[j];
-  for (int j = 0; j < 3; ++j) fv[(3 + j) * FB + F + b] = S[0] * tf[j] + S[1] * tf[3 + j] + S[2] * tf[6 + j];
+  for (int j = 0; j < 3; ++j) fv[j * FB + F + b] = ml * snU[j] + S[0] * tf[j] + S[1] * tf[3 + j] + S[2] * tf[6 + j];
   Real sig[3];
   for (int i = 0; i < 3; ++i) {
     Real s = 0;
     for (int j = 0; j < 3; ++j) s += (muf * gUf[3 * i + j] + tf[3 * i + j]) * Uf[j];
     sig[i] = s;
   }
-  fv[6 * FB + F + b] = dot3(sig, S);
   Real gef[3];
   for (int i = 0; i < 3; ++i) {
     const Real gp = Rm[3 * i] * vc[9 * N + pc] + Rm[3 * i + 1] * vc[10 * N + pc] + Rm[3 * i + 2] * vc[11 * N + pc];
     gef[i] = lin(vc[(9 + i) * N + o], gp);
   }
   const Real snE = nodc * (vc[23 * N + pc] - vc[23 * N + o]) + dot3(k, gef);
-  fv[7 * FB + F + b] = (alf * ms) * snE;
+  fv[3 * FB + F + b] = dot3(sig, S) + (alf * ms) * snE;
   if constexpr (std::is_same<Real, double>::value) {
     const double rhof = lin(W[5 * o], W[5 * pc]);
     sf2[F + b] = 0.5 * ((muf + alf) / rhof) * ms * m.bdc[b];
@@ -290,17 +286,15 @@ void launch_viscous(Handle& h) {
   ViscParams P;
   P.R = h.cfg.c.R;
   P.Cv = h.cfg.Cv;
-  P.Cp = h.cfg.c.Cp;
   P.gamma = h.cfg.gamma;
   P.mu = h.cfg.c.mu;
-  P.Pr = h.cfg.c.Pr;
+  P.alphaFac = h.cfg.c.Cp / (h.cfg.Cv * h.cfg.c.Pr);
   P.As = h.cfg.c.As;
   P.Ts = h.cfg.c.Ts;
   P.sutherland = h.cfg.c.sutherland;
   const int FB = h.m.F + h.m.B;
   double* vj = h.vjac;  // written in both Jacobian modes: the mode may change between residual and assembly
-  ICS_LAUNCH(h, ICS_K_VISC, k_visc_cell<<<grid_for(h.m.N, 128), 128, 0, h.stream>>>(h.m, P, h.W, h.prim, h.TB, h.UB,
-                                                                                     h.vcell));
+  ICS_LAUNCH(h, ICS_K_VISC, k_visc_cell<<<grid_for(h.m.N, 128), 128, 0, h.stream>>>(h.m, P, h.prim, h.TB, h.UB, h.vcell));
   if (h.m.F)
     ICS_LAUNCH(h, ICS_K_VISC, k_visc_face<<<grid_for(h.m.F, 128), 128, 0, h.stream>>>(h.m, h.vcell, h.W, h.prim,
                                                                                        h.fvisc, h.vsf2, vj, FB));
@@ -318,16 +312,14 @@ void launch_viscous_tangent(Handle& h, const Dual* W, const Dual* prim, Dual* vc
   ViscParams P;
   P.R = h.cfg.c.R;
   P.Cv = h.cfg.Cv;
-  P.Cp = h.cfg.c.Cp;
   P.gamma = h.cfg.gamma;
   P.mu = h.cfg.c.mu;
-  P.Pr = h.cfg.c.Pr;
+  P.alphaFac = h.cfg.c.Cp / (h.cfg.Cv * h.cfg.c.Pr);
   P.As = h.cfg.c.As;
   P.Ts = h.cfg.c.Ts;
   P.sutherland = h.cfg.c.sutherland;
   const int FB = h.m.F + h.m.B;
-  ICS_LAUNCH(h, ICS_K_TANGENT, k_visc_cell<Dual><<<grid_for(h.m.N, 128), 128, 0, h.stream>>>(h.m, P, W, prim, h.TB,
-                                                                                             h.UB, vc));
+  ICS_LAUNCH(h, ICS_K_TANGENT, k_visc_cell<Dual><<<grid_for(h.m.N, 128), 128, 0, h.stream>>>(h.m, P, prim, h.TB, h.UB, vc));
   if (h.m.F)
     ICS_LAUNCH(h, ICS_K_TANGENT, k_visc_face<Dual><<<grid_for(h.m.F, 128), 128, 0, h.stream>>>(h.m, vc, W, prim, fv,
                                                                                                nullptr, nullptr, FB));

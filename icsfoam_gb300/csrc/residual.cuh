@@ -53,18 +53,18 @@ __device__ __forceinline__ Real reconstruct(const DevMesh& m, int scheme, int k,
                                             const Real& qn, const Real* __restrict__ grad, double dir) {
   const int N = m.N, F = m.F;
   const double wUp = dir > 0 ? 1.0 : 0.0;
-  if (scheme == ICS_RECON_UPWIND) return wUp * (qo - qn) + qn;
+  if (scheme == ICS_RECON_UPWIND) return dir > 0 ? qo : qn;
   if (scheme == ICS_RECON_VANLEER || scheme == ICS_RECON_MINMOD) {
     const int c = dir > 0 ? o : nb;
     const double d0 = m.dCC[f], d1 = m.dCC[F + f], d2 = m.dCC[2 * F + f];
     const Real gradcf = d0 * grad[(3 * k) * N + c] + d1 * grad[(3 * k + 1) * N + c] + d2 * grad[(3 * k + 2) * N + c];
     return tvd_face(scheme, m.w[f], wUp, qo, qn, gradcf);
   }
-  // MUSCL: upwind value + limited-gradient extrapolation; the neighbour
-  // side's upwind value 0 (qo - qn) + qn is qn itself
+  // MUSCL: upwind value + limited-gradient extrapolation (the small products
+  // are summed before they meet the value: one rounding at its size)
   const int c = dir > 0 ? o : nb;
   const double* d = dir > 0 ? m.dOwn : m.dNei;
-  const Real base = dir > 0 ? (qo - qn) + qn : qn;
+  const Real base = dir > 0 ? qo : qn;
   return base + (d[f] * grad[(3 * k) * N + c] + d[F + f] * grad[(3 * k + 1) * N + c] +
                  d[2 * F + f] * grad[(3 * k + 2) * N + c]);
 }
