@@ -33,7 +33,7 @@ struct ics_handle_s {
 };
 
 namespace ics {
-double rho_l2(Handle& h);
+double rho_l2(Handle& h, double* host_src, bool* finite);
 double device_sum(Handle& h, const double* a, int n);
 
 constexpr size_t EV_POOL = 8192;  // events; folded into the totals when full
@@ -591,18 +591,10 @@ int do_residual(Handle& h, double* host_src) {
   }
   launch_residual(h, ratio, apply);
   h.haveFlux = true;
-  h.lastRhoL2 = rho_l2(h);
+  bool finite = true;
+  h.lastRhoL2 = rho_l2(h, host_src, &finite);
   if (h.cases.n) case_l2(h);
-  if (host_src) {
-    ICS_CUDA(cudaMemcpyAsync(host_src, h.src, 5ull * h.m.N * sizeof(double), cudaMemcpyDeviceToHost, h.stream));
-    ICS_CUDA(cudaStreamSynchronize(h.stream));
-    for (size_t i = 0; i < 5ull * h.m.N; ++i)
-      if (!std::isfinite(host_src[i])) {
-        h.err = "non-finite residual";
-        return ICS_ERR_NONFINITE;
-      }
-  }
-  if (!std::isfinite(h.lastRhoL2)) {
+  if ((host_src && !finite) || !std::isfinite(h.lastRhoL2)) {
     h.err = "non-finite residual";
     return ICS_ERR_NONFINITE;
   }

@@ -51,6 +51,7 @@ struct KrylovScalars {
   double nfr[8 * MAX_INST];  // per instance: norm-factor sums (rho, rhoE, rhoU), |b| per equation
   double res[5 * MAX_INST];  // per-instance L1 residuals (unnormalised sums)
   double l2;              // rho L2 partial result
+  int nonfinite;          // set by k_cellres when a source entry is not finite (read with l2)
   int status;             // breakdown / non-finite flags
 };
 

@@ -1495,13 +1495,22 @@ double device_sum(Handle& h, const double* a, int n) {
   return v;
 }
 
-// rho L2 residual: sqrt(sum (div(phi) V)^2) from the per-cell squares
-double rho_l2(Handle& h) {
+// rho L2 residual: sqrt(sum (div(phi) V)^2) from the per-cell squares, and
+// whether every entry of the source is finite; host_src (if not null) receives
+// the source in the same wait
+double rho_l2(Handle& h, double* host_src, bool* finite) {
   ICS_LAUNCH(h, ICS_K_VECTOR, k_sumsq<<<REDUCE_BLOCKS, RB, 0, h.stream>>>(h.m.N, h.scratch, h.partials, h.counter, &h.ks->l2));
-  double v = 0;
-  ICS_CUDA(cudaMemcpyAsync(&v, &h.ks->l2, sizeof(double), cudaMemcpyDeviceToHost, h.stream));
+  struct {
+    double l2;
+    int nonfinite, status;
+  } v = {0, 0, 0};
+  static_assert(offsetof(KrylovScalars, nonfinite) == offsetof(KrylovScalars, l2) + sizeof(double), "");
+  ICS_CUDA(cudaMemcpyAsync(&v, &h.ks->l2, sizeof(v), cudaMemcpyDeviceToHost, h.stream));
+  if (host_src)
+    ICS_CUDA(cudaMemcpyAsync(host_src, h.src, 5ull * h.m.N * sizeof(double), cudaMemcpyDeviceToHost, h.stream));
   ICS_CUDA(cudaStreamSynchronize(h.stream));
-  return std::sqrt(v);
+  *finite = v.nonfinite == 0;
+  return std::sqrt(v.l2);
 }
 
 // ------------------------------------------------------ passive scalar
