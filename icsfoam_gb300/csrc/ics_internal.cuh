@@ -168,10 +168,6 @@ struct DevMesh {
   // cell [N] and each case's SER factor [n_cases] (< 0: not applied)
   const int* caseOf = nullptr;
   const double* caseSer = nullptr;
-  // and each case's Krylov norm and flags (the fused operator's scaling)
-  const double* caseBeta = nullptr;
-  const int* caseActive = nullptr;
-  const int* caseStatus = nullptr;
 };
 
 // pseudotimeControl state (pseudotimeControl.C): the iteration count of the
@@ -212,6 +208,10 @@ struct CaseDev {
 
 struct CaseSet {
   int n = 0, nseg = 0;
+  int columnCells = 0;       // cells of the largest case with columns of one launch (k_ccolumn)
+  bool columnLarge = false;  // some case is larger
+  cudaStream_t side = nullptr;  // of the small cases' columns in a stack that has both
+  cudaEvent_t fork = nullptr, join = nullptr;
   std::vector<int> start;          // host [n+1]
   CaseDev d;
   int* caseOf = nullptr;           // device [N]
@@ -491,10 +491,9 @@ void sweep_probe(Handle& h, const int* order, int tickets, int spin_limit);
 void from_vec(Handle& h, const void* src, double* dst); // Krylov type -> FP64
 
 inline int prec(const Handle& h) { return h.cfg.c.precision; }
-// w = M^-1 A x by the fused LU-SGS operator passes, x scaled by the reciprocal
-// norm of each row's stacked case and stored in vout when that is given; false
-// (nothing launched) where they do not apply
-bool fused_operator(Handle& h, const void* x, void* w, void* vout);
+// w = M^-1 A x by the fused LU-SGS operator passes; false (nothing launched)
+// where they do not apply
+bool fused_operator(Handle& h, const void* x, void* w);
 // element stride between consecutive Krylov basis vectors (5N rounded up to 64)
 inline size_t kstride(const Handle& h) { return ((5ull * h.m.N + 63) / 64) * 64; }
 inline size_t vbytes(const Handle& h) { return prec(h) == ICS_PREC_MIXED ? 4 : 8; }

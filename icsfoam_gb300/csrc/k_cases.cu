@@ -24,12 +24,13 @@
 //     inactive and its correction is left as it stands while the others go
 //     on.
 // The LU-SGS preconditioner, the SpMV and the fused operator passes are the
-// handle's own (union) kernels: their rows only read rows of the same case, and
-// the fused passes scale each row by its own case's Krylov norm.
+// handle's own (union) kernels: their rows only read rows of the same case.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cmath>
 
-#include "ics_internal.cuh"
+#include "krylov.cuh"
 
 namespace ics {
 
@@ -37,6 +38,12 @@ namespace {
 
 constexpr int SEG_CELLS = 1024;  // cells per reduction segment (5120 vector entries)
 constexpr int CB = 256;          // threads per segment block
+// of the Gram-Schmidt steps, whose threads have all their loads in flight:
+// 60 registers of entries at most
+template <typename TV>
+constexpr int MB = sizeof(TV) == 4 ? 256 : 512;
+template <typename TV>
+constexpr int MB_ENTRIES = 5 * SEG_CELLS / MB<TV>;
 constexpr int PSTRIDE = 8;       // partial sums per segment
 constexpr int HSTRIDE = MAX_DIRS * MAX_DIRS;
 
@@ -45,76 +52,49 @@ __device__ __forceinline__ bool case_on(const CaseDev& D, int c) { return D.acti
 // Block-sum NV values, store them as this segment's partials, and on the
 // last segment of case c to arrive fold the case's partials in segment order
 // into out[0..NV).  True on thread 0 of that block.
-template <int NV>
+template <int NV, int CB>
 __device__ __forceinline__ bool case_finish(const CaseDev& D, int c, double (&v)[NV], double* __restrict__ out) {
-  __shared__ double sm[CB / 32][NV];
+  constexpr int G = FOLD_GROUP<NV>;
+  __shared__ double sm[CB / 32][FOLD_VALUES<NV>];
   __shared__ bool amLast;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    double x = v[k];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) sm[warp][k] = x;
-  }
-  __syncthreads();
+  const bool writer = threadIdx.x < 32 && threadIdx.x % G == 0 && threadIdx.x / G < NV;
+  const int k = threadIdx.x / G;
+  double s = block_sums<NV, CB / 32>(v, sm);
   const int s0 = D.caseSeg[c], ns = D.caseSeg[c + 1] - s0;
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < NV; ++k) {
-      double s = 0;
-      for (int w = 0; w < CB / 32; ++w) s += sm[w][k];
-      D.partials[(size_t)blockIdx.x * PSTRIDE + k] = s;
+  if (ns > 1) {
+    if (threadIdx.x < 32) {
+      if (writer) {
+        D.partials[(size_t)blockIdx.x * PSTRIDE + k] = s;
+        __threadfence();
+      }
+      __syncwarp();
+      if (threadIdx.x == 0) {
+        const unsigned t = atomicAdd(&D.counter[c], 1u);
+        amLast = (t == (unsigned)ns - 1);
+      }
     }
+    __syncthreads();
+    if (!amLast) return false;
     __threadfence();
-    const unsigned t = atomicAdd(&D.counter[c], 1u);
-    amLast = (t == (unsigned)ns - 1);
-  }
-  __syncthreads();
-  if (!amLast) return false;
-  __threadfence();
-  const volatile double* vp = D.partials;
-  double acc[NV];
+    const volatile double* vp = D.partials;
+    double acc[NV];
 #pragma unroll
-  for (int k = 0; k < NV; ++k) acc[k] = 0.0;
-  for (int b = threadIdx.x; b < ns; b += CB)
+    for (int q = 0; q < NV; ++q) acc[q] = 0.0;
+    for (int b = threadIdx.x; b < ns; b += CB)
 #pragma unroll
-    for (int k = 0; k < NV; ++k) acc[k] += vp[(size_t)(s0 + b) * PSTRIDE + k];
-#pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    double x = acc[k];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) sm[warp][k] = x;  // thread 0 read sm before the barrier above
+      for (int q = 0; q < NV; ++q) acc[q] += vp[(size_t)(s0 + b) * PSTRIDE + q];
+    s = block_sums<NV, CB / 32>(acc, sm);
+    if (threadIdx.x == 0) D.counter[c] = 0;
   }
-  __syncthreads();
-  if (threadIdx.x != 0) return false;
-  for (int k = 0; k < NV; ++k) {
-    double s = 0;
-    for (int w = 0; w < CB / 32; ++w) s += sm[w][k];
-    out[k] = s;
-  }
-  D.counter[c] = 0;
-  return true;
-}
-
-__device__ __forceinline__ void case_givens(double h, double beta, double& c, double& s) {
-  if (beta == 0) {
-    c = 1;
-    s = 0;
-  } else if (fabs(beta) > fabs(h)) {
-    const double tau = -h / beta;
-    s = 1.0 / sqrt(1.0 + tau * tau);
-    c = s * tau;
-  } else {
-    const double tau = -beta / h;
-    c = 1.0 / sqrt(1.0 + tau * tau);
-    s = c * tau;
-  }
+  if (threadIdx.x >= 32) return false;
+  if (writer) out[k] = s;
+  __syncwarp();
+  return threadIdx.x == 0;
 }
 
 // start of a cycle for case c: beta = |w|, bh = (beta, 0, ...)
-__device__ void case_beta0(const CaseDev& D, int c) {
-  const double beta = sqrt(D.red[2 * c]);
+__device__ void case_beta0(const CaseDev& D, int c, double nrm2) {
+  const double beta = sqrt(nrm2);
   D.beta[c] = beta;
   double* bh = D.bh + (size_t)c * (MAX_DIRS + 1);
   for (int i = 0; i <= D.m; ++i) bh[i] = 0.0;
@@ -122,87 +102,261 @@ __device__ void case_beta0(const CaseDev& D, int c) {
   if (!(beta > 0.0)) D.status[c] = isfinite(beta) ? 2 : 4;
 }
 
-// Hessenberg column i of case c: apply the previous rotations, make a new one
-// (gmres.C:1013-1027, rotation gmres.C:44-69)
-__device__ void case_hess(const CaseDev& D, int c, int i) {
-  const int m = D.m;
-  double* H = D.H + (size_t)c * HSTRIDE;
-  double* cs = D.c + (size_t)c * MAX_DIRS;
-  double* sn = D.s + (size_t)c * MAX_DIRS;
-  double* bh = D.bh + (size_t)c * (MAX_DIRS + 1);
-  const double beta = sqrt(D.red[2 * c + 1]);
-  for (int j = 0; j < i; ++j) {
-    const double Hji = H[j * m + i];
-    H[j * m + i] = cs[j] * Hji - sn[j] * H[(j + 1) * m + i];
-    H[(j + 1) * m + i] = sn[j] * Hji + cs[j] * H[(j + 1) * m + i];
-  }
-  case_givens(H[i * m + i], beta, cs[i], sn[i]);
-  const double bhi = bh[i];
-  bh[i] = cs[i] * bhi - sn[i] * bh[i + 1];
-  bh[i + 1] = sn[i] * bhi + cs[i] * bh[i + 1];
-  H[i * m + i] = cs[i] * H[i * m + i] - sn[i] * beta;
-  D.beta[c] = beta;
+// Hessenberg column i of case c, |w|^2 = nrm2
+__device__ void case_hess(const CaseDev& D, int c, int i, double nrm2) {
+  D.beta[c] = sqrt(nrm2);
+  hess_column(D.H + (size_t)c * HSTRIDE, D.c + (size_t)c * MAX_DIRS, D.s + (size_t)c * MAX_DIRS,
+              D.bh + (size_t)c * (MAX_DIRS + 1), i, D.m, nrm2);
 }
 
-// One pipelined modified Gram-Schmidt step per case (as the single-system
-// k_mgs): w -= hprev vprev (when vprev), then the sum of w.vnext (or w.w) into
+// ------------------------------------------------- columns of small cases
+// The Gram-Schmidt of a new Krylov vector against the basis and its
+// normalisation (gmres.C:936-1011), one launch for all cases of up to
+// COLUMN_CELLS cells:
+//   for j = 0 .. dir:  h_j = w . v_j;  w -= h_j v_j
+//   v_{dir+1} = w / |w|
+// (dir = -1, the start of a cycle, has the last line only.)  A cluster of
+// COLUMN_BLOCKS blocks holds a case's w in registers for the whole column and
+// exchanges the blocks' sums of a step through distributed shared memory, so a
+// step costs one cluster barrier and two FP64 folds instead of a launch with a
+// reduction tail.  A case's sums depend only on its own size: the thread that
+// takes an entry and the order of the sums are the same in every instance and
+// every stack.  FP32 sums: a thread adds two runs of at most 16 products in
+// FP32, everything across threads is FP64.  Further clusters rotate the cases'
+// Hessenberg columns of the direction before, one block per case.
+//
+// The line is what the registers hold; below it the clusters were never the
+// slower way (a solve of four cycles, us, clusters against steps of one launch,
+// mixed / FP64: 2 cases of 1000 cells 324 : 441 / 407 : 633, 64 of 1000
+// 720 : 730 / 1012 : 1048, 24 of 13000 1522 : 1949 / 2609 : 3202).  24 tubes
+// of 480 to 12000 cells in mixed precision, a column of 5.5 steps on average:
+// 13 us where the steps took 32, bound by the folds and the barrier (1500
+// cycles a step) and, from 6000 cells on, the L2 reads of 8 SMs; in FP64 by the
+// FP64 pipes of those 8 SMs.
+constexpr int COLUMN_BLOCKS = 8;
+constexpr int COLUMN_THREADS = 256;
+constexpr int COLUMN_STRIDE = COLUMN_BLOCKS * COLUMN_THREADS;
+constexpr int COLUMN_ROUNDS = 32;  // entries per thread at most
+constexpr int COLUMN_CELLS = COLUMN_ROUNDS * COLUMN_STRIDE / 5;
+
+__device__ __forceinline__ bool in_column(const CaseDev& D, int c) { return D.start[c + 1] - D.start[c] <= COLUMN_CELLS; }
+
+template <typename TV, int K>
+__global__ void __cluster_dims__(COLUMN_BLOCKS, 1, 1) __launch_bounds__(COLUMN_THREADS, sizeof(TV) * K <= 128 ? 2 : 1)
+    k_ccolumn(CaseDev D, const TV* __restrict__ w, TV* __restrict__ V, long vs, int dir) {
+  namespace cg = cooperative_groups;
+  __shared__ TV sums[COLUMN_THREADS];
+  __shared__ double slot[2][32];  // of the cluster's 8 x 4 folding warps
+  __shared__ double result;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int c = blockIdx.x / COLUMN_BLOCKS;
+  if (c >= D.n) {  // the rotations, not part of the exchange
+    c = blockIdx.x - COLUMN_BLOCKS * D.n;
+    if (tid == 0 && dir > 0 && c < D.n && in_column(D, c) && case_on(D, c)) case_hess(D, c, dir - 1, D.red[2 * c + ((dir - 1) & 1)]);
+    return;
+  }
+  if (!in_column(D, c) || !case_on(D, c)) return;  // the whole cluster
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.barrier_arrive();  // the other blocks' shared memory exists after the wait
+  const int rank = (int)cluster.block_rank();
+  // this block's entries of the case start at first; a thread's follow at
+  // COLUMN_STRIDE from its own, cnt of them
+  const int first = rank * COLUMN_THREADS, n = 5 * (D.start[c + 1] - D.start[c]);
+  const size_t e0 = 5 * (size_t)D.start[c] + first + tid;
+  const int cnt = (n - first - tid + COLUMN_STRIDE - 1) / COLUMN_STRIDE;
+  // rounds that hold any entry of the block: an FP64 instruction costs its
+  // cycles with every lane predicated off too
+  const int used = (n - first + COLUMN_STRIDE - 1) / COLUMN_STRIDE;
+  TV x[K], v[K], vn[K];
+  auto fetch = [&](TV (&r)[K], const TV* __restrict__ src) {
+#pragma unroll
+    for (int q = 0; q < K; ++q) r[q] = q < cnt ? src[q * COLUMN_STRIDE] : TV(0);
+  };
+  fetch(x, w + e0);
+  if (dir >= 0) fetch(v, V + e0);
+  cluster.barrier_wait();
+  double total = 0.0;
+#pragma unroll 1
+  for (int j = 0; j <= dir + 1; ++j) {
+    if (j < dir) fetch(vn, V + (size_t)(j + 1) * vs + e0);  // in flight during the exchange
+    TV a0 = TV(0), a1 = TV(0);
+#pragma unroll
+    for (int q = 0; q < K; ++q)
+      if (q < used) {
+        const TV y = j <= dir ? v[q] : x[q];
+        if (q & 1)
+          a1 = fma(x[q], y, a1);
+        else
+          a0 = fma(x[q], y, a0);
+      }
+    sums[tid] = a0 + a1;
+    __syncthreads();
+    if (warp < 4) {
+      double s = widen(sums[tid]) + widen(sums[tid + 128]);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane < COLUMN_BLOCKS) *cluster.map_shared_rank(&slot[j & 1][4 * rank + warp], lane) = s;
+    }
+    // the slots of step j are written again in step j + 2, after every block
+    // has passed the barrier of step j + 1 and so has read them
+    cluster.sync();
+    if (warp == 0) {
+      double s = slot[j & 1][lane];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == 0) result = s;
+    }
+    __syncthreads();
+    total = result;
+    if (j <= dir) {
+      const TV h = TV(total);
+#pragma unroll
+      for (int q = 0; q < K; ++q)
+        if (q < used) {
+          x[q] -= h * v[q];
+          v[q] = vn[q];
+        }
+      if (rank == 0 && tid == 0) D.H[(size_t)c * HSTRIDE + j * D.m + dir] = total;
+    }
+  }
+  if (rank == 0 && tid == 0) {
+    D.red[2 * c + (dir & 1)] = total;  // the rotation of direction dir - 1 reads the other one meanwhile
+    if (dir < 0) case_beta0(D, c, total);
+  }
+  // the next basis vector (the last direction of a cycle needs none)
+  if (dir + 1 < D.m) {
+    const TV b = TV(sqrt(total)), rb = TV(1) / b, rl = rb * fma(-b, rb, TV(1));
+    TV* out = V + (size_t)(dir + 1) * vs + e0;
+#pragma unroll
+    for (int q = 0; q < K; ++q)
+      if (q < cnt) out[q * COLUMN_STRIDE] = quotient(x[q], rb, rl);
+  }
+}
+
+// ------------------------------------------------- columns of large cases
+// One pipelined modified Gram-Schmidt step per case of more than COLUMN_CELLS
+// cells: w -= hprev vprev (when vprev), then the sum of w.vnext (or w.w) into
 // H[outIdx] (outRed < 0) or red[outRed]; post 1 starts the cycle, post 2
 // finishes Hessenberg column dir.
 template <typename TV>
-__global__ void __launch_bounds__(CB) k_cmgs(CaseDev D, TV* __restrict__ w, const TV* __restrict__ vprev,
+__global__ void __launch_bounds__(MB<TV>) k_cmgs(CaseDev D, TV* __restrict__ w, const TV* __restrict__ vprev,
                                              int hprevIdx, const TV* __restrict__ vnext, int outIdx, int outRed,
                                              int post, int dir) {
   const int c = D.segCase[blockIdx.x];
+  if (in_column(D, c)) return;  // every segment of the case
   const bool on = case_on(D, c);
   double acc[1] = {0.0};
   if (on) {
-    const long e0 = 5L * D.segBeg[blockIdx.x], e1 = 5L * D.segEnd[blockIdx.x];
+    const size_t e0 = 5 * (size_t)D.segBeg[blockIdx.x] + threadIdx.x;
+    const int n = 5 * (D.segEnd[blockIdx.x] - D.segBeg[blockIdx.x]) - threadIdx.x;  // entry q MB<TV> exists: q MB<TV> < n
     const TV h = vprev ? TV(D.H[(size_t)c * HSTRIDE + hprevIdx]) : TV(0);
+    TV x[MB_ENTRIES<TV>], p[MB_ENTRIES<TV>], v[MB_ENTRIES<TV>];  // all loads of a thread in flight
+#pragma unroll
+    for (int q = 0; q < MB_ENTRIES<TV>; ++q) {
+      const bool in = q * MB<TV> < n;
+      x[q] = in ? w[e0 + q * MB<TV>] : TV(0);
+      if (vprev) p[q] = in ? vprev[e0 + q * MB<TV>] : TV(0);
+      if (vnext) v[q] = in ? vnext[e0 + q * MB<TV>] : TV(0);
+    }
     TV t = TV(0);
-    for (long e = e0 + threadIdx.x; e < e1; e += CB) {
-      TV x = w[e];
+#pragma unroll
+    for (int q = 0; q < MB_ENTRIES<TV>; ++q) {
       if (vprev) {
-        x -= h * vprev[e];
-        w[e] = x;
+        x[q] -= h * p[q];
+        if (q * MB<TV> < n) w[e0 + q * MB<TV>] = x[q];
       }
-      t += x * (vnext ? vnext[e] : x);
+      t += x[q] * (vnext ? v[q] : x[q]);
     }
     acc[0] = double(t);
   }
   double* out = outRed < 0 ? D.H + (size_t)c * HSTRIDE + outIdx : D.red + 2 * c + outRed;
-  if (case_finish<1>(D, c, acc, out) && on) {
+  if (case_finish<1, MB<TV>>(D, c, acc, out) && on) {
     if (post == 1)
-      case_beta0(D, c);
+      case_beta0(D, c, *out);
     else if (post == 2)
-      case_hess(D, c, dir);
+      case_hess(D, c, dir, *out);
   }
 }
 
 // v = w / beta of the segment's case
 template <typename TV>
-__global__ void __launch_bounds__(CB) k_cscale(CaseDev D, const TV* __restrict__ w, TV* __restrict__ v) {
+__global__ void __launch_bounds__(MB<TV>) k_cscale(CaseDev D, const TV* __restrict__ w, TV* __restrict__ v) {
   const int c = D.segCase[blockIdx.x];
-  if (!case_on(D, c)) return;
-  const TV beta = TV(D.beta[c]);
-  const long e1 = 5L * D.segEnd[blockIdx.x];
-  for (long e = 5L * D.segBeg[blockIdx.x] + threadIdx.x; e < e1; e += CB) v[e] = w[e] / beta;
+  if (in_column(D, c) || !case_on(D, c)) return;
+  const TV b = TV(D.beta[c]), rb = TV(1) / b, rl = rb * fma(-b, rb, TV(1));
+  const size_t e0 = 5 * (size_t)D.segBeg[blockIdx.x] + threadIdx.x;
+  const int n = 5 * (D.segEnd[blockIdx.x] - D.segBeg[blockIdx.x]) - threadIdx.x;
+  TV x[MB_ENTRIES<TV>];
+#pragma unroll
+  for (int q = 0; q < MB_ENTRIES<TV>; ++q) x[q] = q * MB<TV> < n ? w[e0 + q * MB<TV>] : TV(0);
+#pragma unroll
+  for (int q = 0; q < MB_ENTRIES<TV>; ++q)
+    if (q * MB<TV> < n) v[e0 + q * MB<TV>] = quotient(x[q], rb, rl);
 }
 
-// back substitution H y = bh per case (one thread per case)
-__global__ void k_cbacksub(CaseDev D) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+template <typename TV>
+void column_small(Handle& h, cudaStream_t st, const TV* w, TV* V, long vs, int dir) {
+  const CaseDev& D = h.cases.d;
+  const int blocks = COLUMN_BLOCKS * (D.n + (D.n + COLUMN_BLOCKS - 1) / COLUMN_BLOCKS);
+  const int rounds = (5 * h.cases.columnCells + COLUMN_STRIDE - 1) / COLUMN_STRIDE;
+  auto launch = [&](auto kern) {
+    ICS_LAUNCH(h, ICS_K_MGS, kern<<<blocks, COLUMN_THREADS, 0, st>>>(D, w, V, vs, dir));
+  };
+  if (rounds <= 4)
+    launch(k_ccolumn<TV, 4>);
+  else if (rounds <= 16)
+    launch(k_ccolumn<TV, 16>);
+  else
+    launch(k_ccolumn<TV, COLUMN_ROUNDS>);
+}
+
+template <typename TV>
+void column_large(Handle& h, TV* w, TV* V, long vs, int dir) {
+  const CaseDev& D = h.cases.d;
+  const int ns = h.cases.nseg, m = D.m;
+  for (int j = 0; j <= dir; ++j)
+    ICS_LAUNCH(h, ICS_K_MGS,
+               k_cmgs<TV><<<ns, MB<TV>, 0, h.stream>>>(D, w, j > 0 ? V + (size_t)(j - 1) * vs : nullptr, (j - 1) * m + dir,
+                                                   V + (size_t)j * vs, j * m + dir, -1, 0, dir));
+  if (dir < 0)
+    ICS_LAUNCH(h, ICS_K_MGS, k_cmgs<TV><<<ns, MB<TV>, 0, h.stream>>>(D, w, nullptr, 0, nullptr, 0, 0, 1, 0));
+  else
+    ICS_LAUNCH(h, ICS_K_MGS, k_cmgs<TV><<<ns, MB<TV>, 0, h.stream>>>(D, w, V + (size_t)dir * vs, dir * m + dir, nullptr, 0, 1,
+                                                                 2, dir));
+  if (dir + 1 < m)
+    ICS_LAUNCH(h, ICS_K_VECTOR, k_cscale<TV><<<ns, MB<TV>, 0, h.stream>>>(D, w, V + (size_t)(dir + 1) * vs));
+}
+
+// the column of direction dir for every case, each by its own size; where a
+// stack has both, the small ones' launch runs beside the large ones' steps
+// (one after the other 31.5 ms for a step of 8 tubes of 1600 to 40000 cells,
+// beside 29.0)
+template <typename TV>
+void case_column(Handle& h, TV* w, TV* V, long vs, int dir) {
+  const CaseSet& S = h.cases;
+  const bool beside = S.side && !h.prof;
+  if (beside) {
+    ICS_CUDA(cudaEventRecord(S.fork, h.stream));
+    ICS_CUDA(cudaStreamWaitEvent(S.side, S.fork, 0));
+  }
+  if (S.columnCells) column_small<TV>(h, beside ? S.side : h.stream, w, V, vs, dir);
+  if (S.columnLarge) column_large<TV>(h, w, V, vs, dir);
+  if (beside) {
+    ICS_CUDA(cudaEventRecord(S.join, S.side));
+    ICS_CUDA(cudaStreamWaitEvent(h.stream, S.join, 0));
+  }
+}
+
+// back substitution H y = bh per case (one warp per case)
+__global__ void __launch_bounds__(128) k_cbacksub(CaseDev D) {
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (c >= D.n || !case_on(D, c)) return;
   const int m = D.m;
-  const double* H = D.H + (size_t)c * HSTRIDE;
-  const double* bh = D.bh + (size_t)c * (MAX_DIRS + 1);
-  double* y = D.y + (size_t)c * MAX_DIRS;
-  for (int i = m - 1; i >= 0; --i) {
-    double sum = bh[i];
-    for (int j = i + 1; j < m; ++j) sum -= H[i * m + j] * y[j];
-    const double hii = H[i * m + i];
-    const double st = hii >= 0 ? hii + VSMALL : hii - VSMALL;
-    y[i] = sum / st;
+  if (in_column(D, c)) {  // the last column is not rotated yet
+    if ((threadIdx.x & 31) == 0) case_hess(D, c, m - 1, D.red[2 * c + ((m - 1) & 1)]);
+    __syncwarp();
   }
+  back_substitute(D.H + (size_t)c * HSTRIDE, D.bh + (size_t)c * (MAX_DIRS + 1), D.y + (size_t)c * MAX_DIRS, m);
 }
 
 // x += sum_i y_i V_i on the segment's case
@@ -236,7 +390,7 @@ __global__ void __launch_bounds__(CB) k_cresid(CaseDev D, const double* __restri
         acc[k] += fabs(double(v));
       }
   }
-  case_finish<5>(D, c, acc, D.res + 5 * c);
+  case_finish<5, CB>(D, c, acc, D.res + 5 * c);
 }
 
 // per case: the norm-factor sums (rho, rhoE, |rhoU|) of |A (W - avg W)| + |b|
@@ -259,7 +413,7 @@ __global__ void __launch_bounds__(CB) k_cnormfac(CaseDev D, const double* __rest
     acc[6] += fabs(b3);
     acc[7] += fabs(b4);
   }
-  case_finish<8>(D, c, acc, D.nfr + 8 * c);
+  case_finish<8, CB>(D, c, acc, D.nfr + 8 * c);
 }
 
 // per case: the average of W per equation (gAverage)
@@ -271,7 +425,7 @@ __global__ void __launch_bounds__(CB) k_cwavg(CaseDev D, const double* __restric
 #pragma unroll
     for (int k = 0; k < 5; ++k) acc[k] += W[5 * q + k];
   double* avg = D.avg + 5 * c;
-  if (case_finish<5>(D, c, acc, avg)) {
+  if (case_finish<5, CB>(D, c, acc, avg)) {
     const int nc = D.start[c + 1] - D.start[c];
     for (int k = 0; k < 5; ++k) avg[k] = avg[k] / nc;
   }
@@ -293,7 +447,7 @@ __global__ void __launch_bounds__(CB) k_cl2(CaseDev D, const double* __restrict_
   double acc[1] = {0.0};
   const int c1 = D.segEnd[blockIdx.x];
   for (int q = D.segBeg[blockIdx.x] + threadIdx.x; q < c1; q += CB) acc[0] += a[q];
-  case_finish<1>(D, c, acc, D.l2 + c);
+  case_finish<1, CB>(D, c, acc, D.l2 + c);
 }
 
 template <typename TV>
@@ -363,29 +517,16 @@ int gmres_cases_t(Handle& h, std::vector<int>& caseStatus) {
   to_vec(h, h.src, w);
   auto cycle = [&]() {
     precondition(h, w);
-    ICS_LAUNCH(h, ICS_K_MGS, k_cmgs<TV><<<ns, CB, 0, st>>>(D, w, nullptr, 0, nullptr, 0, 0, 1, 0));
-    // with the fused operator (each row scaled by its own case's norm) the
-    // unnormalised vector alternates between w and t, as in the single-system
-    // cycle; the cycle's residual goes back to w
-    TV* wb[2] = {w, t};
+    case_column<TV>(h, w, V, vs, -1);
     for (int i = 0; i < m; ++i) {
-      TV* vi = V + (size_t)i * vs;
-      TV* wc = w;
-      if (fused_operator(h, wb[i & 1], wb[(i + 1) & 1], vi)) {
-        wc = wb[(i + 1) & 1];
-      } else {
-        ICS_LAUNCH(h, ICS_K_VECTOR, k_cscale<TV><<<ns, CB, 0, st>>>(D, w, vi));
+      const TV* vi = V + (size_t)i * vs;
+      if (!fused_operator(h, vi, w)) {
         spmv(h, vi, w);
         precondition(h, w);
       }
-      for (int j = 0; j <= i; ++j) {
-        const TV* vprev = j > 0 ? V + (size_t)(j - 1) * vs : nullptr;
-        ICS_LAUNCH(h, ICS_K_MGS, k_cmgs<TV><<<ns, CB, 0, st>>>(D, wc, vprev, (j - 1) * m + i, V + (size_t)j * vs,
-                                                               j * m + i, -1, 0, i));
-      }
-      ICS_LAUNCH(h, ICS_K_MGS, k_cmgs<TV><<<ns, CB, 0, st>>>(D, wc, vi, i * m + i, nullptr, 0, 1, 2, i));
+      case_column<TV>(h, w, V, vs, i);
     }
-    ICS_LAUNCH(h, ICS_K_SCALAR, k_cbacksub<<<(n + 63) / 64, 64, 0, st>>>(D));
+    ICS_LAUNCH(h, ICS_K_SCALAR, k_cbacksub<<<(n + 3) / 4, 128, 0, st>>>(D));
     ICS_LAUNCH(h, ICS_K_VECTOR, k_cxupdate<TV><<<ns, CB, 0, st>>>(D, x, V, vs));
     spmv(h, x, t);
     ICS_LAUNCH(h, ICS_K_VECTOR, k_cresid<TV><<<ns, CB, 0, st>>>(D, h.src, t, w));
@@ -477,12 +618,12 @@ void free_cases(Handle& h) {
   CaseSet& S = h.cases;
   if (S.mem) cudaFree(S.mem);
   if (S.hres) cudaFreeHost(S.hres);
+  if (S.fork) cudaEventDestroy(S.fork);
+  if (S.join) cudaEventDestroy(S.join);
+  if (S.side) cudaStreamDestroy(S.side);
   S = CaseSet();
   h.m.caseOf = nullptr;
   h.m.caseSer = nullptr;
-  h.m.caseBeta = nullptr;
-  h.m.caseActive = nullptr;
-  h.m.caseStatus = nullptr;
 }
 
 void set_cases(Handle& h, int n, const int* start) {
@@ -573,6 +714,18 @@ void set_cases(Handle& h, int n, const int* start) {
   S.hactive = S.hstatus + n;
   S.n = n;
   S.nseg = ns;
+  for (int k = 0; k < n; ++k) {
+    const int cells = start[k + 1] - start[k];
+    if (cells <= COLUMN_CELLS)
+      S.columnCells = std::max(S.columnCells, cells);
+    else
+      S.columnLarge = true;
+  }
+  if (S.columnCells && S.columnLarge) {
+    ICS_CUDA(cudaStreamCreateWithFlags(&S.side, cudaStreamNonBlocking));
+    ICS_CUDA(cudaEventCreateWithFlags(&S.fork, cudaEventDisableTiming));
+    ICS_CUDA(cudaEventCreateWithFlags(&S.join, cudaEventDisableTiming));
+  }
   S.start.assign(start, start + n + 1);
   S.ctl.assign(n, PseudoControl());
   S.initRes.assign(5 * n, 0.0);
@@ -584,9 +737,6 @@ void set_cases(Handle& h, int n, const int* start) {
   S.cycles.assign(n, 0);
   h.m.caseOf = S.caseOf;
   h.m.caseSer = S.ser;
-  h.m.caseBeta = D.beta;
-  h.m.caseActive = D.active;
-  h.m.caseStatus = D.status;
 }
 
 int gmres_cases(Handle& h, std::vector<int>& caseStatus) {

@@ -60,15 +60,6 @@ __device__ __forceinline__ void copy_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
 }
 
-// the FP32 value as FP64 without the FP64 pipe (which a conversion occupies
-// as long as an addition): the exponent is rebiased in integers
-__device__ __forceinline__ double widen(float f) {
-  const unsigned b = __float_as_uint(f), e = (b >> 23) & 0xff;
-  if (e == 0 || e == 0xff) return double(f);
-  return __hiloint2double((b & 0x80000000u) | ((e + 896u) << 20) | ((b & 0x7fffffu) >> 3), (b & 7u) << 29);
-}
-__device__ __forceinline__ double widen(double f) { return f; }
-
 __device__ __forceinline__ void zero16(float4& x) { x = make_float4(0, 0, 0, 0); }
 __device__ __forceinline__ void zero16(double2& x) { x = make_double2(0, 0); }
 
@@ -86,12 +77,6 @@ __device__ __forceinline__ typename V16<TV>::T load16(const TV* p, long q, long 
   return v;
 }
 
-// x / b from the reciprocal r = fl(1/b) and its error term rl = r (1 - b r):
-// two operations, within a half unit and 2^-50 of the quotient
-template <typename TV>
-__device__ __forceinline__ TV quotient(TV x, TV r, TV rl) {
-  return fma(x, r, x * rl);
-}
 __device__ __forceinline__ float4 quotient16(const float4& x, float r, float rl) {
   return make_float4(quotient(x.x, r, rl), quotient(x.y, r, rl), quotient(x.z, r, rl), quotient(x.w, r, rl));
 }

@@ -179,37 +179,17 @@ __global__ void __launch_bounds__(128) k_cyc_mv(DevMesh m, const TB* __restrict_
 // of operations: one product per slot in pass 2 (98k rows: 94 -> 45 us) and
 // products accumulated by multiply-adds (pass 1 52 -> 37, pass 3 45 -> 39 us);
 // the FP32 passes are bound by HBM and did not change.
-// SCALED (stacked cases): x is the unnormalised Krylov vector; the kernels use
-// x * (1/beta) (the next basis vector) and store it in vout for their own rows,
-// which removes the separate normalisation pass.  One reciprocal per thread: a
-// division per gathered element would make the FP64 path ALU-bound.
-template <bool SCALED, typename TV>
-__device__ __forceinline__ TV ldx(const TV* __restrict__ x, size_t i, TV rbeta) {
-  return SCALED ? x[i] * rbeta : x[i];
-}
-// the reciprocal norm of row c's stacked case
-template <typename TV>
-__device__ __forceinline__ TV row_rbeta(const DevMesh& m, int c) {
-  const int k = m.caseOf[c];
-  return m.caseActive[k] && m.caseStatus[k] == 0 ? TV(1.0 / m.caseBeta[k]) : TV(1);
-}
-
-template <typename TB, typename TV, int MINB = 1, int UNR = 1, bool SCALED = false>
+template <typename TB, typename TV, int MINB = 1, int UNR = 1>
 __global__ void __launch_bounds__(128, MINB) k_op_level0(DevMesh m, const TB* __restrict__ blk, const TB* __restrict__ dg,
                                                    const TV* __restrict__ x, TV* __restrict__ w,
-                                                   const int* __restrict__ cells, int start, int count,
-                                                   TV* __restrict__ vout) {
+                                                   const int* __restrict__ cells, int start, int count) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   const int c = cells ? cells[start + i] : start + i;
   const int s = c >> 5, lane = c & 31;
-  const TV beta = SCALED ? row_rbeta<TV>(m, c) : TV(1);  // reciprocal
   TV xc[5], acc[5];
 #pragma unroll
-  for (int k = 0; k < 5; ++k) xc[k] = ldx<SCALED>(x, 5 * (size_t)c + k, beta);
-  if (SCALED)
-#pragma unroll
-    for (int k = 0; k < 5; ++k) vout[5 * c + k] = xc[k];
+  for (int k = 0; k < 5; ++k) xc[k] = x[5 * (size_t)c + k];
   const TB* D = dg + (size_t)s * 25 * 32 + lane;
 #pragma unroll
   for (int r = 0; r < 5; ++r) {
@@ -228,7 +208,7 @@ __global__ void __launch_bounds__(128, MINB) k_op_level0(DevMesh m, const TB* __
   int colB = ns > 1 ? sc[32] : 0;
   TV xn[5];
 #pragma unroll
-  for (int k = 0; k < 5; ++k) xn[k] = ns > 0 ? ldx<SCALED>(x, 5 * (size_t)colA + k, beta) : TV(0);
+  for (int k = 0; k < 5; ++k) xn[k] = ns > 0 ? x[5 * (size_t)colA + k] : TV(0);
 #pragma unroll UNR
   for (int t = 0; t < ns; ++t) {
     const int col = colA;
@@ -239,7 +219,7 @@ __global__ void __launch_bounds__(128, MINB) k_op_level0(DevMesh m, const TB* __
     if (t + 2 < ns) colB = sc[(t + 2) * 32];
     if (t + 1 < ns)
 #pragma unroll
-      for (int k = 0; k < 5; ++k) xn[k] = ldx<SCALED>(x, 5 * (size_t)colA + k, beta);
+      for (int k = 0; k < 5; ++k) xn[k] = x[5 * (size_t)colA + k];
     SlotBlock<TB> Bk;
     Bk.load(blk, base + t, lane);
     Bk.template mac<1>(g, xj, acc);
@@ -253,29 +233,25 @@ __global__ void __launch_bounds__(128, MINB) k_op_level0(DevMesh m, const TB* __
       const TV d = TV(Vc * m.Dhb[J * m.nInst + K]);
       const TV* xk = x + 5 * ((size_t)K * m.Nc + cl);
 #pragma unroll
-      for (int k = 0; k < 5; ++k) acc[k] += d * ldx<SCALED>(xk, k, beta);
+      for (int k = 0; k < 5; ++k) acc[k] += d * xk[k];
     }
   }
 #pragma unroll
   for (int k = 0; k < 5; ++k) w[5 * c + k] = acc[k];
 }
 
-template <typename TB, typename TV, int MINB = 1, int UNR = 1, bool SCALED = false>
+template <typename TB, typename TV, int MINB = 1, int UNR = 1>
 __global__ void __launch_bounds__(128, MINB) k_op_level1(DevMesh m, const TB* __restrict__ blk, const TB* __restrict__ dg,
                                                    const TB* __restrict__ rD, const TV* __restrict__ x,
                                                    TV* __restrict__ w, const int* __restrict__ cells, int start,
-                                                   int count, TV* __restrict__ vout) {
+                                                   int count) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   const int c = cells ? cells[start + i] : start + i;
   const int s = c >> 5, lane = c & 31;
-  const TV beta = SCALED ? row_rbeta<TV>(m, c) : TV(1);  // reciprocal
   TV xc[5], acc[5];
 #pragma unroll
-  for (int k = 0; k < 5; ++k) xc[k] = ldx<SCALED>(x, 5 * (size_t)c + k, beta);
-  if (SCALED)
-#pragma unroll
-    for (int k = 0; k < 5; ++k) vout[5 * c + k] = xc[k];
+  for (int k = 0; k < 5; ++k) xc[k] = x[5 * (size_t)c + k];
   const TB* D = dg + (size_t)s * 25 * 32 + lane;
 #pragma unroll
   for (int r = 0; r < 5; ++r) {
@@ -294,7 +270,7 @@ __global__ void __launch_bounds__(128, MINB) k_op_level1(DevMesh m, const TB* __
     // the product's x_j and the sweep's rD w_j meet the same block: one product
     TV xj[5];
 #pragma unroll
-    for (int k = 0; k < 5; ++k) xj[k] = ldx<SCALED>(x, 5 * (size_t)col + k, beta) - rj * w[5 * col + k];
+    for (int k = 0; k < 5; ++k) xj[k] = x[5 * (size_t)col + k] - rj * w[5 * col + k];
     SlotBlock<TB> Bk;
     Bk.load(blk, base + t, lane);
     Bk.template mac<1>(g, xj, acc);
@@ -308,7 +284,7 @@ __global__ void __launch_bounds__(128, MINB) k_op_level1(DevMesh m, const TB* __
       const TV d = TV(Vc * m.Dhb[J * m.nInst + K]);
       const TV* xk = x + 5 * ((size_t)K * m.Nc + cl);
 #pragma unroll
-      for (int k = 0; k < 5; ++k) acc[k] += d * ldx<SCALED>(xk, k, beta);
+      for (int k = 0; k < 5; ++k) acc[k] += d * xk[k];
     }
   }
   const TV rc = TV(rD[c]);
@@ -1025,10 +1001,8 @@ static bool fused_op_available(const Handle& h) {
          m.ncyc == 0;
 }
 
-// vout != nullptr (stacked cases): x is unnormalised; v = x / beta is stored in
-// vout and w = M^-1 A v (w must then differ from x)
 template <typename TB, typename TV>
-static bool fused_op_t(Handle& h, const TV* x, TV* w, TV* vout = nullptr) {
+static bool fused_op_t(Handle& h, const TV* x, TV* w) {
   const DevMesh& m = h.m;
   if (!fused_op_available<TB, TV>(h)) return false;
   const TB* blk = (const TB*)h.blk;
@@ -1051,22 +1025,12 @@ static bool fused_op_t(Handle& h, const TV* x, TV* w, TV* vout = nullptr) {
   // in flight or the compiler's register choice (72-80), and 10 or 12 blocks
   // (51 / 40 registers, the latter spilling) were not faster; FP64 would spill
   constexpr int OPB = sizeof(TB) == 4 ? 8 : 1;
-  if (n0) {
-    if (vout)
-      ICS_LAUNCH(h, ICS_K_OP0, k_op_level0<TB, TV, OPB, 1, true><<<grid_for(n0, 128), 128, 0, h.stream>>>(
-                                   m, blk, dg, x, w, c0, s0, n0, vout));
-    else
-      ICS_LAUNCH(h, ICS_K_OP0, k_op_level0<TB, TV, OPB, 1><<<grid_for(n0, 128), 128, 0, h.stream>>>(
-                                   m, blk, dg, x, w, c0, s0, n0, nullptr));
-  }
-  if (n1) {
-    if (vout)
-      ICS_LAUNCH(h, ICS_K_OP1, k_op_level1<TB, TV, OPB, 1, true><<<grid_for(n1, 128), 128, 0, h.stream>>>(
-                                   m, blk, dg, rD, x, w, c1, s1, n1, vout));
-    else
-      ICS_LAUNCH(h, ICS_K_OP1, k_op_level1<TB, TV, OPB, 1><<<grid_for(n1, 128), 128, 0, h.stream>>>(
-                                   m, blk, dg, rD, x, w, c1, s1, n1, nullptr));
-  }
+  if (n0)
+    ICS_LAUNCH(h, ICS_K_OP0, k_op_level0<TB, TV, OPB, 1><<<grid_for(n0, 128), 128, 0, h.stream>>>(m, blk, dg, x, w, c0,
+                                                                                                 s0, n0));
+  if (n1)
+    ICS_LAUNCH(h, ICS_K_OP1, k_op_level1<TB, TV, OPB, 1><<<grid_for(n1, 128), 128, 0, h.stream>>>(m, blk, dg, rD, x, w,
+                                                                                                 c1, s1, n1));
   // reverse level 1 = forward level 0 rows
   const int a = m.rl_ptr[1], cnt = m.rl_ptr[2] - a;
   const bool contig = m.rl_cstart[1] >= 0;
@@ -1111,10 +1075,9 @@ void lusgs_with(Handle& h, const void* blk, const void* rD, bool fp32, double* r
   ICS_CUDA(cudaGetLastError());
 }
 
-bool fused_operator(Handle& h, const void* x, void* w, void* vout) {
-  if (prec(h) == ICS_PREC_MIXED)
-    return fused_op_t<float, float>(h, (const float*)x, (float*)w, (float*)vout);
-  return fused_op_t<double, double>(h, (const double*)x, (double*)w, (double*)vout);
+bool fused_operator(Handle& h, const void* x, void* w) {
+  if (prec(h) == ICS_PREC_MIXED) return fused_op_t<float, float>(h, (const float*)x, (float*)w);
+  return fused_op_t<double, double>(h, (const double*)x, (double*)w);
 }
 
 void sweep_probe(Handle& h, const int* order, int tickets, int spin_limit) {
