@@ -37,7 +37,7 @@ enum { Q_RHO = 0, Q_P = 1, Q_UX = 2, Q_UY = 3, Q_UZ = 4, Q_E = 5, Q_H = 6, Q_C =
 
 constexpr int SLICE = 32;
 constexpr int SWEEP_TICKET = 32;  // rows per ticket of the sync-free LU-SGS sweeps
-constexpr int REDUCE_BLOCKS = 1216;  // 8 x 152 SMs
+constexpr int REDUCE_BLOCKS = 608;  // 4 x 152 SMs
 constexpr int MAX_DIRS = 64;
 constexpr int MAX_INST = ICS_MAX_INSTANCES;  // Harmonic Balance instances
 

@@ -365,11 +365,14 @@ __global__ void __launch_bounds__(CB) k_cxupdate(CaseDev D, TV* __restrict__ x, 
                                                  long vstride) {
   const int c = D.segCase[blockIdx.x];
   if (!case_on(D, c)) return;
-  const double* y = D.y + (size_t)c * MAX_DIRS;
+  __shared__ TV y[MAX_DIRS];  // converted once, not per element
+  if ((int)threadIdx.x < D.m) y[threadIdx.x] = convert<TV>(D.y[(size_t)c * MAX_DIRS + threadIdx.x]);
+  __syncthreads();
   const long e1 = 5L * D.segEnd[blockIdx.x];
   for (long e = 5L * D.segBeg[blockIdx.x] + threadIdx.x; e < e1; e += CB) {
     TV a = x[e];
-    for (int i = 0; i < D.m; ++i) a += TV(y[i]) * V[(size_t)i * vstride + e];
+#pragma unroll 4
+    for (int i = 0; i < D.m; ++i) a += y[i] * V[(size_t)i * vstride + e];
     x[e] = a;
   }
 }
@@ -385,9 +388,9 @@ __global__ void __launch_bounds__(CB) k_cresid(CaseDev D, const double* __restri
     for (int q = D.segBeg[blockIdx.x] + threadIdx.x; q < c1; q += CB)
 #pragma unroll
       for (int k = 0; k < 5; ++k) {
-        const TV v = TV(b[5 * q + k]) - t[5 * q + k];
+        const TV v = convert<TV>(b[5 * q + k]) - t[5 * q + k];
         r[5 * q + k] = v;
-        acc[k] += fabs(double(v));
+        acc[k] += fabs(widen(v));
       }
   }
   case_finish<5, CB>(D, c, acc, D.res + 5 * c);
@@ -401,8 +404,8 @@ __global__ void __launch_bounds__(CB) k_cnormfac(CaseDev D, const double* __rest
   double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   const int c1 = D.segEnd[blockIdx.x];
   for (int q = D.segBeg[blockIdx.x] + threadIdx.x; q < c1; q += CB) {
-    const double t0 = double(t[5 * q]), t4 = double(t[5 * q + 4]);
-    const double t1 = double(t[5 * q + 1]), t2 = double(t[5 * q + 2]), t3 = double(t[5 * q + 3]);
+    const double t0 = widen(t[5 * q]), t4 = widen(t[5 * q + 4]);
+    const double t1 = widen(t[5 * q + 1]), t2 = widen(t[5 * q + 2]), t3 = widen(t[5 * q + 3]);
     const double b0 = b[5 * q], b1 = b[5 * q + 1], b2 = b[5 * q + 2], b3 = b[5 * q + 3], b4 = b[5 * q + 4];
     acc[0] += fabs(t0) + fabs(b0);
     acc[1] += fabs(t4) + fabs(b4);
@@ -438,7 +441,7 @@ __global__ void __launch_bounds__(CB) k_cwmavg(CaseDev D, const double* __restri
   const int c1 = D.segEnd[blockIdx.x];
   for (int q = D.segBeg[blockIdx.x] + threadIdx.x; q < c1; q += CB)
 #pragma unroll
-    for (int k = 0; k < 5; ++k) out[5 * q + k] = TV(W[5 * q + k] - avg[k]);
+    for (int k = 0; k < 5; ++k) out[5 * q + k] = convert<TV>(W[5 * q + k] - avg[k]);
 }
 
 // per case: sum of the cells' (R_rho V)^2
@@ -454,11 +457,11 @@ template <typename TV>
 __global__ void k_cto_dW(int N, const TV* __restrict__ x, double* __restrict__ dW, int s0, int s1, int s2) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= N) return;
-  dW[5 * c] = double(x[5 * c]);
-  dW[5 * c + 1] = s0 == -1 ? 0.0 : double(x[5 * c + 1]);
-  dW[5 * c + 2] = s1 == -1 ? 0.0 : double(x[5 * c + 2]);
-  dW[5 * c + 3] = s2 == -1 ? 0.0 : double(x[5 * c + 3]);
-  dW[5 * c + 4] = double(x[5 * c + 4]);
+  dW[5 * c] = widen(x[5 * c]);
+  dW[5 * c + 1] = s0 == -1 ? 0.0 : widen(x[5 * c + 1]);
+  dW[5 * c + 2] = s1 == -1 ? 0.0 : widen(x[5 * c + 2]);
+  dW[5 * c + 3] = s2 == -1 ? 0.0 : widen(x[5 * c + 3]);
+  dW[5 * c + 4] = widen(x[5 * c + 4]);
 }
 
 // coupledMatrix::solver::stop (coupledMatrixSolver.C:198-221) for one case

@@ -25,65 +25,55 @@
 namespace ics {
 
 // ------------------------------------------------------------------ reduce
-// Returns true on the one thread (thread 0 of the last block) that wrote out[].
+constexpr int RB = 256;  // threads per reduction block
+
+// Returns true on the one thread (thread 0 of the last block) that may read
+// out[] then.
 template <int NV>
 __device__ __forceinline__ bool reduce_finish(double (&v)[NV], double* __restrict__ partials,
                                               unsigned int* __restrict__ counter, double* __restrict__ out) {
-  __shared__ double sm[32][NV];
+  constexpr int G = FOLD_GROUP<NV>;
+  __shared__ double sm[RB / 32][FOLD_VALUES<NV>];
   __shared__ bool amLast;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    double x = v[k];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) sm[warp][k] = x;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const int nw = blockDim.x >> 5;
-    for (int k = 0; k < NV; ++k) {
-      double s = 0;
-      for (int w = 0; w < nw; ++w) s += sm[w][k];
-      partials[blockIdx.x * NV + k] = s;
+  const int k = threadIdx.x / G;
+  const bool writer = threadIdx.x < 32 && threadIdx.x % G == 0 && k < NV;
+  double s = block_sums<NV, RB / 32>(v, sm);
+  if (gridDim.x > 1) {
+    if (threadIdx.x < 32) {
+      if (writer) {
+        partials[blockIdx.x * NV + k] = s;
+        __threadfence();
+      }
+      __syncwarp();
+      if (threadIdx.x == 0) amLast = atomicAdd(counter, 1u) == gridDim.x - 1;
     }
-    __threadfence();
-    const unsigned t = atomicAdd(counter, 1u);
-    amLast = (t == gridDim.x - 1);
-  }
-  __syncthreads();
-  if (amLast) {  // block-uniform: the last block folds all partials in a fixed order
+    __syncthreads();
+    if (!amLast) return false;  // block-uniform: the last block folds all partials in a fixed order
     __threadfence();
     const volatile double* vp = partials;
     double acc[NV];
 #pragma unroll
-    for (int k = 0; k < NV; ++k) acc[k] = 0.0;
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
+    for (int q = 0; q < NV; ++q) acc[q] = 0.0;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += RB)
 #pragma unroll
-      for (int k = 0; k < NV; ++k) acc[k] += vp[b * NV + k];
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      double x = acc[k];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-      if (lane == 0) sm[warp][k] = x;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const int nw = blockDim.x >> 5;
-      for (int k = 0; k < NV; ++k) {
-        double s = 0;
-        for (int w = 0; w < nw; ++w) s += sm[w][k];
-        out[k] = s;
-      }
-      *counter = 0;
-      return true;
-    }
+      for (int q = 0; q < NV; ++q) acc[q] += vp[b * NV + q];
+    s = block_sums<NV, RB / 32>(acc, sm);
+    if (threadIdx.x == 0) *counter = 0;
   }
-  return false;
+  if (threadIdx.x >= 32) return false;
+  if (writer) out[k] = s;
+  __syncwarp();
+  return threadIdx.x == 0;
 }
 
-constexpr int RB = 256;  // threads per reduction block
+// blocks of a reduction over n items: no more than hold one item per thread.
+// A block's folds cost the same whatever it has summed, so idle blocks are not
+// free: with 1216 blocks and a fold per value the residual of 10k cells took
+// 31 us, and the 80 reductions and vector passes of a time step on 1000 cells
+// 1.61 ms instead of 0.67
+inline int reduce_grid(long n) { return (int)std::max(1L, std::min((long)REDUCE_BLOCKS, (n + RB - 1) / RB)); }
+// blocks of an elementwise pass over n items
+inline int pass_grid(long n) { return (int)std::max(1L, std::min(2L * REDUCE_BLOCKS, (n + RB - 1) / RB)); }
 
 // ------------------------------------------------------------------- spmv
 template <typename TB, typename TV>
@@ -761,7 +751,12 @@ __global__ void k_jacobi_apply(int N, const TB* __restrict__ inv, TV* __restrict
 // ------------------------------------------------------------ vector kernels
 template <typename TS, typename TD>
 __global__ void k_cast(long n, const TS* __restrict__ a, TD* __restrict__ b) {
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) b[i] = TD(a[i]);
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+    if constexpr (sizeof(TS) == 4)
+      b[i] = widen(a[i]);
+    else
+      b[i] = convert<TD>(a[i]);
+  }
 }
 
 __device__ __forceinline__ void addmul16(float4& a, float y, const float4& v) {
@@ -775,23 +770,21 @@ __device__ __forceinline__ void addmul16(double2& a, double y, const double2& v)
   a.y += y * v.y;
 }
 
-// the last direction's Givens rotation, then H y = bh
-__global__ void k_backsub(KrylovScalars* ks, int m) {
+// the last direction's Givens rotation, then H y = bh (one warp)
+__global__ void __launch_bounds__(32) k_backsub(KrylovScalars* ks, int m) {
   if (ks->status) return;
-  dev_hess(ks, m - 1, m);
-  for (int i = m - 1; i >= 0; --i) {
-    double sum = ks->bh[i];
-    for (int j = i + 1; j < m; ++j) sum -= ks->H[i * m + j] * ks->y[j];
-    const double hii = ks->H[i * m + i];
-    const double st = hii >= 0 ? hii + VSMALL : hii - VSMALL;
-    ks->y[i] = sum / st;
-  }
+  if (threadIdx.x == 0) dev_hess(ks, m - 1, m);
+  __syncwarp();
+  back_substitute(ks->H, ks->bh, ks->y, m);
 }
 
 template <typename TV>
-__global__ void k_xupdate(long n, TV* __restrict__ x, const TV* __restrict__ V, const KrylovScalars* __restrict__ ks,
-                          int m, long vstride) {
+__global__ void __launch_bounds__(RB) k_xupdate(long n, TV* __restrict__ x, const TV* __restrict__ V,
+                                                const KrylovScalars* __restrict__ ks, int m, long vstride) {
+  __shared__ TV y[MAX_DIRS];  // converted once, not per element
   if (ks->status) return;
+  if ((int)threadIdx.x < m) y[threadIdx.x] = convert<TV>(ks->y[threadIdx.x]);
+  __syncthreads();
   using VT = typename V16<TV>::T;
   constexpr int L = V16<TV>::n;
   const long nv = n / L;
@@ -799,13 +792,13 @@ __global__ void k_xupdate(long n, TV* __restrict__ x, const TV* __restrict__ V, 
   VT* x4 = reinterpret_cast<VT*>(x);
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < nv; q += stride) {
     VT a = x4[q];
-    for (int i = 0; i < m; ++i)
-      addmul16(a, TV(ks->y[i]), reinterpret_cast<const VT*>(V + (size_t)i * vstride)[q]);
+#pragma unroll 4
+    for (int i = 0; i < m; ++i) addmul16(a, y[i], reinterpret_cast<const VT*>(V + (size_t)i * vstride)[q]);
     x4[q] = a;
   }
   for (long q = nv * L + blockIdx.x * (long)blockDim.x + threadIdx.x; q < n; q += stride) {
     TV a = x[q];
-    for (int i = 0; i < m; ++i) a += TV(ks->y[i]) * V[(size_t)i * vstride + q];
+    for (int i = 0; i < m; ++i) a += y[i] * V[(size_t)i * vstride + q];
     x[q] = a;
   }
 }
@@ -830,9 +823,9 @@ __global__ void __launch_bounds__(RB) k_resid(int Nc, const double* __restrict__
   for (int c = inst_ * Nc + blockIdx.x * blockDim.x + threadIdx.x; c < cend_; c += gridDim.x * blockDim.x) {
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
-      const TV v = TV(b[5 * c + k]) - t[5 * c + k];
+      const TV v = convert<TV>(b[5 * c + k]) - t[5 * c + k];
       r[5 * c + k] = v;
-      acc[k] += fabs(double(v));
+      acc[k] += fabs(widen(v));
     }
   }
   reduce_finish<5>(acc, partials, counter, out);
@@ -848,8 +841,8 @@ __global__ void __launch_bounds__(RB) k_normfac(int Nc, const double* __restrict
   ICS_INSTANCE_RANGE(Nc)
   double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   for (int c = inst_ * Nc + blockIdx.x * blockDim.x + threadIdx.x; c < cend_; c += gridDim.x * blockDim.x) {
-    const double t0 = double(t[5 * c]), t4 = double(t[5 * c + 4]);
-    const double t1 = double(t[5 * c + 1]), t2 = double(t[5 * c + 2]), t3 = double(t[5 * c + 3]);
+    const double t0 = widen(t[5 * c]), t4 = widen(t[5 * c + 4]);
+    const double t1 = widen(t[5 * c + 1]), t2 = widen(t[5 * c + 2]), t3 = widen(t[5 * c + 3]);
     const double b0 = b[5 * c], b1 = b[5 * c + 1], b2 = b[5 * c + 2], b3 = b[5 * c + 3], b4 = b[5 * c + 4];
     acc[0] += fabs(t0) + fabs(b0);
     acc[1] += fabs(t4) + fabs(b4);
@@ -863,7 +856,8 @@ __global__ void __launch_bounds__(RB) k_normfac(int Nc, const double* __restrict
   reduce_finish<8>(acc, partials, counter, out);
 }
 
-__global__ void __launch_bounds__(RB) k_wsum(int Nc, const double* __restrict__ W, double* __restrict__ partials,
+// the averages of W per equation and instance (gAverage)
+__global__ void __launch_bounds__(RB) k_wavg(int Nc, const double* __restrict__ W, double* __restrict__ partials,
                                              unsigned int* __restrict__ counter, double* __restrict__ out) {
   constexpr int NV_ = 5;
   ICS_INSTANCE_RANGE(Nc)
@@ -871,7 +865,8 @@ __global__ void __launch_bounds__(RB) k_wsum(int Nc, const double* __restrict__ 
   for (int c = inst_ * Nc + blockIdx.x * blockDim.x + threadIdx.x; c < cend_; c += gridDim.x * blockDim.x)
 #pragma unroll
     for (int k = 0; k < 5; ++k) acc[k] += W[5 * c + k];
-  reduce_finish<5>(acc, partials, counter, out);
+  if (reduce_finish<5>(acc, partials, counter, out))
+    for (int k = 0; k < 5; ++k) out[k] = out[k] / Nc;
 }
 
 template <typename TV>
@@ -881,23 +876,18 @@ __global__ void k_wmavg(int N, int Nc, const double* __restrict__ W, const Krylo
   if (c >= N) return;
   const double* avg = ks->avg + 5 * (c / Nc);
 #pragma unroll
-  for (int k = 0; k < 5; ++k) out[5 * c + k] = TV(W[5 * c + k] - avg[k]);
-}
-
-// instance averages (gAverage per field) from the instance sums
-__global__ void k_avg(KrylovScalars* ks, int Nc, int nInst) {
-  for (int k = 0; k < 5 * nInst; ++k) ks->avg[k] = ks->avg[k] / Nc;
+  for (int k = 0; k < 5; ++k) out[5 * c + k] = convert<TV>(W[5 * c + k] - avg[k]);
 }
 
 template <typename TV>
 __global__ void k_to_dW(int N, const TV* __restrict__ x, double* __restrict__ dW, int s0, int s1, int s2) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= N) return;
-  dW[5 * c] = double(x[5 * c]);
-  dW[5 * c + 1] = s0 == -1 ? 0.0 : double(x[5 * c + 1]);
-  dW[5 * c + 2] = s1 == -1 ? 0.0 : double(x[5 * c + 2]);
-  dW[5 * c + 3] = s2 == -1 ? 0.0 : double(x[5 * c + 3]);
-  dW[5 * c + 4] = double(x[5 * c + 4]);
+  dW[5 * c] = widen(x[5 * c]);
+  dW[5 * c + 1] = s0 == -1 ? 0.0 : widen(x[5 * c + 1]);
+  dW[5 * c + 2] = s1 == -1 ? 0.0 : widen(x[5 * c + 2]);
+  dW[5 * c + 3] = s2 == -1 ? 0.0 : widen(x[5 * c + 3]);
+  dW[5 * c + 4] = widen(x[5 * c + 4]);
 }
 
 __global__ void __launch_bounds__(RB) k_sumsq(int N, const double* __restrict__ a, double* __restrict__ partials,
@@ -1107,7 +1097,7 @@ int precondition(Handle& h, void* r) {
 void to_vec(Handle& h, const double* src, void* dst) {
   const long n = 5L * h.m.N;
   if (prec(h) == ICS_PREC_MIXED)
-    ICS_LAUNCH(h, ICS_K_VECTOR, k_cast<double, float><<<REDUCE_BLOCKS, RB, 0, h.stream>>>(n, src, (float*)dst));
+    ICS_LAUNCH(h, ICS_K_VECTOR, k_cast<double, float><<<pass_grid(n), RB, 0, h.stream>>>(n, src, (float*)dst));
   else
     ICS_CUDA(cudaMemcpyAsync(dst, src, n * sizeof(double), cudaMemcpyDeviceToDevice, h.stream));
 }
@@ -1115,7 +1105,7 @@ void to_vec(Handle& h, const double* src, void* dst) {
 void from_vec(Handle& h, const void* src, double* dst) {
   const long n = 5L * h.m.N;
   if (prec(h) == ICS_PREC_MIXED)
-    ICS_LAUNCH(h, ICS_K_VECTOR, k_cast<float, double><<<REDUCE_BLOCKS, RB, 0, h.stream>>>(n, (const float*)src, dst));
+    ICS_LAUNCH(h, ICS_K_VECTOR, k_cast<float, double><<<pass_grid(n), RB, 0, h.stream>>>(n, (const float*)src, dst));
   else
     ICS_CUDA(cudaMemcpyAsync(dst, src, n * sizeof(double), cudaMemcpyDeviceToDevice, h.stream));
 }
@@ -1147,8 +1137,7 @@ static bool stop_test(const Handle& h, const ResIO& r) {
 
 // grid of the per-instance reductions: the instances share REDUCE_BLOCKS
 static dim3 inst_grid(const Handle& h) {
-  const int bx = REDUCE_BLOCKS / h.m.nInst;
-  return dim3(bx < 1 ? 1 : bx, h.m.nInst);
+  return dim3(std::max(1, std::min(REDUCE_BLOCKS / h.m.nInst, reduce_grid(h.m.Nc))), h.m.nInst);
 }
 
 // final L1 residuals from the per-instance sums in h.ksHost->res; false when
@@ -1178,8 +1167,7 @@ static void norm_factors_t(Handle& h, std::vector<double>& nf, ResIO& r) {
   TV* t = (TV*)h.kt;
   const dim3 g = inst_grid(h);
   ICS_CUDA(cudaMemsetAsync(&ks->status, 0, sizeof(int), st));
-  ICS_LAUNCH(h, ICS_K_VECTOR, k_wsum<<<g, RB, 0, st>>>(Nc, h.W, h.partials, h.counter, ks->avg));
-  ICS_LAUNCH(h, ICS_K_SCALAR, k_avg<<<1, 1, 0, st>>>(ks, Nc, nI));
+  ICS_LAUNCH(h, ICS_K_VECTOR, k_wavg<<<g, RB, 0, st>>>(Nc, h.W, h.partials, h.counter, ks->avg));
   ICS_LAUNCH(h, ICS_K_VECTOR, k_wmavg<TV><<<grid_for(N, 256), 256, 0, st>>>(N, Nc, h.W, ks, w));
   spmv_t<TB, TV>(h, w, t);
   ICS_LAUNCH(h, ICS_K_VECTOR, k_normfac<TV><<<g, RB, 0, st>>>(Nc, h.src, t, h.partials, h.counter, ks->nfr));
@@ -1307,8 +1295,8 @@ static int gmres_t(Handle& h, ResIO& p) {
       }
       krylov_column(h, sizeof(TV) == 4, n5, w, V, vs, i, m);
     }
-    ICS_LAUNCH(h, ICS_K_SCALAR, k_backsub<<<1, 1, 0, st>>>(ks, m));
-    ICS_LAUNCH(h, ICS_K_VECTOR, k_xupdate<TV><<<REDUCE_BLOCKS, RB, 0, st>>>(n5, x, V, ks, m, vs));
+    ICS_LAUNCH(h, ICS_K_SCALAR, k_backsub<<<1, 32, 0, st>>>(ks, m));
+    ICS_LAUNCH(h, ICS_K_VECTOR, k_xupdate<TV><<<pass_grid(n5 / V16<TV>::n), RB, 0, st>>>(n5, x, V, ks, m, vs));
     spmv_t<TB, TV>(h, x, t);
     ICS_LAUNCH(h, ICS_K_VECTOR,
                k_resid<TV><<<inst_grid(h), RB, 0, st>>>(h.m.Nc, h.src, t, w, h.partials, h.counter, ks->res));
@@ -1451,7 +1439,7 @@ void autotune_linalg(Handle& h, std::vector<std::pair<std::string, double>>& log
 
 // sum of a device array (deterministic fixed-order reduction)
 double device_sum(Handle& h, const double* a, int n) {
-  ICS_LAUNCH(h, ICS_K_VECTOR, k_sumsq<<<REDUCE_BLOCKS, RB, 0, h.stream>>>(n, a, h.partials, h.counter, &h.ks->red[8]));
+  ICS_LAUNCH(h, ICS_K_VECTOR, k_sumsq<<<reduce_grid(n), RB, 0, h.stream>>>(n, a, h.partials, h.counter, &h.ks->red[8]));
   double v = 0;
   ICS_CUDA(cudaMemcpyAsync(&v, &h.ks->red[8], sizeof(double), cudaMemcpyDeviceToHost, h.stream));
   ICS_CUDA(cudaStreamSynchronize(h.stream));
@@ -1462,7 +1450,7 @@ double device_sum(Handle& h, const double* a, int n) {
 // whether every entry of the source is finite; host_src (if not null) receives
 // the source in the same wait
 double rho_l2(Handle& h, double* host_src, bool* finite) {
-  ICS_LAUNCH(h, ICS_K_VECTOR, k_sumsq<<<REDUCE_BLOCKS, RB, 0, h.stream>>>(h.m.N, h.scratch, h.partials, h.counter, &h.ks->l2));
+  ICS_LAUNCH(h, ICS_K_VECTOR, k_sumsq<<<reduce_grid(h.m.N), RB, 0, h.stream>>>(h.m.N, h.scratch, h.partials, h.counter, &h.ks->l2));
   struct {
     double l2;
     int nonfinite, status;
@@ -1659,10 +1647,10 @@ int scalar_gmres(Handle& h, double* dx, ics_solver_perf* perf) {
   double* t = (double*)h.kt;
   double* red = ks->red;
   ICS_CUDA(cudaMemsetAsync(&ks->status, 0, sizeof(int), st));
-  ICS_LAUNCH(h, ICS_K_PASSIVE, k_s_sum<<<REDUCE_BLOCKS, RB, 0, st>>>(N, h.srhoS, h.partials, h.counter, &red[2]));
+  ICS_LAUNCH(h, ICS_K_PASSIVE, k_s_sum<<<reduce_grid(N), RB, 0, st>>>(N, h.srhoS, h.partials, h.counter, &red[2]));
   ICS_LAUNCH(h, ICS_K_PASSIVE, k_s_wmavg<<<grid_for(N, 256), 256, 0, st>>>(N, h.srhoS, &red[2], w));
   s_spmv(h, w, t);
-  ICS_LAUNCH(h, ICS_K_PASSIVE, k_s_normfac<<<REDUCE_BLOCKS, RB, 0, st>>>(N, h.ssrc, t, h.partials, h.counter, &red[3]));
+  ICS_LAUNCH(h, ICS_K_PASSIVE, k_s_normfac<<<reduce_grid(N), RB, 0, st>>>(N, h.ssrc, t, h.partials, h.counter, &red[3]));
   double hv[2];
   ICS_CUDA(cudaMemcpyAsync(hv, &red[3], 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
   ICS_CUDA(cudaStreamSynchronize(st));
@@ -1682,10 +1670,10 @@ int scalar_gmres(Handle& h, double* dx, ics_solver_perf* perf) {
       s_precondition(h, w);
       krylov_column(h, false, N, w, V, vs, i, m);
     }
-    ICS_LAUNCH(h, ICS_K_SCALAR, k_backsub<<<1, 1, 0, st>>>(ks, m));
-    ICS_LAUNCH(h, ICS_K_VECTOR, k_xupdate<double><<<REDUCE_BLOCKS, RB, 0, st>>>(N, dx, V, ks, m, vs));
+    ICS_LAUNCH(h, ICS_K_SCALAR, k_backsub<<<1, 32, 0, st>>>(ks, m));
+    ICS_LAUNCH(h, ICS_K_VECTOR, k_xupdate<double><<<pass_grid(N / 2), RB, 0, st>>>(N, dx, V, ks, m, vs));
     s_spmv(h, dx, t);
-    ICS_LAUNCH(h, ICS_K_PASSIVE, k_s_resid<<<REDUCE_BLOCKS, RB, 0, st>>>(N, h.ssrc, t, w, h.partials, h.counter,
+    ICS_LAUNCH(h, ICS_K_PASSIVE, k_s_resid<<<reduce_grid(N), RB, 0, st>>>(N, h.ssrc, t, w, h.partials, h.counter,
                                                                          &red[5]));
     double rs = 0;
     int stt = 0;

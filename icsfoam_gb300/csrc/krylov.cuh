@@ -40,14 +40,31 @@ __device__ __forceinline__ double dot16(const double2& a, const double2& b, doub
   return fma(a.y, b.y, fma(a.x, b.x, acc));
 }
 
-// the FP32 value as FP64 without the FP64 pipe (which a conversion occupies
-// as long as an addition): the exponent is rebiased in integers
+// Conversions without the FP64 pipe (which a conversion occupies as long as an
+// addition): the exponent is rebiased in integers, and FP64 to FP32 rounds to
+// nearest even.  Subnormal numbers, infinities and NaN take the conversion.
 __device__ __forceinline__ double widen(float f) {
-  const unsigned b = __float_as_uint(f), e = (b >> 23) & 0xff;
-  if (e == 0 || e == 0xff) return double(f);
-  return __hiloint2double((b & 0x80000000u) | ((e + 896u) << 20) | ((b & 0x7fffffu) >> 3), (b & 7u) << 29);
+  const unsigned b = __float_as_uint(f), a = b & 0x7fffffffu, sign = b & 0x80000000u;
+  if (a - 0x00800000u < 0x7f000000u) return __hiloint2double(sign | ((a >> 3) + (896u << 20)), b << 29);
+  return a == 0 ? __hiloint2double(sign, 0) : double(f);
 }
 __device__ __forceinline__ double widen(double f) { return f; }
+
+__device__ __forceinline__ float narrow(double d) {
+  const unsigned hi = __double2hiint(d), lo = __double2loint(d), a = hi & 0x7fffffffu, sign = hi & 0x80000000u;
+  if (a - (897u << 20) < (253u << 20)) {  // a result of exponent 2^-126 .. 2^126, whose rounding may carry
+    const unsigned f = ((a - (896u << 20)) << 3) | (lo >> 29), rest = lo & 0x1fffffffu;
+    return __uint_as_float(sign | (f + (rest > 0x10000000u - (f & 1))));
+  }
+  return (a | lo) == 0 ? __uint_as_float(sign) : float(d);
+}
+template <typename TD>
+__device__ __forceinline__ TD convert(double x) {
+  if constexpr (sizeof(TD) == 4)
+    return narrow(x);
+  else
+    return x;
+}
 
 // x / b from the reciprocal r = fl(1/b) and its error term rl = r (1 - b r):
 // two operations, within a half unit and 2^-50 of the quotient
@@ -193,22 +210,9 @@ __device__ __forceinline__ void back_substitute(const double* __restrict__ H, co
 }
 
 // after the Gram-Schmidt of direction i: H[j][i] for j <= i are in H, nrm2[i]
-// holds |w|^2; rotate column i with the previous Givens rotations and make a
-// new one (gmres.C:1013-1027, rotation gmres.C:44-69)
+// holds |w|^2
 __device__ __forceinline__ void dev_hess(KrylovScalars* ks, int i, int m) {
-  if (ks->status) return;
-  double* H = ks->H;
-  const double beta = sqrt(ks->nrm2[i]);
-  for (int j = 0; j < i; ++j) {
-    const double Hji = H[j * m + i];
-    H[j * m + i] = ks->c[j] * Hji - ks->s[j] * H[(j + 1) * m + i];
-    H[(j + 1) * m + i] = ks->s[j] * Hji + ks->c[j] * H[(j + 1) * m + i];
-  }
-  givens(H[i * m + i], beta, ks->c[i], ks->s[i]);
-  const double bhi = ks->bh[i];
-  ks->bh[i] = ks->c[i] * bhi - ks->s[i] * ks->bh[i + 1];
-  ks->bh[i + 1] = ks->s[i] * bhi + ks->c[i] * ks->bh[i + 1];
-  H[i * m + i] = ks->c[i] * H[i * m + i] - ks->s[i] * beta;
+  if (!ks->status) hess_column(ks->H, ks->c, ks->s, ks->bh, i, m, ks->nrm2[i]);
 }
 
 // start of a cycle: bh = (beta, 0...)
