@@ -118,7 +118,7 @@ struct SlotBlock<float> {
     return e;
   }
 
- private:
+  // what a product needs of the words alone
   template <typename TV>
   struct Terms {
     TV a2, S0, S1, S2, U0, U1, U2, th, a1, pu, c;

@@ -452,9 +452,9 @@ __global__ void __launch_bounds__(128) k_lusgs_level(DevMesh m, const TB* __rest
 constexpr int SWEEP_SPIN_LIMIT = 1 << 22;
 constexpr int SWEEP_PAD = 8;  // words per row of the sweep outputs
 constexpr int SWEEP_THREADS = 32;  // one warp per block
-// rows a warp takes at once (sweep_row16 / sweep_row)
+// rows a warp takes at once (sweep_row16 / sweep_row4)
 template <typename TB, typename TV>
-constexpr int sweep_rows = sizeof(TB) == 8 && sizeof(TV) == 8 ? 2 : SWEEP_TICKET;
+constexpr int sweep_rows = sizeof(TB) == 8 && sizeof(TV) == 8 ? 2 : 8;
 
 __device__ __forceinline__ int ld_relaxed_int(const int* p) {
   int v;
@@ -500,6 +500,10 @@ __device__ __forceinline__ bool sweep_ready(const TV* v) {
          sweep_word_set(v[4]);
 }
 
+// FWD: in = the right-hand side r (5 words per row), out = the forward
+// result; !FWD: in = the forward result (padded), out = the reverse result,
+// also written to r (5 words per row).  `out` holds the sentinel on entry.
+//
 // FP64 rows, 16 lanes each (two rows per warp): lane (p, i) = (lane / 5, lane
 // % 5) of a row handles component i of its p-th neighbour of three, so the
 // three neighbours are polled, scaled and multiplied at once.  GB300 issues a
@@ -596,113 +600,95 @@ __device__ __forceinline__ void sweep_row16(const DevMesh& m, const TB* __restri
   }
 }
 
-// FWD: in = the right-hand side r (5 words per row), out = the forward
-// result; !FWD: in = the forward result (padded), out = the reverse result,
-// also written to r (5 words per row).  `out` holds the sentinel on entry.
+// Rows with FP32 blocks, 4 lanes each (eight rows per warp): lane p of a row polls,
+// scales and multiplies its p-th neighbour of three, lane 0 subtracts the
+// products in the order of lusgs_fwd_row / lusgs_rev_row.  A level costs the
+// L2 path of its results and the row's dependent instructions, so fewer words
+// per poll of a warp (8 rows x 3 neighbours) and one block product after the
+// other's on its own lane shorten it: 0.86 us a level on a 227k-cell RCM
+// box (181 levels), 1.5 with one row per lane.  A warp's rows go on together
+// (they are of one level, and none waits for another).
 template <typename TB, typename TV, bool FWD>
-__device__ __forceinline__ void sweep_row(const DevMesh& m, const TB* __restrict__ blk, const TB* __restrict__ rD,
-                                          const TV* in, TV* out, TV* r, int c, int* status, int spin_limit) {
-  const int s = c >> 5, lane = c & 31;
-  const int sb = m.slot_base[s];
-  const int nl = m.nlow[c], ns = m.nslot[c];
-  // the neighbours of this sweep: slots [0, nl) forward, [nl, ns) backward
-  const int nn = FWD ? nl : ns - nl;
-  auto slot = [&](int p) { return FWD ? p : ns - 1 - p; };
-  // everything that does not depend on the neighbours' results (columns,
-  // blocks, their rD) is loaded before the first poll
-  constexpr int PF = 3;
-  int colp[PF];
-  SlotBlock<TB> bp[PF];
-  TV rdp[PF];
+__device__ __forceinline__ void sweep_row4(const DevMesh& m, const TB* __restrict__ blk, const TB* __restrict__ rD,
+                                           const TV* in, TV* out, TV* r, int c, int* status,
+                                           int spin_limit) {
+  const int p = threadIdx.x & 3;  // lane 3: idle
+  const bool row = c >= 0;
+  int sb = 0, nl = 0, nn = 0, ns = 0, lane = 0;
+  TV acc[5] = {0, 0, 0, 0, 0}, rc = TV(0);
+  if (row) {
+    const int s = c >> 5;
+    lane = c & 31;
+    sb = m.slot_base[s];
+    nl = m.nlow[c];
+    ns = m.nslot[c];
+    nn = FWD ? nl : ns - nl;
+    if (p == 0) {
 #pragma unroll
-  for (int p = 0; p < PF; ++p) {
-    if (p < nn) {
-      const int t = slot(p);
-      colp[p] = m.scol[(sb + t) * 32 + lane];
-      bp[p].load(blk, sb + t, lane);
-      rdp[p] = FWD ? TV(rD[colp[p]]) : TV(1);
+      for (int k = 0; k < 5; ++k) acc[k] = FWD ? __ldcg(in + 5 * (size_t)c + k) : __ldcg(in + SWEEP_PAD * (size_t)c + k);
+      if (!FWD) rc = TV(rD[c]);
     }
   }
   const TV g = TV(m.gamma);
-  TV acc[5];
-#pragma unroll
-  for (int k = 0; k < 5; ++k) acc[k] = FWD ? __ldcg(in + 5 * c + k) : __ldcg(in + SWEEP_PAD * c + k);
-  TV* mine = out + (size_t)SWEEP_PAD * c;
-  // poll the prefetched neighbours together: (bounded; gives up on bit 8)
-  TV rv[PF][5];
-  unsigned pending = 0;
-#pragma unroll
-  for (int p = 0; p < PF; ++p)
-    if (p < nn) pending |= 1u << p;
-  {
+  for (int q0 = 0; __any_sync(0xffffffffu, q0 < nn); q0 += 3) {
+    const int q = q0 + p;
+    const bool on = p < 3 && q < nn;
+    SlotBlock<TB> B = {};
+    TV rj = TV(1), v[5] = {0, 0, 0, 0, 0}, y[5] = {0, 0, 0, 0, 0};
+    int col = 0, t = 0;
+    if (on) {
+      t = FWD ? q : ns - 1 - q;
+      col = m.scol[(sb + t) * 32 + lane];
+      B.load(blk, sb + t, lane);
+      if (FWD) rj = TV(rD[col]);
+    }
+    // the terms of the product that do not wait for the neighbour, made before
+    // the wait (the empty statement keeps them there)
+    typename SlotBlock<TB>::template Terms<TV> terms(g, B.w);
+    if constexpr (sizeof(TV) == 4) asm volatile("" : "+f"(terms.th), "+f"(terms.a1), "+f"(terms.pu));
+    bool ready = !on;
     int it = 0;
     while (true) {
-#pragma unroll
-      for (int p = 0; p < PF; ++p)
-        if (pending & (1u << p)) {
-          ld_relaxed5(out + (size_t)SWEEP_PAD * colp[p], rv[p]);
-          if (sweep_ready(rv[p])) pending &= ~(1u << p);
-        }
-      if (!pending) break;
+      if (!ready) {
+        ld_relaxed5(out + SWEEP_PAD * (size_t)col, v);
+        ready = sweep_ready(v);
+      }
+      if (__all_sync(0xffffffffu, ready)) break;
       ++it;
-      if (it > spin_limit || ((it & 63) == 0 && (ld_relaxed_int(status) & 8))) {
-        if (it > spin_limit) atomicOr(status, 8);
-        const TV z[5] = {TV(0), TV(0), TV(0), TV(0), TV(0)};
-        st_relaxed5(mine, z);
+      bool stop = it > spin_limit;
+      if (stop && threadIdx.x == 0) atomicOr(status, 8);
+      if ((it & 63) == 0) stop = stop || (ld_relaxed_int(status) & 8);
+      if (__any_sync(0xffffffffu, stop)) {
+        const TV z[5] = {0, 0, 0, 0, 0};
+        if (row && p == 0) st_relaxed5(out + SWEEP_PAD * (size_t)c, z);
         return;
       }
     }
-  }
+    if (on) {
+      TV d[5];
 #pragma unroll
-  for (int p = 0; p < PF; ++p) {
-    if (p < nn) {
-      TV dj[5], y[5];
+      for (int k = 0; k < 5; ++k) d[k] = FWD ? rj * v[k] : v[k];
+      terms.apply(g, d, y);
+      if (m.vjslot) vj_sub<TB>(m, sb + t, lane, col, d, y);
+    }
 #pragma unroll
-      for (int k = 0; k < 5; ++k) dj[k] = rdp[p] * rv[p][k];
-      bp[p].mv(g, dj, y);
-      if (m.vjslot) vj_sub<TB>(m, sb + slot(p), lane, colp[p], dj, y);
-#pragma unroll
-      for (int a = 0; a < 5; ++a) acc[a] -= y[a];
+    for (int k = 0; k < 5; ++k) {  // an idle lane's product is zero
+      const TV y1 = __shfl_down_sync(0xffffffffu, y[k], 1, 4), y2 = __shfl_down_sync(0xffffffffu, y[k], 2, 4);
+      acc[k] = ((acc[k] - y[k]) - y1) - y2;
     }
   }
-#pragma unroll 1
-  for (int p = PF; p < nn; ++p) {  // rows with more neighbours than prefetched
-    const int t = slot(p);
-    const int col = m.scol[(sb + t) * 32 + lane];
-    TV rj5[5];
-    int it = 0;
-    while (true) {
-      ld_relaxed5(out + (size_t)SWEEP_PAD * col, rj5);
-      if (sweep_ready(rj5)) break;
-      ++it;
-      if (it > spin_limit || ((it & 63) == 0 && (ld_relaxed_int(status) & 8))) {
-        if (it > spin_limit) atomicOr(status, 8);
-        const TV z[5] = {TV(0), TV(0), TV(0), TV(0), TV(0)};
-        st_relaxed5(mine, z);
-        return;
-      }
+  if (row && p == 0) {
+    TV z[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      if (!FWD) acc[k] = rc * acc[k];
+      z[k] = sweep_word(acc[k]);
     }
-    const TV rj = FWD ? TV(rD[col]) : TV(1);
-    TV dj[5], y[5];
+    st_relaxed5(out + SWEEP_PAD * (size_t)c, z);
+    if (!FWD)
 #pragma unroll
-    for (int k = 0; k < 5; ++k) dj[k] = rj * rj5[k];
-    SlotBlock<TB> Bk;
-    Bk.load(blk, sb + t, lane);
-    Bk.mv(g, dj, y);
-    if (m.vjslot) vj_sub<TB>(m, sb + t, lane, col, dj, y);
-#pragma unroll
-    for (int a = 0; a < 5; ++a) acc[a] -= y[a];
+      for (int k = 0; k < 5; ++k) r[5 * (size_t)c + k] = acc[k];
   }
-  if (!FWD) {
-    const TV rc = TV(rD[c]);
-#pragma unroll
-    for (int k = 0; k < 5; ++k) acc[k] = rc * acc[k];
-#pragma unroll
-    for (int k = 0; k < 5; ++k) r[5 * c + k] = acc[k];
-  }
-#pragma unroll
-  for (int k = 0; k < 5; ++k) acc[k] = sweep_word(acc[k]);
-  st_relaxed5(mine, acc);
 }
 
 template <typename TB, typename TV, bool FWD>
@@ -717,13 +703,11 @@ __global__ void __launch_bounds__(SWEEP_THREADS) k_lusgs_sweep(DevMesh m, const 
     if (threadIdx.x == 0) t = (int)atomicAdd(ticket, 1u);
     t = __shfl_sync(0xffffffffu, t, 0);
     if (t >= total) return;
-    if constexpr (ROWS == 2) {
-      const int c = order[t * 2 + (threadIdx.x >> 4)];
+    const int c = order[t * ROWS + threadIdx.x / (32 / ROWS)];
+    if constexpr (ROWS == 2)
       sweep_row16<TB, FWD>(m, blk, rD, in, out, r, c, status, spin_limit);
-    } else {
-      const int c = order[t * SWEEP_TICKET + threadIdx.x];
-      if (c >= 0) sweep_row<TB, TV, FWD>(m, blk, rD, in, out, r, c, status, spin_limit);
-    }
+    else
+      sweep_row4<TB, TV, FWD>(m, blk, rD, in, out, r, c, status, spin_limit);
     __syncwarp();
   }
 }
@@ -917,14 +901,16 @@ static void rev_level(Handle& h, const TB* blk, const TB* rD, TV* r, const int* 
                                        h.m, blk, rD, r, cells, start, cnt));
 }
 
-// Resident warps of a sync-free sweep: about four levels' worth, so that the
-// loads of the next levels' rows are in flight while a level is polled, and no
-// more pollers than that.  Measured on a 227k-cell RCM box (181 levels, ROWS
-// per warp 2 in FP64, 32 in FP32): one / two / four / eight levels 537 / 340 /
-// 276 / 278 us per FP64 sweep; FP32 268 us whatever the grid.
+// Resident warps of a sync-free sweep: a few levels' worth, so that the loads
+// of the next levels' rows are in flight while a level is polled, and no more
+// pollers than that.  Measured on a 227k-cell RCM box (181 levels): two rows
+// per warp (FP64 blocks), one / two / four / eight levels 537 / 340 / 276 /
+// 278 us per sweep; eight rows per warp, two / three / four / six / eight
+// levels 235 / 186 / 165 / 157 / 157 us (1M cells in the natural order 531 /
+// 450 / 443 / 427 / 438).
 static int sweep_grid(const DevMesh& m, int tickets, int rows) {
   const long warps = (long)tickets * (SWEEP_TICKET / rows);
-  const long g = std::min(std::max(4 * warps / m.nfl, 152L), 152L * 32);
+  const long g = std::min(std::max((rows == 2 ? 4 : 6) * warps / m.nfl, 152L), 152L * 32);
   return (int)std::min(g, warps);
 }
 
