@@ -429,6 +429,104 @@ __global__ void __launch_bounds__(128) k_lusgs_level(DevMesh m, const TB* __rest
     lusgs_fwd_row<TB, TV, true>(m, blk, rD, r, c);
 }
 
+// ------------------------------------------------- FP64 rows on five lanes
+// The FP64 products of few rows.  A warp's FP64 instruction holds its scheduler
+// for 64 cycles, so a row per thread costs a warp 175 x 64 cycles for a product
+// with six neighbours however few warps there are, while most of the 608
+// schedulers idle.  Here five lanes share a row, one component each, six rows
+// to a warp: 35 instructions per warp, in the same order per component.
+// A row costs 7% more of the pipe in all, so the row-per-thread kernels stay for
+// many rows.  By events around a launch (5 us of them), a row per thread against
+// five lanes, product / second level / reverse: 5k rows 12.7 : 9.8 / 15.3 : 10.5
+// / 14.8 : 10.3 us, 23.5k 18.3 : 13.7 / 20.6 : 15.8 / 18.5 : 13.8, 32k 18.9 :
+// 17.1 / 22.2 : 20.2 / 20.3 : 16.7; from 39k rows (two full warps per scheduler)
+// on neither way is ahead at every size, within 5% on average.
+// ROWS_PRODUCT: w = A x (k_spmv, k_op_level0); ROWS_LEVEL1: k_op_level1;
+// ROWS_REVERSE: the reverse sweep of a level, w in place (k_lusgs_level MODE 1).
+enum { ROWS_PRODUCT, ROWS_LEVEL1, ROWS_REVERSE };
+constexpr int ROWS5_WARP = 6;
+constexpr int ROWS5_THREADS = 64;
+constexpr int ROWS5_LIMIT = 36000;
+
+template <int MODE>
+__global__ void __launch_bounds__(ROWS5_THREADS) k_rows5(DevMesh m, const double* __restrict__ blk,
+                                                         const double* __restrict__ dg,
+                                                         const double* __restrict__ rD, const double* x, double* w,
+                                                         const int* __restrict__ cells, int start, int count) {
+  const int l = threadIdx.x & 31, r = l / 5, i = l - 5 * r;  // lanes 30, 31: idle
+  const int row = (int)((blockIdx.x * ROWS5_THREADS + threadIdx.x) >> 5) * ROWS5_WARP + r;
+  const bool on = r < ROWS5_WARP && row < count;
+  const int c = on ? (cells ? cells[start + row] : start + row) : 0;
+  const int lane = c & 31, base = m.slot_base[c >> 5];
+  const int first = MODE == ROWS_REVERSE && on ? m.nlow[c] : 0, ns = on ? m.nslot[c] : 0;
+  double acc = 0.0;
+  if (MODE == ROWS_REVERSE) {
+    if (on) acc = w[5 * (size_t)c + i];
+  } else if (on) {
+    const double* D = dg + ((size_t)(c >> 5) * 25 + 5 * i) * 32 + lane;
+#pragma unroll
+    for (int j = 0; j < 5; ++j) acc += D[j * 32] * x[5 * (size_t)c + j];
+  }
+  const int trips = __reduce_max_sync(0xffffffffu, ns - first);
+#pragma unroll 2
+  for (int q = 0; q < trips; ++q) {
+    const bool in = q < ns - first;
+    const int t = MODE == ROWS_REVERSE ? ns - 1 - q : q;
+    double B[5], xj[5], d = 0.0;
+    int col = 0;
+    if (in) {
+      col = m.scol[(base + t) * 32 + lane];
+      const double* bp = blk + ((size_t)(base + t) * 25 + 5 * i) * 32 + lane;
+#pragma unroll
+      for (int j = 0; j < 5; ++j) B[j] = bp[j * 32];
+      if (MODE == ROWS_LEVEL1) {  // the product's x_j and the sweep's rD w_j meet the same block
+        d = x[5 * (size_t)col + i] - rD[col] * w[5 * (size_t)col + i];
+      } else {
+        const double* from = MODE == ROWS_REVERSE ? w : x;
+#pragma unroll
+        for (int j = 0; j < 5; ++j) xj[j] = from[5 * (size_t)col + j];
+      }
+    }
+    if (MODE == ROWS_LEVEL1)
+#pragma unroll
+      for (int j = 0; j < 5; ++j) xj[j] = __shfl_sync(0xffffffffu, d, min(5 * r, 25) + j);
+    if (in) {
+#pragma unroll
+      for (int j = 0; j < 5; ++j) {
+        if (MODE == ROWS_REVERSE) xj[j] = -xj[j];
+        acc += B[j] * xj[j];
+      }
+      if (m.vjslot) {
+        double y[5] = {0, 0, 0, 0, 0};
+        vj_sub<double>(m, base + t, lane, col, xj, y);
+#pragma unroll
+        for (int j = 0; j < 5; ++j)
+          if (j == i) acc += y[j];
+      }
+    }
+  }
+  if (!on) return;
+  if (MODE != ROWS_REVERSE && m.nInst > 1 && hb_in_zone(m, c)) {
+    const int J = c / m.Nc, cl = c - J * m.Nc;
+    const double Vc = m.V[c];
+    for (int K = 0; K < m.nInst; ++K) {
+      if (K == J) continue;
+      acc += Vc * m.Dhb[J * m.nInst + K] * x[5 * ((size_t)K * m.Nc + cl) + i];
+    }
+  }
+  w[5 * (size_t)c + i] = MODE == ROWS_PRODUCT ? acc : rD[c] * acc;
+}
+
+template <int MODE>
+static bool rows5(Handle& h, int kind, const double* blk, const double* dg, const double* rD, const double* x, double* w,
+                  const int* cells, int start, int count) {
+  if (count > ROWS5_LIMIT) return false;
+  const int perBlock = ROWS5_WARP * ROWS5_THREADS / 32;
+  ICS_LAUNCH(h, kind, k_rows5<MODE><<<grid_for(count, perBlock), ROWS5_THREADS, 0, h.stream>>>(h.m, blk, dg, rD, x, w, cells,
+                                                                                              start, count));
+  return true;
+}
+
 // ----------------------------------------------- sync-free LU-SGS sweeps
 // One launch per sweep for schedules with many levels (RCM / natural
 // numbering).  A resident set of warps draws consecutive tickets; ticket t
@@ -884,7 +982,11 @@ __global__ void __launch_bounds__(RB) k_sumsq(int N, const double* __restrict__ 
 // -------------------------------------------------------------- dispatch
 template <typename TB, typename TV>
 static void spmv_t(Handle& h, const TV* x, TV* y) {
-  ICS_LAUNCH(h, ICS_K_SPMV, k_spmv<TB, TV><<<grid_for(h.m.N, 128), 128, 0, h.stream>>>(h.m, (const TB*)h.blk, (const TB*)h.dg, x, y));
+  bool split = false;
+  if constexpr (sizeof(TB) == 8)
+    split = rows5<ROWS_PRODUCT>(h, ICS_K_SPMV, (const double*)h.blk, (const double*)h.dg, nullptr, x, y, nullptr, 0, h.m.N);
+  if (!split)
+    ICS_LAUNCH(h, ICS_K_SPMV, k_spmv<TB, TV><<<grid_for(h.m.N, 128), 128, 0, h.stream>>>(h.m, (const TB*)h.blk, (const TB*)h.dg, x, y));
   if (h.m.ncrow > 0)
     ICS_LAUNCH(h, ICS_K_SPMV, k_cyc_mv<TB, TV><<<grid_for(h.m.ncrow, 128), 128, 0, h.stream>>>(h.m, (const TB*)h.cblk, x, y));
 }
@@ -893,6 +995,8 @@ static void spmv_t(Handle& h, const TV* x, TV* y) {
 // one reverse level: one row per thread, or two (Handle::tuneRevRows)
 template <typename TB, typename TV>
 static void rev_level(Handle& h, const TB* blk, const TB* rD, TV* r, const int* cells, int start, int cnt) {
+  if constexpr (sizeof(TB) == 8)
+    if (rows5<ROWS_REVERSE>(h, ICS_K_LUSGS_REV, blk, nullptr, rD, nullptr, r, cells, start, cnt)) return;
   if (h.tuneRevRows == 2)
     ICS_LAUNCH(h, ICS_K_LUSGS_REV, k_lusgs_rev2<TB, TV><<<grid_for((cnt + 1) / 2, 128), 128, 0, h.stream>>>(
                                        h.m, blk, rD, r, cells, start, cnt));
@@ -1001,10 +1105,15 @@ static bool fused_op_t(Handle& h, const TV* x, TV* w) {
   // in flight or the compiler's register choice (72-80), and 10 or 12 blocks
   // (51 / 40 registers, the latter spilling) were not faster; FP64 would spill
   constexpr int OPB = sizeof(TB) == 4 ? 8 : 1;
-  if (n0)
+  bool split0 = false, split1 = false;
+  if constexpr (sizeof(TB) == 8) {
+    split0 = n0 && rows5<ROWS_PRODUCT>(h, ICS_K_OP0, blk, dg, nullptr, x, w, c0, s0, n0);
+    split1 = n1 && rows5<ROWS_LEVEL1>(h, ICS_K_OP1, blk, dg, rD, x, w, c1, s1, n1);
+  }
+  if (n0 && !split0)
     ICS_LAUNCH(h, ICS_K_OP0, k_op_level0<TB, TV, OPB, 1><<<grid_for(n0, 128), 128, 0, h.stream>>>(m, blk, dg, x, w, c0,
                                                                                                  s0, n0));
-  if (n1)
+  if (n1 && !split1)
     ICS_LAUNCH(h, ICS_K_OP1, k_op_level1<TB, TV, OPB, 1><<<grid_for(n1, 128), 128, 0, h.stream>>>(m, blk, dg, rD, x, w,
                                                                                                  c1, s1, n1));
   // reverse level 1 = forward level 0 rows
