@@ -96,7 +96,7 @@ void dfree(void* p) {
 
 void free_all(Handle& h) {
   DevMesh& m = h.m;
-  void* ptrs[] = {m.own, m.nei, m.Sf, m.magSf, m.w, m.nodc, m.dOwn, m.dNei, m.dCC, m.nf, m.bnf, m.C, m.V,
+  void* ptrs[] = {m.own, m.nei, m.Sf, m.magSf, m.w, m.gO, m.gN, m.gC, m.gB, m.nodc, m.dOwn, m.dNei, m.dCC, m.nf, m.bnf, m.C, m.V,
                   m.bcell, m.bpatch, m.bSf, m.bmagSf, m.bdOwn, m.bdc, m.patches, m.cptr, m.cface, m.bptr,
                   m.bface, m.slot_base, m.scol, m.sface, m.nlow, m.nslot, m.fl_cells, m.rl_cells, m.fl_lptr,
                   m.rl_lptr, m.sweep_pad, m.sweep_ticket, m.sw_fwd, m.sw_rev, m.chain, h.W, h.W0, h.W00, h.Wprev, h.prim, h.pB, h.TB, h.UB, h.phiB, h.pseudoCo, h.rPDT,
@@ -281,6 +281,10 @@ void build_mesh(Handle& h, const ics_mesh_desc* d) {
   m.magSf = upload(magSf);
   m.nf = upload(nf);
   m.w = upload(std::vector<double>(d->weights, d->weights + F));
+  m.gO = dalloc<double>(3ull * F);
+  m.gN = dalloc<double>(3ull * F);
+  m.gC = dalloc<double>(3ull * N);
+  m.gB = dalloc<double>(3ull * B);
   m.nodc = upload(std::vector<double>(d->nonorth_delta_coeffs, d->nonorth_delta_coeffs + F));
   m.dc = upload(std::vector<double>(d->delta_coeffs, d->delta_coeffs + F));
   m.dOwn = upload(dOwn);
@@ -385,6 +389,7 @@ void build_mesh(Handle& h, const ics_mesh_desc* d) {
   }
   m.bptr = upload(bcnt);
   m.bface = upload(bface);
+  launch_gauss_coefficients(h);
   // sliced-ELL: row c slots = its faces in face order (lower part first)
   const int ns = (N + SLICE - 1) / SLICE;
   m.nslices = ns;

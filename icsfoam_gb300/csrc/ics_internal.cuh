@@ -69,6 +69,14 @@ struct DevMesh {
   double* Sf = nullptr;      // [3][F] SoA
   double* magSf = nullptr;   // [F]
   double* w = nullptr;       // [F]
+  // Gauss gradient coefficients: of the neighbour's difference from the owner in
+  // the owner's gradient S (1 - w) / V_own, of the opposite one in the
+  // neighbour's -S w / V_nei, of a boundary value's S / V, and of the cell's own
+  // value: its outward areas' sum over V (rounding, where the faces close the cell)
+  double* gO = nullptr;      // [3][F]
+  double* gN = nullptr;      // [3][F]
+  double* gC = nullptr;      // [3][N]
+  double* gB = nullptr;      // [3][B]
   double* nodc = nullptr;    // [F]
   double* dc = nullptr;      // [F] deltaCoeffs 1/|C_nei - C_own|
   double* dOwn = nullptr;    // [3][F] Cf - C[own]
@@ -412,6 +420,7 @@ struct Launch {
 // ------------------------------------------------------------------ kernels
 void launch_fields(Handle& h);
 void launch_grad(Handle& h);
+void launch_gauss_coefficients(Handle& h);
 void launch_face_flux(Handle& h);
 void launch_residual(Handle& h, double serRatio, bool applySer);
 void launch_jacobian(Handle& h);

@@ -243,50 +243,43 @@ __global__ void __launch_bounds__(128) k_adj_lim(DevMesh m, unsigned mask, unsig
     if (hasGrad && LIMITED) {
       // recompute the Gauss gradient and the bounds exactly as k_grad does
       const double qc = q[k * N + c];
-      double G[3] = {0.0, 0.0, 0.0};
-      double qmax = qc, qmin = qc;
+      double G[3] = {m.gC[c] * qc, m.gC[N + c] * qc, m.gC[2 * N + c] * qc};
+      double dmax = 0.0, dmin = 0.0;
       int srcMax = c, srcMin = c;  // -1: a boundary value
       for (int e = e0; e < e1; ++e) {
         const int code = m.cface[e];
         const bool isOwn = code >= 0;
         const int f = isOwn ? code : ~code;
         const int other = isOwn ? m.nei[f] : m.own[f];
-        const double wf = m.w[f];
-        const double S0 = flip(m.Sf[f], !isOwn), S1 = flip(m.Sf[F + f], !isOwn), S2 = flip(m.Sf[2 * F + f], !isOwn);
-        const double qo = q[k * N + other];
-        const double qown = isOwn ? qc : qo, qnei = isOwn ? qo : qc;
-        const double sf = wf * (qown - qnei) + qnei;
-        G[0] = G[0] + S0 * sf;
-        G[1] = G[1] + S1 * sf;
-        G[2] = G[2] + S2 * sf;
-        if (okey(qo) > okey(qmax)) {
-          qmax = qo;
+        const double* g = isOwn ? m.gO : m.gN;
+        const double dq = q[k * N + other] - qc;
+        G[0] = G[0] + g[f] * dq;
+        G[1] = G[1] + g[F + f] * dq;
+        G[2] = G[2] + g[2 * F + f] * dq;
+        if (okey(dq) > okey(dmax)) {
+          dmax = dq;
           srcMax = other;
         }
-        if (okey(qo) < okey(qmin)) {
-          qmin = qo;
+        if (okey(dq) < okey(dmin)) {
+          dmin = dq;
           srcMin = other;
         }
       }
       for (int e = b0; e < b1; ++e) {
         const int b = m.bface[e];
-        const double v = bq[k * B + b];
-        G[0] = G[0] + m.bSf[b] * v;
-        G[1] = G[1] + m.bSf[B + b] * v;
-        G[2] = G[2] + m.bSf[2 * B + b] * v;
-        if (okey(v) > okey(qmax)) {
-          qmax = v;
+        const double v = bq[k * B + b] - qc;
+        G[0] = G[0] + m.gB[b] * v;
+        G[1] = G[1] + m.gB[B + b] * v;
+        G[2] = G[2] + m.gB[2 * B + b] * v;
+        if (okey(v) > okey(dmax)) {
+          dmax = v;
           srcMax = -1;
         }
-        if (okey(v) < okey(qmin)) {
-          qmin = v;
+        if (okey(v) < okey(dmin)) {
+          dmin = v;
           srcMin = -1;
         }
       }
-      G[0] = G[0] * rV;
-      G[1] = G[1] * rV;
-      G[2] = G[2] * rV;
-      double dmax = qmax - qc, dmin = qmin - qc;
       if (m.limWiden > 0.0) {
         const double wd = m.limWiden * (dmax - dmin);
         dmax = dmax + wd;

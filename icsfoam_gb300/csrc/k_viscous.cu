@@ -45,36 +45,36 @@ __global__ void __launch_bounds__(128) k_visc_cell(DevMesh m, ViscParams P, cons
   const int N = m.N, F = m.F, B = m.B;
   Real Uc[3] = {prim[2 * N + c], prim[3 * N + c], prim[4 * N + c]};
   const Real ec = P.Cv * prim[N + c];  // e = Cv T
-  Real g[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, ge[3] = {0, 0, 0};
+  // the Gauss gradients, with the products of area, weight and 1 / V of k_grad
+  Real g[9], ge[3];
+  for (int i = 0; i < 3; ++i) {
+    const double C = m.gC[i * N + c];
+    for (int j = 0; j < 3; ++j) g[3 * i + j] = C * Uc[j];
+    ge[i] = C * ec;
+  }
   for (int e = m.cptr[c]; e < m.cptr[c + 1]; ++e) {
     const int code = m.cface[e];
     const bool isOwn = code >= 0;
     const int f = isOwn ? code : ~code;
     const int other = isOwn ? m.nei[f] : m.own[f];
-    const double wf = m.w[f];
-    // outward area vector
-    const double S[3] = {flip(m.Sf[f], !isOwn), flip(m.Sf[F + f], !isOwn), flip(m.Sf[2 * F + f], !isOwn)};
-    const Real Uo[3] = {prim[2 * N + other], prim[3 * N + other], prim[4 * N + other]};
-    const Real eo = P.Cv * prim[N + other];
-    for (int j = 0; j < 3; ++j) {
-      const Real a = isOwn ? Uc[j] : Uo[j], b = isOwn ? Uo[j] : Uc[j];
-      const Real sf = wf * (a - b) + b;
-      for (int i = 0; i < 3; ++i) g[3 * i + j] = g[3 * i + j] + S[i] * sf;
+    const double* Gf = isOwn ? m.gO : m.gN;
+    const double G[3] = {Gf[f], Gf[F + f], Gf[2 * F + f]};
+    const Real dU[3] = {prim[2 * N + other] - Uc[0], prim[3 * N + other] - Uc[1], prim[4 * N + other] - Uc[2]};
+    const Real de = P.Cv * (prim[N + other] - prim[N + c]);
+    for (int i = 0; i < 3; ++i) {
+      for (int j = 0; j < 3; ++j) g[3 * i + j] = g[3 * i + j] + G[i] * dU[j];
+      ge[i] = ge[i] + G[i] * de;
     }
-    const Real a = isOwn ? ec : eo, b = isOwn ? eo : ec;
-    const Real sf = wf * (a - b) + b;
-    for (int i = 0; i < 3; ++i) ge[i] = ge[i] + S[i] * sf;
   }
   for (int e = m.bptr[c]; e < m.bptr[c + 1]; ++e) {
     const int b = m.bface[e];
-    const double S[3] = {m.bSf[b], m.bSf[B + b], m.bSf[2 * B + b]};
+    const double S[3] = {m.gB[b], m.gB[B + b], m.gB[2 * B + b]};  // over V
     const int pc = m.bpartner ? m.bpartner[b] : -1;
     if (pc >= 0) {
       // coupled face: interpolate with the partner, its velocity rotated
       const double* Rm = m.patches[m.bpatch[b]].R;
       const double wb = m.bw[b];
       const Real Un[3] = {prim[2 * N + pc], prim[3 * N + pc], prim[4 * N + pc]};
-      const Real en = P.Cv * prim[N + pc];
       Real upv[3];
       if (plag_mode(m, b))  // U phase-lagged across an HB phase-lag patch
         plag_vec(m, b, pc, prim + 2 * N, prim + 3 * N, prim + 4 * N, upv);
@@ -82,22 +82,19 @@ __global__ void __launch_bounds__(128) k_visc_cell(DevMesh m, ViscParams P, cons
         for (int j = 0; j < 3; ++j) upv[j] = Rm[3 * j] * Un[0] + Rm[3 * j + 1] * Un[1] + Rm[3 * j + 2] * Un[2];
       for (int j = 0; j < 3; ++j) {
         const Real up = upv[j];
-        const Real sf = wb * (Uc[j] - up) + up;
+        const Real sf = (1.0 - wb) * (up - Uc[j]);
         for (int i = 0; i < 3; ++i) g[3 * i + j] += S[i] * sf;
       }
-      const Real sf = wb * (ec - en) + en;
+      const Real sf = (1.0 - wb) * (P.Cv * (prim[N + pc] - prim[N + c]));
       for (int i = 0; i < 3; ++i) ge[i] += S[i] * sf;
       continue;
     }
-    const double Ub[3] = {UB[b], UB[B + b], UB[2 * B + b]};
-    const double eb = P.Cv * TB[b];
+    const Real Ub[3] = {UB[b] - Uc[0], UB[B + b] - Uc[1], UB[2 * B + b] - Uc[2]};
+    const Real eb = P.Cv * (TB[b] - prim[N + c]);
     for (int j = 0; j < 3; ++j)
       for (int i = 0; i < 3; ++i) g[3 * i + j] += S[i] * Ub[j];
     for (int i = 0; i < 3; ++i) ge[i] += S[i] * eb;
   }
-  const double rV = 1.0 / m.V[c];  // one division for the twelve components
-  for (int q = 0; q < 9; ++q) g[q] = g[q] * rV;
-  for (int q = 0; q < 3; ++q) ge[q] = ge[q] * rV;
   const Real mu = mu_of(P, prim[N + c]);
   const Real tr = g[0] + g[4] + g[8];
   for (int q = 0; q < 9; ++q) vc[q * N + c] = g[q];
