@@ -176,7 +176,7 @@ def kernel_bytes(kind, N, F, B, nslots, mixed, nlev):
     if kind == "face":       # MUSCL face flux: gathered cell fields + face geometry + outputs
         return 264 * N + 232 * F
     if kind == "grad":
-        return 268 * N + 96 * F
+        return 284 * N + 112 * F
     if kind == "cellres":
         return 136 * N + 64 * F
     if kind == "jac_rows":
@@ -193,7 +193,9 @@ def kernel_bytes(kind, N, F, B, nslots, mixed, nlev):
     if kind == "op1":   # pass 2: (A x) + forward sweep + first reverse on the other half
         return 25 * pb * N / 2 + ow * pb * F + 10 * pv * N + pb * N + 4 * F
     if kind == "mgs":
-        return 20 * pv * N
+        # a column of GMRES(8), mean over a cycle's nine launches: w once in each, 36 basis vectors,
+        # eight written
+        return 5 * pv * N * 53 / 9
     return None
 
 
@@ -214,8 +216,8 @@ def kernel_bound(kind, mixed):
 # FP64 flops of one unit of work (a face for "face", a cell for "grad"),
 # HLLC + MUSCL / cellLimited<Venkatakrishnan>: counted by ncu from the
 # executed DFMA (2 flops), DADD and DMUL instructions of one launch
-# (profiles/fp64_face_grad_bump_128x64x64.md), divided by the faces / cells
-FP64_FLOPS_PER_UNIT = {"face": 319.8, "grad": 1013.2}
+# (profiles/fp64_residual_bump_125x63x61.md), divided by the faces / cells
+FP64_FLOPS_PER_UNIT = {"face": 297.0, "grad": 876.1}
 
 
 def load_peaks():

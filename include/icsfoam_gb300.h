@@ -488,12 +488,14 @@ int ics_timer_stop(ics_handle h, double* ms);
 typedef struct {
   int32_t face_block;      /* threads per block of the face-flux kernel (64 / 128)       */
   int32_t grad_block;      /* threads per block of the gradient kernel (64 / 128)        */
-  int32_t mgs_blocks;      /* grid of the Gram-Schmidt steps (152 / 304 / 456 / 608)      */
+  int32_t mgs_blocks;      /* 152 / 304 / 456 / 608, kept in saved tunings: no effect (a
+                              Gram-Schmidt column sizes its own grid)                    */
   int32_t fused_operator;  /* 1: fused M^-1 A passes on two-level schedules, 0: SpMV then
                               LU-SGS sweeps                                              */
   int32_t from_cache;      /* 1: taken from an earlier tuning of a case of the same shape */
   int32_t reverse_rows;    /* rows per thread of the reverse LU-SGS level sweep (1 / 2:
-                              two rows' slot loads in flight together)                   */
+                              two rows' slot loads in flight together); no effect on an
+                              FP64 level of up to 36000 rows                             */
 } ics_tuning;
 /* Time each candidate launch choice on the handle's current state and
  * assembled Jacobian (CUDA events on its stream) and keep the fastest, for
