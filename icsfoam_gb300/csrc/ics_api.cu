@@ -73,20 +73,28 @@ Launch::~Launch() {
 
 namespace {
 
+// A handle's memory is filled on the handle's own stream, where its kernels
+// run: a copy or fill on the default stream is not ordered before them (the
+// stream is a non-blocking one), and a copy from pageable memory may return
+// while it is still under way.
 template <typename T>
-T* dalloc(size_t n) {
+T* dalloc(Handle& h, size_t n) {
   T* p = nullptr;
   if (n == 0) n = 1;
   cudaError_t e = cudaMalloc(&p, n * sizeof(T));
   if (e != cudaSuccess) throw CudaError(e, "cudaMalloc", __FILE__, __LINE__);
-  ICS_CUDA(cudaMemset(p, 0, n * sizeof(T)));
+  ICS_CUDA(cudaMemsetAsync(p, 0, n * sizeof(T), h.stream));
   return p;
 }
 
+// waits: the source may be a temporary
 template <typename T>
-T* upload(const std::vector<T>& v) {
-  T* p = dalloc<T>(v.size());
-  if (!v.empty()) ICS_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+T* upload(Handle& h, const std::vector<T>& v) {
+  T* p = dalloc<T>(h, v.size());
+  if (!v.empty()) {
+    ICS_CUDA(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, h.stream));
+    ICS_CUDA(cudaStreamSynchronize(h.stream));
+  }
   return p;
 }
 
@@ -199,21 +207,21 @@ void ensure_workspace(Handle& h) {
     void* ptrs[] = {h.blk, h.dg, h.dginv, h.rD, h.kw, h.kx, h.kb, h.kt, h.kv};
     for (void* q : ptrs) dfree(q);
     // off-diagonal slots: factored in FP32, full in FP64 (blocks.cuh)
-    h.blk = dalloc<char>((size_t)h.m.nslots * slot_words(p == ICS_PREC_MIXED) * 32 * eb);
-    h.dg = dalloc<char>((size_t)h.m.nslices * 25 * 32 * eb);
-    h.dginv = dalloc<char>((size_t)h.m.nslices * 25 * 32 * eb);
-    h.rD = dalloc<char>((size_t)h.m.N * eb);
-    h.kw = dalloc<char>(kstride(h) * eb);  // whole 16-byte chunks
-    h.kx = dalloc<char>(n5 * eb);
-    h.kb = dalloc<char>(n5 * eb);
-    h.kt = dalloc<char>(n5 * eb);
-    h.kv = dalloc<char>(kstride(h) * eb * m);
+    h.blk = dalloc<char>(h, (size_t)h.m.nslots * slot_words(p == ICS_PREC_MIXED) * 32 * eb);
+    h.dg = dalloc<char>(h, (size_t)h.m.nslices * 25 * 32 * eb);
+    h.dginv = dalloc<char>(h, (size_t)h.m.nslices * 25 * 32 * eb);
+    h.rD = dalloc<char>(h, (size_t)h.m.N * eb);
+    h.kw = dalloc<char>(h, kstride(h) * eb);  // whole 16-byte chunks
+    h.kx = dalloc<char>(h, n5 * eb);
+    h.kb = dalloc<char>(h, n5 * eb);
+    h.kt = dalloc<char>(h, n5 * eb);
+    h.kv = dalloc<char>(h, kstride(h) * eb * m);
     h.kvDirs = m;
     h.kvPrec = p;
     h.haveMatrix = false;
   } else if (h.kvDirs < m) {
     dfree(h.kv);
-    h.kv = dalloc<char>(kstride(h) * eb * m);
+    h.kv = dalloc<char>(h, kstride(h) * eb * m);
     h.kvDirs = m;
   }
 }
@@ -275,30 +283,30 @@ void build_mesh(Handle& h, const ics_mesh_desc* d) {
   std::vector<double> C(3 * N);
   for (int i = 0; i < N; ++i)
     for (int k = 0; k < 3; ++k) C[k * N + i] = d->C[3 * i + k];
-  m.own = upload(std::vector<int>(d->owner, d->owner + F));
-  m.nei = upload(std::vector<int>(d->neighbour, d->neighbour + F));
-  m.Sf = upload(Sf);
-  m.magSf = upload(magSf);
-  m.nf = upload(nf);
-  m.w = upload(std::vector<double>(d->weights, d->weights + F));
-  m.gO = dalloc<double>(3ull * F);
-  m.gN = dalloc<double>(3ull * F);
-  m.gC = dalloc<double>(3ull * N);
-  m.gB = dalloc<double>(3ull * B);
-  m.nodc = upload(std::vector<double>(d->nonorth_delta_coeffs, d->nonorth_delta_coeffs + F));
-  m.dc = upload(std::vector<double>(d->delta_coeffs, d->delta_coeffs + F));
-  m.dOwn = upload(dOwn);
-  m.dNei = upload(dNei);
-  m.dCC = upload(dCC);
-  m.C = upload(C);
-  m.V = upload(std::vector<double>(d->V, d->V + N));
-  m.bcell = upload(std::vector<int>(d->b_cell, d->b_cell + B));
-  m.bpatch = upload(std::vector<int>(d->b_patch, d->b_patch + B));
-  m.bSf = upload(bSf);
-  m.bmagSf = upload(bmag);
-  m.bnf = upload(bnf);
-  m.bdOwn = upload(bdOwn);
-  m.bdc = upload(std::vector<double>(d->b_delta_coeffs, d->b_delta_coeffs + B));
+  m.own = upload(h, std::vector<int>(d->owner, d->owner + F));
+  m.nei = upload(h, std::vector<int>(d->neighbour, d->neighbour + F));
+  m.Sf = upload(h, Sf);
+  m.magSf = upload(h, magSf);
+  m.nf = upload(h, nf);
+  m.w = upload(h, std::vector<double>(d->weights, d->weights + F));
+  m.gO = dalloc<double>(h, 3ull * F);
+  m.gN = dalloc<double>(h, 3ull * F);
+  m.gC = dalloc<double>(h, 3ull * N);
+  m.gB = dalloc<double>(h, 3ull * B);
+  m.nodc = upload(h, std::vector<double>(d->nonorth_delta_coeffs, d->nonorth_delta_coeffs + F));
+  m.dc = upload(h, std::vector<double>(d->delta_coeffs, d->delta_coeffs + F));
+  m.dOwn = upload(h, dOwn);
+  m.dNei = upload(h, dNei);
+  m.dCC = upload(h, dCC);
+  m.C = upload(h, C);
+  m.V = upload(h, std::vector<double>(d->V, d->V + N));
+  m.bcell = upload(h, std::vector<int>(d->b_cell, d->b_cell + B));
+  m.bpatch = upload(h, std::vector<int>(d->b_patch, d->b_patch + B));
+  m.bSf = upload(h, bSf);
+  m.bmagSf = upload(h, bmag);
+  m.bnf = upload(h, bnf);
+  m.bdOwn = upload(h, bdOwn);
+  m.bdc = upload(h, std::vector<double>(d->b_delta_coeffs, d->b_delta_coeffs + B));
   std::vector<Patch> pts(std::max(1, d->n_patches));
   for (int p = 0; p < d->n_patches; ++p) {
     const ics_patch_desc& q = d->patches[p];
@@ -312,7 +320,7 @@ void build_mesh(Handle& h, const ics_mesh_desc* d) {
     for (int k = 0; k < 9; ++k) pts[p].R[k] = q.rotation[k];
     if (q.kind < 0 || q.kind > ICS_PATCH_CYCLIC) throw std::string("unknown patch kind");
   }
-  m.patches = upload(pts);
+  m.patches = upload(h, pts);
   m.npatches = d->n_patches;
   // coupled (cyclic) faces
   {
@@ -350,16 +358,16 @@ void build_mesh(Handle& h, const ics_mesh_desc* d) {
         }
       }
       ptr.push_back((int)cycFaces.size());
-      m.bpartner = upload(partner);
-      m.bw = upload(w);
-      m.bdelta = upload(delta);
-      m.bdNei = upload(nbrd);
-      m.bnodc = upload(nodc);
+      m.bpartner = upload(h, partner);
+      m.bw = upload(h, w);
+      m.bdelta = upload(h, delta);
+      m.bdNei = upload(h, nbrd);
+      m.bnodc = upload(h, nodc);
       m.ncyc = (int)cycFaces.size();
       m.ncrow = (int)rows.size();
-      m.cyc_face = upload(cycFaces);
-      m.cyc_row = upload(rows);
-      m.cyc_ptr = upload(ptr);
+      m.cyc_face = upload(h, cycFaces);
+      m.cyc_row = upload(h, rows);
+      m.cyc_ptr = upload(h, ptr);
     }
   }
   // cell -> faces CSR in face order
@@ -377,8 +385,8 @@ void build_mesh(Handle& h, const ics_mesh_desc* d) {
       cface[fill[d->neighbour[f]]++] = ~f;
     }
   }
-  m.cptr = upload(cnt);
-  m.cface = upload(cface);
+  m.cptr = upload(h, cnt);
+  m.cface = upload(h, cface);
   std::vector<int> bcnt(N + 1, 0);
   for (int b = 0; b < B; ++b) bcnt[d->b_cell[b] + 1]++;
   for (int i = 0; i < N; ++i) bcnt[i + 1] += bcnt[i];
@@ -387,8 +395,8 @@ void build_mesh(Handle& h, const ics_mesh_desc* d) {
     std::vector<int> fill(bcnt.begin(), bcnt.end() - 1);
     for (int b = 0; b < B; ++b) bface[fill[d->b_cell[b]]++] = b;
   }
-  m.bptr = upload(bcnt);
-  m.bface = upload(bface);
+  m.bptr = upload(h, bcnt);
+  m.bface = upload(h, bface);
   launch_gauss_coefficients(h);
   // sliced-ELL: row c slots = its faces in face order (lower part first)
   const int ns = (N + SLICE - 1) / SLICE;
@@ -432,11 +440,11 @@ void build_mesh(Handle& h, const ics_mesh_desc* d) {
       prev = col;
     }
   }
-  m.slot_base = upload(slot_base);
-  m.scol = upload(scol);
-  m.sface = upload(sface);
-  m.nslot = upload(nslot);
-  m.nlow = upload(nlow);
+  m.slot_base = upload(h, slot_base);
+  m.scol = upload(h, scol);
+  m.sface = upload(h, sface);
+  m.nslot = upload(h, nslot);
+  m.nlow = upload(h, nlow);
   // LU-SGS levels
   std::vector<int> lev(N, 0), rlev(N, 0);
   for (int c = 0; c < N; ++c)
@@ -471,66 +479,66 @@ void build_mesh(Handle& h, const ics_mesh_desc* d) {
     m.fuse_last = (b - a) == (m.rl_ptr[1] - m.rl_ptr[0]) &&
                   std::equal(fcells.begin() + a, fcells.begin() + b, rcells.begin() + m.rl_ptr[0]);
   }
-  m.fl_cells = upload(fcells);
-  m.rl_cells = upload(rcells);
-  m.fl_lptr = upload(m.fl_ptr);
+  m.fl_cells = upload(h, fcells);
+  m.rl_cells = upload(h, rcells);
+  m.fl_lptr = upload(h, m.fl_ptr);
   // the sync-free sweeps: every schedule of more than two levels.  Measured
   // against one CTA that walks the levels (us per forward sweep, FP64 / FP32):
   // 12^3 RCM box 48 / 47 against 176 / 58, 24^3 97 / 96 against 556 / 131,
   // 61^3 276 / 268 against 7069 / 1010.
   if (m.nfl > 2) {
-    m.sweep_pad = dalloc<double>(16ull * N);
+    m.sweep_pad = dalloc<double>(h, 16ull * N);
     const std::vector<int> sf = ticket_order(fcells, m.fl_ptr), sr = ticket_order(rcells, m.rl_ptr);
     m.nsw_fwd = (int)(sf.size() / SWEEP_TICKET);
     m.nsw_rev = (int)(sr.size() / SWEEP_TICKET);
-    m.sw_fwd = upload(sf);
-    m.sw_rev = upload(sr);
+    m.sw_fwd = upload(h, sf);
+    m.sw_rev = upload(h, sr);
     // one unbroken chain: every row couples to the one before and the one
     // after, and to no other (a break would let a non-finite value of one
     // part reach the next through the zero products across it)
     bool chain = F == N - 1;
     for (int f = 0; f < F && chain; ++f) chain = d->neighbour[f] == d->owner[f] + 1;
-    if (chain) m.chain = dalloc<double>(chain_table_words(N));
+    if (chain) m.chain = dalloc<double>(h, chain_table_words(N));
   }
-  m.sweep_ticket = dalloc<unsigned int>(2);
-  m.rl_lptr = upload(m.rl_ptr);
+  m.sweep_ticket = dalloc<unsigned int>(h, 2);
+  m.rl_lptr = upload(h, m.rl_ptr);
 }
 
 void alloc_state(Handle& h) {
   const int N = h.m.N, F = h.m.F, B = h.m.B;
-  h.W = dalloc<double>(5ull * N);
-  h.W0 = dalloc<double>(5ull * N);
-  h.W00 = dalloc<double>(5ull * N);
-  h.Wprev = dalloc<double>(5ull * N);
-  h.prim = dalloc<double>(5ull * N);
-  h.pB = dalloc<double>(B);
-  h.TB = dalloc<double>(B);
-  h.UB = dalloc<double>(3ull * B);
-  h.phiB = dalloc<double>(B);
-  h.pseudoCo = dalloc<double>(N);
-  h.rPDT = dalloc<double>(N);
-  h.ddtCoeff = dalloc<double>(N);
-  h.q = dalloc<double>((size_t)NQ * N);
-  h.bq = dalloc<double>((size_t)NQ * B);
-  h.clin = dalloc<double>((size_t)N + B);
-  h.grad = dalloc<double>((size_t)NQ * 3 * N);
-  h.fflux = dalloc<double>(5ull * (F + B));
-  h.frec = dalloc<double>(8ull * F);
-  h.flam = dalloc<double>((size_t)F + B);
+  h.W = dalloc<double>(h, 5ull * N);
+  h.W0 = dalloc<double>(h, 5ull * N);
+  h.W00 = dalloc<double>(h, 5ull * N);
+  h.Wprev = dalloc<double>(h, 5ull * N);
+  h.prim = dalloc<double>(h, 5ull * N);
+  h.pB = dalloc<double>(h, B);
+  h.TB = dalloc<double>(h, B);
+  h.UB = dalloc<double>(h, 3ull * B);
+  h.phiB = dalloc<double>(h, B);
+  h.pseudoCo = dalloc<double>(h, N);
+  h.rPDT = dalloc<double>(h, N);
+  h.ddtCoeff = dalloc<double>(h, N);
+  h.q = dalloc<double>(h, (size_t)NQ * N);
+  h.bq = dalloc<double>(h, (size_t)NQ * B);
+  h.clin = dalloc<double>(h, (size_t)N + B);
+  h.grad = dalloc<double>(h, (size_t)NQ * 3 * N);
+  h.fflux = dalloc<double>(h, 5ull * (F + B));
+  h.frec = dalloc<double>(h, 8ull * F);
+  h.flam = dalloc<double>(h, (size_t)F + B);
   if (h.m.ncyc) {
-    h.cfrec = dalloc<double>(8ull * h.m.ncyc);
-    h.cblk = dalloc<double>(25ull * h.m.ncyc);  // FP64 size; FP32 blocks use half
+    h.cfrec = dalloc<double>(h, 8ull * h.m.ncyc);
+    h.cblk = dalloc<double>(h, 25ull * h.m.ncyc);  // FP64 size; FP32 blocks use half
   }
-  h.bjac = dalloc<double>(25ull * B);
-  h.src = dalloc<double>(5ull * N);
-  h.dW = dalloc<double>(5ull * N);
-  h.partials = dalloc<double>((size_t)REDUCE_BLOCKS * 16);
-  h.counter = dalloc<unsigned int>(MAX_INST + 4);
-  h.ks = dalloc<KrylovScalars>(1);
-  h.colSlots = dalloc<double>(column_slot_words());
+  h.bjac = dalloc<double>(h, 25ull * B);
+  h.src = dalloc<double>(h, 5ull * N);
+  h.dW = dalloc<double>(h, 5ull * N);
+  h.partials = dalloc<double>(h, (size_t)REDUCE_BLOCKS * 16);
+  h.counter = dalloc<unsigned int>(h, MAX_INST + 4);
+  h.ks = dalloc<KrylovScalars>(h, 1);
+  h.colSlots = dalloc<double>(h, column_slot_words());
   ICS_CUDA(cudaMallocHost(&h.ksHost, sizeof(KrylovScalars)));
-  h.scratch = dalloc<double>(5ull * N + 8);
-  h.ibuf = dalloc<int>((size_t)N + 8);
+  h.scratch = dalloc<double>(h, 5ull * N + 8);
+  h.ibuf = dalloc<int>(h, (size_t)N + 8);
 }
 
 // sqrt(sum over instances of |s0|^2 + |s1|^2 + |v0|^2), scalars rho, rhoE and
@@ -587,10 +595,10 @@ int do_residual(Handle& h, double* host_src) {
   launch_face_flux(h);
   if (h.cfg.c.viscous) {
     if (!h.vcell) {
-      h.vcell = dalloc<double>(24ull * h.m.N);
-      h.fvisc = dalloc<double>(4ull * (h.m.F + h.m.B));
-      h.vsf2 = dalloc<double>((size_t)h.m.F + h.m.B);
-      h.vjac = dalloc<double>(2ull * (h.m.F + h.m.B));
+      h.vcell = dalloc<double>(h, 24ull * h.m.N);
+      h.fvisc = dalloc<double>(h, 4ull * (h.m.F + h.m.B));
+      h.vsf2 = dalloc<double>(h, (size_t)h.m.F + h.m.B);
+      h.vjac = dalloc<double>(h, 2ull * (h.m.F + h.m.B));
     }
     launch_viscous(h);
   }
@@ -811,7 +819,8 @@ int ics_create(const ics_mesh_desc* mesh, const ics_config* cfg, ics_handle* out
     alloc_state(hd);
     ensure_workspace(hd);
     std::vector<double> co(hd.m.N, cfg->pseudo_co_num);
-    ICS_CUDA(cudaMemcpy(hd.pseudoCo, co.data(), co.size() * sizeof(double), cudaMemcpyHostToDevice));
+    ICS_CUDA(cudaMemcpyAsync(hd.pseudoCo, co.data(), co.size() * sizeof(double), cudaMemcpyHostToDevice, hd.stream));
+    ICS_CUDA(cudaStreamSynchronize(hd.stream));
     return ICS_OK;
   });
   if (st) {
@@ -894,15 +903,16 @@ int ics_set_boundary_state(ics_handle hh, const double* pb, const double* Ub, co
   return guard(hh, [&](Handle& h) {
     const size_t B = h.m.B;
     h.haveExact = false;
-    if (pb) ICS_CUDA(cudaMemcpy(h.pB, pb, B * sizeof(double), cudaMemcpyHostToDevice));
-    if (Tb) ICS_CUDA(cudaMemcpy(h.TB, Tb, B * sizeof(double), cudaMemcpyHostToDevice));
-    if (phib) ICS_CUDA(cudaMemcpy(h.phiB, phib, B * sizeof(double), cudaMemcpyHostToDevice));
+    if (pb) ICS_CUDA(cudaMemcpyAsync(h.pB, pb, B * sizeof(double), cudaMemcpyHostToDevice, h.stream));
+    if (Tb) ICS_CUDA(cudaMemcpyAsync(h.TB, Tb, B * sizeof(double), cudaMemcpyHostToDevice, h.stream));
+    if (phib) ICS_CUDA(cudaMemcpyAsync(h.phiB, phib, B * sizeof(double), cudaMemcpyHostToDevice, h.stream));
+    std::vector<double> t(Ub ? 3 * B : 0);
     if (Ub) {
-      std::vector<double> t(3 * B);
       for (size_t b = 0; b < B; ++b)
         for (int k = 0; k < 3; ++k) t[k * B + b] = Ub[3 * b + k];
-      ICS_CUDA(cudaMemcpy(h.UB, t.data(), 3 * B * sizeof(double), cudaMemcpyHostToDevice));
+      ICS_CUDA(cudaMemcpyAsync(h.UB, t.data(), 3 * B * sizeof(double), cudaMemcpyHostToDevice, h.stream));
     }
+    ICS_CUDA(cudaStreamSynchronize(h.stream));
     return ICS_OK;
   });
 }
@@ -962,7 +972,8 @@ int ics_set_conservative(ics_handle hh, const double* W, int32_t set_old) {
 int ics_set_pseudo_co(ics_handle hh, const double* co) {
   if (!co) return ICS_ERR_ARG;
   return guard(hh, [&](Handle& h) {
-    ICS_CUDA(cudaMemcpy(h.pseudoCo, co, h.m.N * sizeof(double), cudaMemcpyHostToDevice));
+    ICS_CUDA(cudaMemcpyAsync(h.pseudoCo, co, h.m.N * sizeof(double), cudaMemcpyHostToDevice, h.stream));
+    ICS_CUDA(cudaStreamSynchronize(h.stream));
     return ICS_OK;
   });
 }
@@ -1280,14 +1291,14 @@ int ics_test_sweep_timeout(ics_handle hh, int32_t skip_row, int32_t spin_limit) 
       return ICS_ERR_STATE;
     }
     if (skip_row < 0 || skip_row >= N) return ICS_ERR_ARG;
-    if (!h.m.sweep_pad) h.m.sweep_pad = dalloc<double>(16ull * N);  // schedules with few levels
+    if (!h.m.sweep_pad) h.m.sweep_pad = dalloc<double>(h, 16ull * N);  // schedules with few levels
     // the forward tickets with skip_row left out
     std::vector<int> cells(N);
     ICS_CUDA(cudaMemcpy(cells.data(), h.m.fl_cells, N * sizeof(int), cudaMemcpyDeviceToHost));
     std::vector<int> order = ticket_order(cells, h.m.fl_ptr);
     for (int& c : order)
       if (c == skip_row) c = -1;
-    int* dev = upload(order);
+    int* dev = upload(h, order);
     ICS_CUDA(cudaMemsetAsync(&h.ks->status, 0, sizeof(int), h.stream));
     sweep_probe(h, dev, (int)(order.size() / SWEEP_TICKET), spin_limit);
     ICS_CUDA(cudaStreamSynchronize(h.stream));
@@ -1329,7 +1340,7 @@ struct CkptIO {
   void dev(double* d, size_t n) {
     const size_t nb = n * sizeof(double);
     if (out) ICS_CUDA(cudaMemcpy(out + pos, d, nb, cudaMemcpyDeviceToHost));
-    if (in) ICS_CUDA(cudaMemcpy(d, in + pos, nb, cudaMemcpyHostToDevice));
+    if (in) ICS_CUDA(cudaMemcpyAsync(d, in + pos, nb, cudaMemcpyHostToDevice, h.stream));
     pos += nb;
   }
 };
@@ -1456,6 +1467,7 @@ int ics_load_checkpoint(ics_handle hh, const void* buf, int64_t bytes) {
     ICS_CUDA(cudaStreamSynchronize(h.stream));
     CkptHeader tmp = hd;
     ckpt_walk(h, tmp, nullptr, (const char*)buf);
+    ICS_CUDA(cudaStreamSynchronize(h.stream));
     h.timeIndex = hd.timeIndex;
     h.initResValid = hd.initResValid != 0;
     h.prevResValid = hd.prevResValid != 0;
@@ -1491,20 +1503,20 @@ int ics_scalar_enable(ics_handle hh, const double* s, const int32_t* patch_fixed
   return guard(hh, [&](Handle& h) {
     const size_t N = h.m.N, F = h.m.F, B = h.m.B, P = h.m.npatches;
     if (!h.ss) {
-      h.ss = dalloc<double>(N);
-      h.ssB = dalloc<double>(B);
-      h.srhoS = dalloc<double>(N);
-      h.srhoS0 = dalloc<double>(N);
-      h.srhoS00 = dalloc<double>(N);
-      h.sgrad = dalloc<double>(3 * N);
-      h.sgradL = dalloc<double>(3 * N);
-      h.sface = dalloc<double>(5 * (F + B));
-      h.sblk = dalloc<double>((size_t)h.m.nslots * 32);
-      h.sdg = dalloc<double>(N);
-      h.srD = dalloc<double>(N);
-      h.ssrc = dalloc<double>(N);
-      h.sFixed = dalloc<int>(P ? P : 1);
-      h.sValue = dalloc<double>(P ? P : 1);
+      h.ss = dalloc<double>(h, N);
+      h.ssB = dalloc<double>(h, B);
+      h.srhoS = dalloc<double>(h, N);
+      h.srhoS0 = dalloc<double>(h, N);
+      h.srhoS00 = dalloc<double>(h, N);
+      h.sgrad = dalloc<double>(h, 3 * N);
+      h.sgradL = dalloc<double>(h, 3 * N);
+      h.sface = dalloc<double>(h, 5 * (F + B));
+      h.sblk = dalloc<double>(h, (size_t)h.m.nslots * 32);
+      h.sdg = dalloc<double>(h, N);
+      h.srD = dalloc<double>(h, N);
+      h.ssrc = dalloc<double>(h, N);
+      h.sFixed = dalloc<int>(h, P ? P : 1);
+      h.sValue = dalloc<double>(h, P ? P : 1);
     }
     std::vector<int> fx(P, 0);
     std::vector<double> val(P, 0.0);
@@ -1513,8 +1525,8 @@ int ics_scalar_enable(ics_handle hh, const double* s, const int32_t* patch_fixed
       val[p] = patch_value ? patch_value[p] : 0.0;
     }
     if (P) {
-      ICS_CUDA(cudaMemcpy(h.sFixed, fx.data(), P * sizeof(int), cudaMemcpyHostToDevice));
-      ICS_CUDA(cudaMemcpy(h.sValue, val.data(), P * sizeof(double), cudaMemcpyHostToDevice));
+      ICS_CUDA(cudaMemcpyAsync(h.sFixed, fx.data(), P * sizeof(int), cudaMemcpyHostToDevice, h.stream));
+      ICS_CUDA(cudaMemcpyAsync(h.sValue, val.data(), P * sizeof(double), cudaMemcpyHostToDevice, h.stream));
     }
     ICS_CUDA(cudaMemcpyAsync(h.ss, s, N * sizeof(double), cudaMemcpyHostToDevice, h.stream));
     k_scalar_init<<<grid_for(N, 256), 256, 0, h.stream>>>((int)N, h.ss, h.W, h.srhoS);
@@ -1877,8 +1889,9 @@ int ics_set_hb(ics_handle hh, int32_t n, const double* D) {
     if (h.m.Dhb) ICS_CUDA(cudaFree(h.m.Dhb));
     h.m.Dhb = nullptr;
     if (n > 1) {
-      h.m.Dhb = dalloc<double>((size_t)n * n);
-      ICS_CUDA(cudaMemcpy(h.m.Dhb, D, sizeof(double) * n * n, cudaMemcpyHostToDevice));
+      h.m.Dhb = dalloc<double>(h, (size_t)n * n);
+      ICS_CUDA(cudaMemcpyAsync(h.m.Dhb, D, sizeof(double) * n * n, cudaMemcpyHostToDevice, h.stream));
+      ICS_CUDA(cudaStreamSynchronize(h.stream));
     }
     h.m.nInst = n;
     h.m.Nc = h.m.N / n;
@@ -1928,8 +1941,9 @@ int ics_set_hb_zone(ics_handle hh, const int32_t* zone, int32_t cyl_coords, cons
     if (zone) {
       std::vector<unsigned char> mask(h.m.N);
       for (int c = 0; c < h.m.N; ++c) mask[c] = zone[c % h.m.Nc] != 0;
-      h.hbZoneBuf = dalloc<unsigned char>(h.m.N);
-      ICS_CUDA(cudaMemcpy(h.hbZoneBuf, mask.data(), h.m.N, cudaMemcpyHostToDevice));
+      h.hbZoneBuf = dalloc<unsigned char>(h, h.m.N);
+      ICS_CUDA(cudaMemcpyAsync(h.hbZoneBuf, mask.data(), h.m.N, cudaMemcpyHostToDevice, h.stream));
+      ICS_CUDA(cudaStreamSynchronize(h.stream));
       h.m.hbZone = h.hbZoneBuf;
     }
     h.m.hbCyl = cyl_coords ? 1 : 0;
@@ -1970,8 +1984,8 @@ int ics_set_phase_lag(ics_handle hh, const int32_t* mode, const double* P) {
     free_exact(h);  // the stencil gains the other instances' partners
     drop_graphs(h);
     if (!mode) return ICS_OK;
-    h.m.plagMode = upload(std::vector<int>(mode, mode + np));
-    h.m.plagP = upload(std::vector<double>(P, P + (size_t)np * n * n));
+    h.m.plagMode = upload(h, std::vector<int>(mode, mode + np));
+    h.m.plagP = upload(h, std::vector<double>(P, P + (size_t)np * n * n));
     return ICS_OK;
   });
 }
@@ -2014,11 +2028,11 @@ int ics_set_mrf(ics_handle hh, const double* omega, const double* face_velocity,
       for (int k = 0; k < 3; ++k) om[(size_t)k * N + i] = omega[3 * i + k];
     for (int b = 0; b < B; ++b)
       for (int k = 0; k < 3; ++k) bu[(size_t)k * B + b] = boundary_U[3 * b + k];
-    m.mrfOm = upload(om);
-    m.mrfU = upload(std::vector<double>(face_velocity, face_velocity + F + B));
+    m.mrfOm = upload(h, om);
+    m.mrfU = upload(h, std::vector<double>(face_velocity, face_velocity + F + B));
     if (B > 0) {
-      m.mrfBU = upload(bu);
-      m.mrfBIn = upload(std::vector<int>(included, included + B));
+      m.mrfBU = upload(h, bu);
+      m.mrfBIn = upload(h, std::vector<int>(included, included + B));
     }
     m.mrfEvery = mode == ICS_MRF_EVERY_UPDATE;
     // createFields.H:262-263: the boundary velocity is assigned at once

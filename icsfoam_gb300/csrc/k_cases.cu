@@ -709,14 +709,15 @@ void set_cases(Handle& h, int n, const int* start) {
   };
   const size_t bytes = layout(nullptr);
   ICS_CUDA(cudaMalloc(&S.mem, bytes));
-  ICS_CUDA(cudaMemset(S.mem, 0, bytes));
+  ICS_CUDA(cudaMemsetAsync(S.mem, 0, bytes, h.stream));
   layout((char*)S.mem);
-  ICS_CUDA(cudaMemcpy(dSegCase, segCase.data(), ns * sizeof(int), cudaMemcpyHostToDevice));
-  ICS_CUDA(cudaMemcpy(dSegBeg, segBeg.data(), ns * sizeof(int), cudaMemcpyHostToDevice));
-  ICS_CUDA(cudaMemcpy(dSegEnd, segEnd.data(), ns * sizeof(int), cudaMemcpyHostToDevice));
-  ICS_CUDA(cudaMemcpy(dCaseSeg, caseSeg.data(), (n + 1) * sizeof(int), cudaMemcpyHostToDevice));
-  ICS_CUDA(cudaMemcpy(dStart, start, (n + 1) * sizeof(int), cudaMemcpyHostToDevice));
-  ICS_CUDA(cudaMemcpy(S.caseOf, caseOf.data(), N * sizeof(int), cudaMemcpyHostToDevice));
+  ICS_CUDA(cudaMemcpyAsync(dSegCase, segCase.data(), ns * sizeof(int), cudaMemcpyHostToDevice, h.stream));
+  ICS_CUDA(cudaMemcpyAsync(dSegBeg, segBeg.data(), ns * sizeof(int), cudaMemcpyHostToDevice, h.stream));
+  ICS_CUDA(cudaMemcpyAsync(dSegEnd, segEnd.data(), ns * sizeof(int), cudaMemcpyHostToDevice, h.stream));
+  ICS_CUDA(cudaMemcpyAsync(dCaseSeg, caseSeg.data(), (n + 1) * sizeof(int), cudaMemcpyHostToDevice, h.stream));
+  ICS_CUDA(cudaMemcpyAsync(dStart, start, (n + 1) * sizeof(int), cudaMemcpyHostToDevice, h.stream));
+  ICS_CUDA(cudaMemcpyAsync(S.caseOf, caseOf.data(), N * sizeof(int), cudaMemcpyHostToDevice, h.stream));
+  ICS_CUDA(cudaStreamSynchronize(h.stream));
   D.segCase = dSegCase;
   D.segBeg = dSegBeg;
   D.segEnd = dSegEnd;

@@ -225,7 +225,10 @@ void build_exact_pattern(Handle& h) {
   }
   auto up = [&](const std::vector<int>& v) {
     int* p = xalloc<int>(v.size());
-    if (!v.empty()) ICS_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice));
+    if (!v.empty()) {
+      ICS_CUDA(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice, h.stream));
+      ICS_CUDA(cudaStreamSynchronize(h.stream));
+    }
     return p;
   };
   h.xptr = up(ptr);
