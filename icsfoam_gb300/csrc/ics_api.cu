@@ -634,6 +634,8 @@ int do_jacobian(Handle& h) {
   return ICS_OK;
 }
 
+constexpr const char* TIMEOUT_TEXT = "a bounded device wait of the linear solver gave up";
+
 int do_solve(Handle& h, ics_solver_perf* perf) {
   Range rg("ics gmres");
   if (!h.haveMatrix) {
@@ -665,7 +667,7 @@ int do_solve(Handle& h, ics_solver_perf* perf) {
     p.converged = conv && st == ICS_OK;
     h.haveIncrement = true;
     if (perf) *perf = p;
-    if (st) h.err = st == ICS_ERR_TIMEOUT ? "LU-SGS sweep wait gave up" : "non-finite Krylov residual in a case";
+    if (st) h.err = st == ICS_ERR_TIMEOUT ? TIMEOUT_TEXT : "non-finite Krylov residual in a case";
     return st;
   }
   const int st = gmres_solve(h, &p, h.initRes);
@@ -673,7 +675,9 @@ int do_solve(Handle& h, ics_solver_perf* perf) {
   h.initResValid = true;
   for (int J = 0; J < h.m.nInst; ++J) std::memcpy(h.ctl[J].residuals, &h.initRes[5 * J], 5 * sizeof(double));
   if (perf) *perf = p;
-  if (st) h.err = st == ICS_ERR_BREAKDOWN ? "zero Krylov norm" : "non-finite Krylov residual";
+  if (st)
+    h.err = st == ICS_ERR_TIMEOUT ? TIMEOUT_TEXT
+                                  : (st == ICS_ERR_BREAKDOWN ? "zero Krylov norm" : "non-finite Krylov residual");
   return st;
 }
 
@@ -1314,6 +1318,16 @@ int ics_test_sweep_timeout(ics_handle hh, int32_t skip_row, int32_t spin_limit) 
   });
 }
 
+int ics_test_column_wait(ics_handle hh, int32_t spin_limit) {
+  if (!hh || spin_limit < 0) return ICS_ERR_ARG;
+  return guard(hh, [&](Handle& h) {
+    ICS_CUDA(cudaStreamSynchronize(h.stream));
+    h.columnProbe = spin_limit;
+    drop_graphs(h);  // the captured launches hold the grid and the bound
+    return ICS_OK;
+  });
+}
+
 // checkpoint / resume ----------------------------------------------------------
 // Raw binary: a fixed header, then the arrays in a fixed order.  Everything
 // the next pseudo iteration reads is included (state, old time levels,
@@ -1567,7 +1581,7 @@ int ics_scalar_transport(ics_handle hh, int32_t n_iterations, ics_solver_perf* p
       }
       const int st = scalar_gmres(h, dx, &pf);
       if (st && st != ICS_ERR_BREAKDOWN) {
-        h.err = "non-finite scalar Krylov residual";
+        h.err = st == ICS_ERR_TIMEOUT ? TIMEOUT_TEXT : "non-finite scalar Krylov residual";
         return st;
       }
       launch_scalar_update(h, dx);

@@ -19,8 +19,10 @@
 //
 // The slots start as a sentinel (all bits set, which no sum is published as)
 // and are written once per column; a column resets the slots of the next one.
-// The waits are bounded (status bit 8).  One further block, outside the
-// exchange, rotates the Hessenberg column of the direction before.
+// The waits are bounded: a block whose wait runs out, or that sees while it
+// waits that another's has (status bit 8), leaves the column.  One further
+// block, outside the exchange, rotates the Hessenberg column of the direction
+// before.
 //
 // FP32 sums: a thread adds two runs of at most 36 products in FP32 (and runs of
 // 32 of what its registers do not hold), everything across threads is FP64.
@@ -99,7 +101,7 @@ constexpr int column_ring = T * U <= 512 * 12 ? 4 : 3;
 template <typename TV, int T, int U, bool REST>
 __global__ void __launch_bounds__(T, 1)
     k_column(long n, long slice, TV* __restrict__ w, TV* __restrict__ V, long vs, int dir, int m, KrylovScalars* ks,
-             double* __restrict__ slots, double* __restrict__ next_slots) {
+             double* __restrict__ slots, double* __restrict__ next_slots, int G, int spin_limit) {
   using VT = typename V16<TV>::T;
   using ST = std::conditional_t<REST, double, TV>;
   constexpr int L = V16<TV>::n;
@@ -108,8 +110,8 @@ __global__ void __launch_bounds__(T, 1)
   __shared__ ST sums[T];
   __shared__ double warpSum[4];
   __shared__ double result;
+  __shared__ bool gaveUp;
   const int tid = threadIdx.x, lane = tid & 31;
-  const int G = (int)gridDim.x - 1;
   if ((int)blockIdx.x == G) {  // the helper: not part of the exchange
     if (tid == 0 && dir > 0) dev_hess(ks, dir - 1, m);
     return;
@@ -144,7 +146,10 @@ __global__ void __launch_bounds__(T, 1)
 #pragma unroll
   for (int hv = 0; hv < RING; ++hv) issue(hv);
   for (int s = tid; s < m + 2; s += T) next_slots[(size_t)s * G + blockIdx.x] = __longlong_as_double(-1LL);
-  if (ks->status) return;
+  if (ks->status) {
+    copy_wait<0>();
+    return;
+  }
   VT x[U];
 #pragma unroll
   for (int u = 0; u < U; ++u) {
@@ -261,6 +266,7 @@ __global__ void __launch_bounds__(T, 1)
       // every slot of the step, all loads of a poll in flight together
       double v[5];
       int it = 0;
+      bool stop = false;
       if (G > PAUSE_BLOCKS) __nanosleep(PAUSE_FIRST);
       while (true) {
 #pragma unroll
@@ -274,10 +280,12 @@ __global__ void __launch_bounds__(T, 1)
 #pragma unroll
         for (int k = 0; k < 5; ++k) ready = ready && __double_as_longlong(v[k]) != -1LL;
         if (__all_sync(0xffffffffu, ready)) break;
-        if (++it > COLUMN_SPIN_LIMIT) {
-          if (lane == 0) atomicOr(&ks->status, 8);
-          break;
-        }
+        ++it;
+        stop = it > spin_limit;
+        if (stop && lane == 0) atomicOr(&ks->status, 8);
+        if ((it & 63) == 0) stop = stop || (ld_relaxed_int(&ks->status) & 8);
+        stop = __any_sync(0xffffffffu, stop);
+        if (stop) break;
         if (G > PAUSE_BLOCKS) __nanosleep(PAUSE_NEXT);
       }
 #pragma unroll
@@ -291,7 +299,8 @@ __global__ void __launch_bounds__(T, 1)
       for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
       if (lane == 0) {
         result = s;
-        if (blockIdx.x == 0) {
+        gaveUp = stop;
+        if (blockIdx.x == 0 && !stop) {
           if (j <= dir)
             ks->H[j * m + dir] = s;
           else if (dir >= 0)
@@ -300,6 +309,10 @@ __global__ void __launch_bounds__(T, 1)
       }
     }
     __syncthreads();
+    if (gaveUp) {
+      copy_wait<0>();
+      return;
+    }
     total = result;
     h = TV(total);
   }
@@ -326,9 +339,12 @@ void launch_column(Handle& h, int blocks, long slice, long n, TV* w, TV* V, long
   const size_t smem = (size_t)column_ring<T, U> * (U / 2) * T * 16;
   ICS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   KrylovScalars* ks = h.ks;
-  void* args[] = {&n, &slice, &w, &V, &vs, &dir, &m, &ks, &slots, &next};
+  int spin = h.columnProbe ? h.columnProbe : COLUMN_SPIN_LIMIT;
+  void* args[] = {&n, &slice, &w, &V, &vs, &dir, &m, &ks, &slots, &next, &blocks, &spin};
+  // with the probe the last block of the exchange (and the helper) never runs
+  const int grid = h.columnProbe && blocks > 1 ? blocks - 1 : blocks + 1;
   ICS_LAUNCH(h, ICS_K_MGS,
-             ICS_CUDA(cudaLaunchCooperativeKernel((const void*)kern, dim3(blocks + 1), dim3(T), args, smem, h.stream)));
+             ICS_CUDA(cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(T), args, smem, h.stream)));
 }
 
 // the instance with the fewest chunks per thread that holds a slice: chunks a

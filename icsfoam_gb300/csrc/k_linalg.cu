@@ -554,11 +554,6 @@ constexpr int SWEEP_THREADS = 32;  // one warp per block
 template <typename TB, typename TV>
 constexpr int sweep_rows = sizeof(TB) == 8 && sizeof(TV) == 8 ? 2 : 8;
 
-__device__ __forceinline__ int ld_relaxed_int(const int* p) {
-  int v;
-  asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
 __device__ __forceinline__ void ld_relaxed5(const float* p, float* v) {
   asm volatile("ld.relaxed.gpu.global.v4.f32 {%0, %1, %2, %3}, [%4];"
                : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
@@ -1359,6 +1354,11 @@ static int smooth_t(Handle& h, ResIO& p) {
 }
 
 
+// the error of a solve from its status flags
+static int krylov_error(int status) {
+  return status & 8 ? ICS_ERR_TIMEOUT : status & 4 ? ICS_ERR_NONFINITE : ICS_ERR_BREAKDOWN;
+}
+
 template <typename TB, typename TV>
 static int gmres_t(Handle& h, ResIO& p) {
   const int N = h.m.N, m = h.cfg.c.n_directions;
@@ -1425,8 +1425,7 @@ static int gmres_t(Handle& h, ResIO& p) {
     ICS_CUDA(cudaMemcpyAsync(&h.ksHost->status, &ks->status, sizeof(int), cudaMemcpyDeviceToHost, st));
     ICS_CUDA(cudaStreamSynchronize(st));
     if (h.ksHost->status) {
-      status = (h.ksHost->status & 8) ? ICS_ERR_TIMEOUT
-                                      : ((h.ksHost->status & 4) ? ICS_ERR_NONFINITE : ICS_ERR_BREAKDOWN);
+      status = krylov_error(h.ksHost->status);
       p.nIter++;
       break;
     }
@@ -1777,7 +1776,7 @@ int scalar_gmres(Handle& h, double* dx, ics_solver_perf* perf) {
     ICS_CUDA(cudaStreamSynchronize(st));
     perf->n_iterations++;
     if (stt) {
-      status = (stt & 4) ? ICS_ERR_NONFINITE : ICS_ERR_BREAKDOWN;
+      status = krylov_error(stt);
       break;
     }
     perf->final_res[0] = rs / nf;

@@ -8,6 +8,12 @@
 
 namespace ics {
 
+__device__ __forceinline__ int ld_relaxed_int(const int* p) {
+  int v;
+  asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
 // 16-byte vector of the Krylov element type
 template <typename TV>
 struct V16;
@@ -219,7 +225,7 @@ __device__ __forceinline__ void dev_hess(KrylovScalars* ks, int i, int m) {
 __device__ __forceinline__ void dev_beta0(KrylovScalars* ks, double beta, int m) {
   for (int i = 0; i <= m; ++i) ks->bh[i] = 0.0;
   ks->bh[0] = beta;
-  if (!(beta > 0.0)) ks->status = isfinite(beta) ? 2 : 4;
+  if (!(beta > 0.0)) atomicOr(&ks->status, isfinite(beta) ? 2 : 4);  // beside bit 8 of a wait that gave up
 }
 
 }  // namespace ics

@@ -361,6 +361,11 @@ int ics_get_scalar(ics_handle h, double* s, double* rhoS);
  * Returns ICS_ERR_TIMEOUT when the waits report as designed (ICS_OK when no
  * row depends on skip_row); the context stays usable.                       */
 int ics_test_sweep_timeout(ics_handle h, int32_t skip_row, int32_t spin_limit);
+/* The same probe of the Gram-Schmidt columns: with spin_limit > 0 the handle's
+ * columns run without the last block of their exchange (systems of more than
+ * one block: over 128 16-byte chunks) and the others give up after spin_limit
+ * polls, so that solves return ICS_ERR_TIMEOUT; 0 restores them.            */
+int ics_test_column_wait(ics_handle h, int32_t spin_limit);
 
 /* ---- checkpoint / resume (the reference writes OpenFOAM time directories
  * and a pseudotimeState dictionary, pseudotimeControl.C:59-63,84-89) ------- */
