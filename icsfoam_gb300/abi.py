@@ -182,6 +182,7 @@ _MEASURE["case_stats"] = (C.c_int, [_P, _P, _P, _P])
 
 # bounded-wait probe (CUDA library only)
 _MEASURE["test_sweep_timeout"] = (C.c_int, [_P, C.c_int32, C.c_int32])
+_MEASURE["test_sweep_wait"] = (C.c_int, [_P, C.c_int32, C.c_int32])
 _MEASURE["test_column_wait"] = (C.c_int, [_P, C.c_int32])
 
 # checkpoint / resume (CUDA library only)
@@ -558,6 +559,10 @@ class CaseHandle:
     def test_sweep_timeout(self, skip_row: int, spin_limit: int) -> int:
         """Status of the bounded-wait probe (ICS_ERR_TIMEOUT expected when rows depend on skip_row)."""
         return int(self.b.fn["test_sweep_timeout"](self.h, int(skip_row), int(spin_limit)))
+
+    def test_sweep_wait(self, skip_row: int, spin_limit: int) -> None:
+        """Leave a row out of the forward sweeps of all solves (spin_limit 0: put it back)."""
+        self._check(self.b.fn["test_sweep_wait"](self.h, int(skip_row), int(spin_limit)), "test_sweep_wait")
 
     def test_column_wait(self, spin_limit: int) -> None:
         """Leave the last block of the Gram-Schmidt columns out (0: put it back)."""

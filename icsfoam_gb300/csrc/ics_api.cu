@@ -115,7 +115,7 @@ void free_all(Handle& h) {
                   h.ss, h.ssB, h.srhoS, h.srhoS0, h.srhoS00, h.sgrad, h.sgradL, h.sface, h.sblk, h.sdg, h.srD,
                   h.ssrc, h.sFixed, h.sValue,
                   h.blk, h.dg,
-                  h.dginv, h.rD, h.kv, h.kw, h.kx, h.kb, h.kt, h.dW, h.partials, h.counter, h.ks, h.colSlots, h.scratch,
+                  h.dginv, h.rD, h.kv, h.kw, h.kx, h.kb, h.kt, h.dW, h.partials, h.counter, h.ks, h.colSlots, h.sweepProbeOrder, h.scratch,
                   h.ibuf};
   drop_graphs(h);
   free_exact(h);
@@ -1285,7 +1285,17 @@ int ics_timer_stop(ics_handle hh, double* ms) {
   });
 }
 
-// failure-detection probe ------------------------------------------------------
+// failure-detection probes -----------------------------------------------------
+// the forward tickets with a row left out: it never writes its result
+static std::vector<int> tickets_without(Handle& h, int row) {
+  std::vector<int> cells(h.m.N);
+  ICS_CUDA(cudaMemcpy(cells.data(), h.m.fl_cells, cells.size() * sizeof(int), cudaMemcpyDeviceToHost));
+  std::vector<int> order = ticket_order(cells, h.m.fl_ptr);
+  for (int& c : order)
+    if (c == row) c = -1;
+  return order;
+}
+
 int ics_test_sweep_timeout(ics_handle hh, int32_t skip_row, int32_t spin_limit) {
   if (!hh || spin_limit < 1) return ICS_ERR_ARG;
   return guard(hh, [&](Handle& h) {
@@ -1296,12 +1306,7 @@ int ics_test_sweep_timeout(ics_handle hh, int32_t skip_row, int32_t spin_limit) 
     }
     if (skip_row < 0 || skip_row >= N) return ICS_ERR_ARG;
     if (!h.m.sweep_pad) h.m.sweep_pad = dalloc<double>(h, 16ull * N);  // schedules with few levels
-    // the forward tickets with skip_row left out
-    std::vector<int> cells(N);
-    ICS_CUDA(cudaMemcpy(cells.data(), h.m.fl_cells, N * sizeof(int), cudaMemcpyDeviceToHost));
-    std::vector<int> order = ticket_order(cells, h.m.fl_ptr);
-    for (int& c : order)
-      if (c == skip_row) c = -1;
+    const std::vector<int> order = tickets_without(h, skip_row);
     int* dev = upload(h, order);
     ICS_CUDA(cudaMemsetAsync(&h.ks->status, 0, sizeof(int), h.stream));
     sweep_probe(h, dev, (int)(order.size() / SWEEP_TICKET), spin_limit);
@@ -1313,6 +1318,26 @@ int ics_test_sweep_timeout(ics_handle hh, int32_t skip_row, int32_t spin_limit) 
     if (st & 8) {
       h.err = "a sync-free sweep wait gave up (as the probe intends)";
       return ICS_ERR_TIMEOUT;
+    }
+    return ICS_OK;
+  });
+}
+
+int ics_test_sweep_wait(ics_handle hh, int32_t skip_row, int32_t spin_limit) {
+  if (!hh || spin_limit < 0) return ICS_ERR_ARG;
+  return guard(hh, [&](Handle& h) {
+    if (spin_limit && (skip_row < 0 || skip_row >= h.m.N || !h.m.sw_fwd)) {
+      h.err = "test_sweep_wait needs a cell of a mesh with sync-free sweeps";
+      return ICS_ERR_ARG;
+    }
+    ICS_CUDA(cudaStreamSynchronize(h.stream));
+    dfree(h.sweepProbeOrder);
+    h.sweepProbeOrder = nullptr;
+    h.sweepProbe = 0;
+    drop_graphs(h);  // the captured launches hold the order and the bound
+    if (spin_limit) {
+      h.sweepProbeOrder = upload(h, tickets_without(h, skip_row));
+      h.sweepProbe = spin_limit;
     }
     return ICS_OK;
   });
@@ -1810,6 +1835,7 @@ int krylov_entry(ics_handle hh, const double* rhs, double* sol, const ics_krylov
     stage_in(h, rhs, d, 0);
     ics_krylov_result r{};
     const int st = solve(h, d, x, *opts, &r);
+    if (st == ICS_ERR_TIMEOUT) h.err = TIMEOUT_TEXT;
     if (result) *result = r;
     stage_out(h, x, sol, 0);
     return st;

@@ -305,6 +305,8 @@ struct Handle {
   KrylovScalars* ks = nullptr;  // device
   KrylovScalars* ksHost = nullptr;  // pinned mirror
   double* colSlots = nullptr;   // partial sums of the Gram-Schmidt columns (k_column.cu)
+  int sweepProbe = 0;           // > 0: forward sweeps run in sweepProbeOrder, which lacks a row, with this wait bound
+  int* sweepProbeOrder = nullptr;
   int columnProbe = 0;          // > 0: columns run without their last block, with this wait bound
   int sms = 0;                  // multiprocessors of the device
   // host-side residual bookkeeping (setCoAndDeltaT.H, pseudotimeControl):

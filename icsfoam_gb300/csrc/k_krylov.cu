@@ -218,6 +218,7 @@ int gmres_matfree(Handle& h, const Ops& A, const double* b, double* x, const ics
     return std::sqrt(s);
   };
   ICS_CUDA(cudaMemsetAsync(x, 0, n * sizeof(double), st));
+  ICS_CUDA(cudaMemsetAsync(&h.ks->status, 0, sizeof(int), st));  // of the preconditioner's bounded waits
   const double bnorm = norm64(b);
   res->iterations = res->cycles = 0;
   res->rel_residual = 0.0;
@@ -293,8 +294,11 @@ int gmres_matfree(Handle& h, const Ops& A, const double* b, double* x, const ics
     // true residual r = b - A x
     A.op(x, d2);
     ICS_LAUNCH(h, ICS_K_VECTOR, k_sub64<<<G, KB, 0, st>>>(n, b, d2, d1));
-    beta = norm64(d1);
+    int status = 0;
+    ICS_CUDA(cudaMemcpyAsync(&status, &h.ks->status, sizeof(int), cudaMemcpyDeviceToHost, st));
+    beta = norm64(d1);  // waits for the stream
     res->rel_residual = beta / bnorm;
+    if (status & 8) return ICS_ERR_TIMEOUT;
     if (!std::isfinite(beta)) return ICS_ERR_NONFINITE;
     if (beta <= o.rel_tol * bnorm) {
       res->converged = 1;

@@ -1032,12 +1032,14 @@ static void lusgs_t(Handle& h, TV* r, const TB* blkIn = nullptr, const TB* rDIn 
     ICS_CUDA(cudaMemsetAsync(fwd, 0xff, 2 * padBytes, st));  // the sentinel in both outputs
     ICS_CUDA(cudaMemsetAsync(m.sweep_ticket, 0, 2 * sizeof(unsigned int), st));
     const int grid = sweep_grid(m, m.nsw_fwd, sweep_rows<TB, TV>);
+    const int spin = h.sweepProbe ? h.sweepProbe : SWEEP_SPIN_LIMIT;
+    const int* fwdOrder = h.sweepProbe ? h.sweepProbeOrder : m.sw_fwd;
     ICS_LAUNCH(h, ICS_K_LUSGS_FWD, k_lusgs_sweep<TB, TV, true><<<grid, SWEEP_THREADS, 0, st>>>(
-                                       m, blk, rD, r, fwd, nullptr, m.sw_fwd, m.nsw_fwd, m.sweep_ticket, status,
-                                       SWEEP_SPIN_LIMIT));
+                                       m, blk, rD, r, fwd, nullptr, fwdOrder, m.nsw_fwd, m.sweep_ticket, status,
+                                       spin));
     ICS_LAUNCH(h, ICS_K_LUSGS_REV, k_lusgs_sweep<TB, TV, false><<<grid, SWEEP_THREADS, 0, st>>>(
                                        m, blk, rD, fwd, rev, r, m.sw_rev, m.nsw_rev, m.sweep_ticket + 1, status,
-                                       SWEEP_SPIN_LIMIT));
+                                       spin));
     return;
   }
   // One or two levels (colour-blocked numberings): a launch per level.

@@ -361,6 +361,12 @@ int ics_get_scalar(ics_handle h, double* s, double* rhoS);
  * Returns ICS_ERR_TIMEOUT when the waits report as designed (ICS_OK when no
  * row depends on skip_row); the context stays usable.                       */
 int ics_test_sweep_timeout(ics_handle h, int32_t skip_row, int32_t spin_limit);
+/* The same for all sweeps of the handle's solves: with spin_limit > 0 the
+ * forward sweeps run without skip_row, and ics_solve_increment,
+ * ics_precondition, ics_tangent_solve and ics_adjoint_solve return
+ * ICS_ERR_TIMEOUT when a row depends on it; 0 restores them.  For meshes whose
+ * LU-SGS has more than two levels (ICS_ERR_ARG elsewhere).                  */
+int ics_test_sweep_wait(ics_handle h, int32_t skip_row, int32_t spin_limit);
 /* The same probe of the Gram-Schmidt columns: with spin_limit > 0 the handle's
  * columns run without the last block of their exchange (systems of more than
  * one block: over 128 16-byte chunks) and the others give up after spin_limit
