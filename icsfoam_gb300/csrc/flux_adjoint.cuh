@@ -162,8 +162,8 @@ __device__ __forceinline__ void flux_ausm_adjoint(const FState& L, const FState&
   const double uL = dot3(L.U, S) * im - um, uR = dot3(R.U, S) * im - um;
   const bool cOwnL = L.c >= uL, cOwnR = R.c >= -uR;
   const double mL = cOwnL ? L.c : uL, mR = cOwnR ? R.c : -uR;
+  const double cl = L.c * L.c / mL, cr = R.c * R.c / mR;  // ordered by flux_ausm's own quotients
   const double imL = 1.0 / mL, imR = 1.0 / mR;
-  const double cl = L.c * L.c * imL, cr = R.c * R.c * imR;
   const bool cfL = cl <= cr;
   const double cf = cfL ? cl : cr;
   const double icf = 1.0 / cf;

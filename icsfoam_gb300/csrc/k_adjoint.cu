@@ -177,9 +177,9 @@ __global__ void __launch_bounds__(128) k_adj_face(DevMesh m, ResParams P, const 
     if (TVD && used && (sch == ICS_RECON_VANLEER || sch == ICS_RECON_MINMOD)) {
       const double qo = q[k * N + o], qn = q[k * N + nb];
       const double d0 = m.dCC[f], d1 = m.dCC[F + f], d2 = m.dCC[2 * F + f];
-      const double gl = d0 * grad[(3 * k) * N + o] + d1 * grad[(3 * k + 1) * N + o] + d2 * grad[(3 * k + 2) * N + o];
-      const double gr = d0 * grad[(3 * k) * N + nb] + d1 * grad[(3 * k + 1) * N + nb] +
-                        d2 * grad[(3 * k + 2) * N + nb];
+      const double gl = project(d0, d1, d2, grad[(3 * k) * N + o], grad[(3 * k + 1) * N + o], grad[(3 * k + 2) * N + o]);
+      const double gr = project(d0, d1, d2, grad[(3 * k) * N + nb], grad[(3 * k + 1) * N + nb],
+                                grad[(3 * k + 2) * N + nb]);
       const double wf = m.w[f];
       double dl[3], dr[3];  // d(value)/d(qo, qn, projected gradient)
 #pragma unroll
@@ -253,9 +253,9 @@ __global__ void __launch_bounds__(128) k_adj_lim(DevMesh m, unsigned mask, unsig
         const int other = isOwn ? m.nei[f] : m.own[f];
         const double* g = isOwn ? m.gO : m.gN;
         const double dq = q[k * N + other] - qc;
-        G[0] = G[0] + g[f] * dq;
-        G[1] = G[1] + g[F + f] * dq;
-        G[2] = G[2] + g[2 * F + f] * dq;
+        G[0] = madd(g[f], dq, G[0]);
+        G[1] = madd(g[F + f], dq, G[1]);
+        G[2] = madd(g[2 * F + f], dq, G[2]);
         if (okey(dq) > okey(dmax)) {
           dmax = dq;
           srcMax = other;
@@ -268,9 +268,9 @@ __global__ void __launch_bounds__(128) k_adj_lim(DevMesh m, unsigned mask, unsig
       for (int e = b0; e < b1; ++e) {
         const int b = m.bface[e];
         const double v = bq[k * B + b] - qc;
-        G[0] = G[0] + m.gB[b] * v;
-        G[1] = G[1] + m.gB[B + b] * v;
-        G[2] = G[2] + m.gB[2 * B + b] * v;
+        G[0] = madd(m.gB[b], v, G[0]);
+        G[1] = madd(m.gB[B + b], v, G[1]);
+        G[2] = madd(m.gB[2 * B + b], v, G[2]);
         if (okey(v) > okey(dmax)) {
           dmax = v;
           srcMax = -1;
@@ -281,15 +281,15 @@ __global__ void __launch_bounds__(128) k_adj_lim(DevMesh m, unsigned mask, unsig
         }
       }
       if (m.limWiden > 0.0) {
-        const double wd = m.limWiden * (dmax - dmin);
-        dmax = dmax + wd;
-        dmin = dmin - wd;
+        const double range = dmax - dmin;
+        dmax = madd(m.limWiden, range, dmax);
+        dmin = madd(-m.limWiden, range, dmin);
       }
       // the largest positive / most negative face extrapolation and its d
       double epos = 0.0, eneg = 0.0, dpos[3] = {0, 0, 0}, dneg[3] = {0, 0, 0};
       bool small = false;
       auto faceExtrap = [&](double d0, double d1, double d2) {
-        const double ex = d0 * G[0] + d1 * G[1] + d2 * G[2];
+        const double ex = project(d0, d1, d2, G[0], G[1], G[2]);
         if (ogt(ex, SMALL)) {
           if (okey(ex) > okey(epos)) {
             epos = ex;
@@ -337,26 +337,28 @@ __global__ void __launch_bounds__(128) k_adj_lim(DevMesh m, unsigned mask, unsig
         sel = 3;
       }
       const bool anyFace = (e1 > e0) || (b1 > b0);
-      double lim = 1.0, lr = 1.0, dra = 0.0, drb = 0.0;
-      if (anyFace && sel != 0) {
+      double lim = 1.0, dra = 0.0, drb = 0.0;
+      double num = ra, den = rb;
+      if (LIMITED == 2) venkatakrishnan(ra, rb, num, den);
+      const bool below = anyFace && sel != 0 && num < den;  // as k_grad decides it
+      if (below) {
         if (LIMITED == 2) {
-          const double num = ra * ra + 2 * ra * rb, iden = 1.0 / (ra * ra + ra * rb + 2 * rb * rb);
-          lr = num * iden;
+          const double iden = 1.0 / den, lr = num * iden;
+          lim = lr;
           dra = ((2 * ra + 2 * rb) - lr * (2 * ra + rb)) * iden;
           drb = (2 * ra - lr * (ra + 4 * rb)) * iden;
         } else {
           dra = 1.0 / rb;
-          lr = ra / rb;
-          drb = -lr * dra;
+          lim = ra / rb;
+          drb = -lim * dra;
         }
-        lim = fmin(1.0, lr);
       }
       // g = lim G: G_bar = lim g_bar + (limiter terms), lim_bar = g_bar . G
       const double limBar = gb[0] * G[0] + gb[1] * G[1] + gb[2] * G[2];
       gb[0] *= lim;
       gb[1] *= lim;
       gb[2] *= lim;
-      if (anyFace && (sel == 1 || sel == 2) && !(1.0 <= lr)) {
+      if (below && sel != 3) {
         const double raBar = limBar * dra, rbBar = limBar * drb;
         double dmaxBar = 0.0, dminBar = 0.0;
         if (sel == 1) {

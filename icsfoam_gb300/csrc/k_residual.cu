@@ -40,7 +40,7 @@ __global__ void k_fields(int N, int B, const Real* __restrict__ W, const Real* _
     const Real rho = W[5 * i];
     const Real p = prim[i], T = prim[N + i];
     const Real U0 = prim[2 * N + i], U1 = prim[3 * N + i], U2 = prim[4 * N + i];
-    const Real E = P.Cv * T + 0.5 * (U0 * U0 + U1 * U1 + U2 * U2);
+    const Real E = total_energy(P.Cv, T, U0, U1, U2);
     const Real H = fmax(E, SMALL) + fmax(p / rho, SMALL);
     const Real cl = sqrt(P.gamma * (P.R * T));  // sqrt(gamma / psi)
     q[Q_RHO * N + i] = rho;
@@ -152,9 +152,9 @@ __global__ void __launch_bounds__(128) k_grad(DevMesh m, const Real* __restrict_
     for (int k = 0; k < NQ; ++k) {
       if (!((mask >> k) & 1)) continue;
       const Real dq = q[k * N + other] - qc[k];
-      g[k][0] = g[k][0] + G0 * dq;
-      g[k][1] = g[k][1] + G1 * dq;
-      g[k][2] = g[k][2] + G2 * dq;
+      g[k][0] = madd(G0, dq, g[k][0]);
+      g[k][1] = madd(G1, dq, g[k][1]);
+      g[k][2] = madd(G2, dq, g[k][2]);
       if (LIMITED) {
         qmax[k] = omax(qmax[k], dq);
         qmin[k] = omin(qmin[k], dq);
@@ -177,9 +177,9 @@ __global__ void __launch_bounds__(128) k_grad(DevMesh m, const Real* __restrict_
         if (!((mask >> k) & 1)) continue;
         const Real qn = plag ? plag_q(m, q, k, b, pc) : q[k * N + pc];
         const Real dq = qn - qc[k], sf = (1.0 - wb) * dq;
-        g[k][0] = g[k][0] + G0 * sf;
-        g[k][1] = g[k][1] + G1 * sf;
-        g[k][2] = g[k][2] + G2 * sf;
+        g[k][0] = madd(G0, sf, g[k][0]);
+        g[k][1] = madd(G1, sf, g[k][1]);
+        g[k][2] = madd(G2, sf, g[k][2]);
         if (LIMITED) {
           qmax[k] = omax(qmax[k], dq);
           qmin[k] = omin(qmin[k], dq);
@@ -191,9 +191,9 @@ __global__ void __launch_bounds__(128) k_grad(DevMesh m, const Real* __restrict_
     for (int k = 0; k < NQ; ++k) {
       if (!((mask >> k) & 1)) continue;
       const Real v = bq[k * B + b] - qc[k];
-      g[k][0] = g[k][0] + G0 * v;
-      g[k][1] = g[k][1] + G1 * v;
-      g[k][2] = g[k][2] + G2 * v;
+      g[k][0] = madd(G0, v, g[k][0]);
+      g[k][1] = madd(G1, v, g[k][1]);
+      g[k][2] = madd(G2, v, g[k][2]);
       if (LIMITED) {
         qmax[k] = omax(qmax[k], v);
         qmin[k] = omin(qmin[k], v);
@@ -214,9 +214,9 @@ __global__ void __launch_bounds__(128) k_grad(DevMesh m, const Real* __restrict_
       epos[k] = 0.0;
       eneg[k] = 0.0;
       if (widen) {  // cellLimited coefficient k < 1
-        const Real wd = m.limWiden * (qmax[k] - qmin[k]);
-        qmax[k] = qmax[k] + wd;
-        qmin[k] = qmin[k] - wd;
+        const Real range = qmax[k] - qmin[k];
+        qmax[k] = madd(m.limWiden, range, qmax[k]);
+        qmin[k] = madd(-m.limWiden, range, qmin[k]);
       }
     }
     // comparisons and extrema through the integer image of the doubles (okey)
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(128) k_grad(DevMesh m, const Real* __restrict_
 #pragma unroll
       for (int k = 0; k < NQ; ++k) {
         if (!((mask >> k) & 1)) continue;
-        faceExtrap(k, d0 * g[k][0] + d1 * g[k][1] + d2 * g[k][2]);
+        faceExtrap(k, project(d0, d1, d2, g[k][0], g[k][1], g[k][2]));
       }
     }
     for (int e = b0; e < b1; ++e) {
@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(128) k_grad(DevMesh m, const Real* __restrict_
 #pragma unroll
       for (int k = 0; k < NQ; ++k) {
         if (!((mask >> k) & 1)) continue;
-        faceExtrap(k, d0 * g[k][0] + d1 * g[k][1] + d2 * g[k][2]);
+        faceExtrap(k, project(d0, d1, d2, g[k][0], g[k][1], g[k][2]));
       }
     }
     const bool anyFace = (e1 > e0) || (b1 > b0);
@@ -277,9 +277,11 @@ __global__ void __launch_bounds__(128) k_grad(DevMesh m, const Real* __restrict_
         }
         have = true;
       }
-      // Venkatakrishnan (r^2 + 2r)/(r^2 + r + 2) and minmod min(r, 1), capped at 1
-      const Real lr = LIMITED == 2 ? (ra * ra + 2 * ra * rb) / (ra * ra + ra * rb + 2 * rb * rb) : ra / rb;
-      const Real lim = have && mag(lr) < mag(1.0) ? lr : Real(1.0);
+      // Venkatakrishnan and minmod r, capped at 1 where the numerator reaches
+      // the denominator
+      Real num = ra, den = rb;
+      if (LIMITED == 2) venkatakrishnan(ra, rb, num, den);
+      const Real lim = have && mag(num) < mag(den) ? num / den : Real(1.0);
       g[k][0] = g[k][0] * lim;
       g[k][1] = g[k][1] * lim;
       g[k][2] = g[k][2] * lim;

@@ -27,6 +27,42 @@ __device__ __forceinline__ int recon_of(const ResParams& P, int q) {
   return P.reconT;
 }
 
+// Sums of products with every rounding written out.  The residual, its forward
+// product (Real = Dual, whose value takes the same roundings) and its reverse
+// product decide their limiter branches on these values; left to the compiler's
+// contraction the kernels could round them differently and, at a tie, take
+// different branches.
+__device__ __forceinline__ double madd(double a, double b, double c) { return ::fma(a, b, c); }
+__device__ __forceinline__ Dual madd(double a, const Dual& b, const Dual& c) {
+  return Dual(::fma(a, b.v, c.v), ::fma(a, b.d, c.d));
+}
+// d . g
+template <typename Real>
+__device__ __forceinline__ Real project(double d0, double d1, double d2, const Real& g0, const Real& g1,
+                                        const Real& g2) {
+  return madd(d2, g2, madd(d1, g1, madd(d0, g0, Real(0.0))));
+}
+// specific total energy Cv T + |U|^2 / 2
+__device__ __forceinline__ double total_energy(double Cv, double T, double U0, double U1, double U2) {
+  return ::fma(Cv, T, 0.5 * ::fma(U2, U2, ::fma(U1, U1, __dmul_rn(U0, U0))));
+}
+__device__ __forceinline__ Dual total_energy(double Cv, const Dual& T, const Dual& U0, const Dual& U1,
+                                             const Dual& U2) {
+  return Dual(total_energy(Cv, T.v, U0.v, U1.v, U2.v), Cv * T.d + U0.v * U0.d + U1.v * U1.d + U2.v * U2.d);
+}
+// numerator and denominator of Venkatakrishnan's (r^2 + 2 r) / (r^2 + r + 2),
+// r = ra / rb; equal where r = 2 exactly, a linear profile on uniform cells
+__device__ __forceinline__ void venkatakrishnan(double ra, double rb, double& num, double& den) {
+  const double aa = __dmul_rn(ra, ra), ab = __dmul_rn(ra, rb), bb = __dmul_rn(rb, rb);
+  num = ::fma(2.0, ab, aa);
+  den = __dadd_rn(::fma(2.0, bb, ab), aa);
+}
+__device__ __forceinline__ void venkatakrishnan(const Dual& ra, const Dual& rb, Dual& num, Dual& den) {
+  venkatakrishnan(ra.v, rb.v, num.v, den.v);
+  num.d = 2.0 * (ra.d * (ra.v + rb.v) + ra.v * rb.d);
+  den.d = ra.d * (2.0 * ra.v + rb.v) + rb.d * (ra.v + 4.0 * rb.v);
+}
+
 // TVD limitedScheme face value from the two cell values and the upwind
 // cell's gradient projected on C_nei - C_own (NVD/TVD r with vanLeer or Minmod)
 template <typename Real, typename GT>
@@ -57,7 +93,7 @@ __device__ __forceinline__ Real reconstruct(const DevMesh& m, int scheme, int k,
   if (scheme == ICS_RECON_VANLEER || scheme == ICS_RECON_MINMOD) {
     const int c = dir > 0 ? o : nb;
     const double d0 = m.dCC[f], d1 = m.dCC[F + f], d2 = m.dCC[2 * F + f];
-    const Real gradcf = d0 * grad[(3 * k) * N + c] + d1 * grad[(3 * k + 1) * N + c] + d2 * grad[(3 * k + 2) * N + c];
+    const Real gradcf = project(d0, d1, d2, grad[(3 * k) * N + c], grad[(3 * k + 1) * N + c], grad[(3 * k + 2) * N + c]);
     return tvd_face(scheme, m.w[f], wUp, qo, qn, gradcf);
   }
   // MUSCL: upwind value + limited-gradient extrapolation (the small products
@@ -65,8 +101,8 @@ __device__ __forceinline__ Real reconstruct(const DevMesh& m, int scheme, int k,
   const int c = dir > 0 ? o : nb;
   const double* d = dir > 0 ? m.dOwn : m.dNei;
   const Real base = dir > 0 ? qo : qn;
-  return base + (d[f] * grad[(3 * k) * N + c] + d[F + f] * grad[(3 * k + 1) * N + c] +
-                 d[2 * F + f] * grad[(3 * k + 2) * N + c]);
+  return base + project(d[f], d[F + f], d[2 * F + f], grad[(3 * k) * N + c], grad[(3 * k + 1) * N + c],
+                        grad[(3 * k + 2) * N + c]);
 }
 
 ResParams res_params(const Handle& h);
