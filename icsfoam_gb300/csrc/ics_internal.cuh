@@ -352,15 +352,15 @@ struct Handle {
   double* xblk = nullptr;  // [nnz][25]
   long long xnnz = 0;
   int xncol = 0;
-  // whether xblk holds the exact Jacobian at the current state, and how many
-  // ics_vjp calls at this state the reverse chain has served instead; a
-  // change of state (haveExact = false) restarts the count
+  // whether xblk holds the exact Jacobian at the current state, and whether
+  // ics_vjp was answered at this state by the reverse chain instead; a change
+  // of state (haveExact = false) clears both
   struct ExactState {
     bool have = false;
-    int served = 0;
+    bool reversed = false;
     ExactState& operator=(bool b) {
       have = b;
-      served = 0;
+      reversed = false;
       return *this;
     }
     operator bool() const { return have; }

@@ -411,9 +411,11 @@ int ics_assemble_exact_jacobian(ics_handle h, int64_t* nnz_blocks, int32_t* n_co
  * pointer may be NULL.  ICS_ERR_STATE when not assembled at this state.    */
 int ics_get_exact_jacobian(ics_handle h, int32_t* row_ptr, int32_t* cols, double* blocks);
 /* Vector-Jacobian product JTu = (d(R V)/dW)^T u with the exact Jacobian: the
- * assembled one when it is there, else, where ics_vjp_recompute covers the
- * case, its reverse chain (equal up to round-off) for the first sixteen calls
- * at a state, and an assembly after those.  Pointers as in ics_jvp.         */
+ * assembled one where ics_assemble_exact_jacobian (or ics_get_exact_jacobian)
+ * was called at this state, else the reverse chain of ics_vjp_recompute where
+ * that covers the case (equal up to round-off), else an assembly.  Equal calls
+ * at a state give equal bits until the program assembles; a program that makes
+ * over some 300 products at one state does so first.  Pointers as in ics_jvp. */
 int ics_vjp(ics_handle h, const double* u, double* JTu, int32_t device);
 /* The same vector-Jacobian product by reverse mode, storing no Jacobian:
  * the face and cell maps of the residual are transposed in reverse order and
