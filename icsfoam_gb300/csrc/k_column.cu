@@ -19,10 +19,11 @@
 //
 // The slots start as a sentinel (all bits set, which no sum is published as)
 // and are written once per column; a column resets the slots of the next one.
-// The waits are bounded: a block whose wait runs out, or that sees while it
-// waits that another's has (status bit 8), leaves the column.  One further
-// block, outside the exchange, rotates the Hessenberg column of the direction
-// before.
+// The waits are bounded: a block whose wait runs out sets status bit 8, and from
+// then on every wait of every block ends within 64 polls, with a NaN for a sum
+// (the solve reports the flag; a test of it in each step would cost 1% of a
+// small system's solve).  One further block, outside the exchange, rotates the
+// Hessenberg column of the direction before.
 //
 // FP32 sums: a thread adds two runs of at most 36 products in FP32 (and runs of
 // 32 of what its registers do not hold), everything across threads is FP64.
@@ -98,6 +99,10 @@ constexpr int BATCH = 4;
 template <int T, int U>
 constexpr int column_ring = T * U <= 512 * 12 ? 4 : 3;
 
+// the sentinel of an unwritten slot: a NaN that no addition produces
+__device__ __forceinline__ double no_sum() { return __longlong_as_double(-1LL); }
+__device__ __forceinline__ bool is_no_sum(double s) { return __double_as_longlong(s) == -1LL; }
+
 template <typename TV, int T, int U, bool REST>
 __global__ void __launch_bounds__(T, 1)
     k_column(long n, long slice, TV* __restrict__ w, TV* __restrict__ V, long vs, int dir, int m, KrylovScalars* ks,
@@ -110,7 +115,6 @@ __global__ void __launch_bounds__(T, 1)
   __shared__ ST sums[T];
   __shared__ double warpSum[4];
   __shared__ double result;
-  __shared__ bool gaveUp;
   const int tid = threadIdx.x, lane = tid & 31;
   if ((int)blockIdx.x == G) {  // the helper: not part of the exchange
     if (tid == 0 && dir > 0) dev_hess(ks, dir - 1, m);
@@ -145,7 +149,7 @@ __global__ void __launch_bounds__(T, 1)
   };
 #pragma unroll
   for (int hv = 0; hv < RING; ++hv) issue(hv);
-  for (int s = tid; s < m + 2; s += T) next_slots[(size_t)s * G + blockIdx.x] = __longlong_as_double(-1LL);
+  for (int s = tid; s < m + 2; s += T) next_slots[(size_t)s * G + blockIdx.x] = no_sum();
   if (ks->status) {
     copy_wait<0>();
     return;
@@ -260,13 +264,12 @@ __global__ void __launch_bounds__(T, 1)
       double* row = slots + (size_t)j * G;
       if (lane == 0) {
         double s = (warpSum[0] + warpSum[1]) + (warpSum[2] + warpSum[3]);
-        if (__double_as_longlong(s) == -1LL) s = __longlong_as_double(0x7fffffffffffffffLL);
+        if (is_no_sum(s)) s = __longlong_as_double(0x7fffffffffffffffLL);
         asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(row + blockIdx.x), "d"(s) : "memory");
       }
       // every slot of the step, all loads of a poll in flight together
       double v[5];
       int it = 0;
-      bool stop = false;
       if (G > PAUSE_BLOCKS) __nanosleep(PAUSE_FIRST);
       while (true) {
 #pragma unroll
@@ -278,14 +281,12 @@ __global__ void __launch_bounds__(T, 1)
         }
         bool ready = true;
 #pragma unroll
-        for (int k = 0; k < 5; ++k) ready = ready && __double_as_longlong(v[k]) != -1LL;
+        for (int k = 0; k < 5; ++k) ready = ready && !is_no_sum(v[k]);
         if (__all_sync(0xffffffffu, ready)) break;
-        ++it;
-        stop = it > spin_limit;
-        if (stop && lane == 0) atomicOr(&ks->status, 8);
-        if ((it & 63) == 0) stop = stop || (ld_relaxed_int(&ks->status) & 8);
-        stop = __any_sync(0xffffffffu, stop);
-        if (stop) break;
+        if ((++it & 63) == 0) {
+          if (it > spin_limit && lane == 0) atomicOr(&ks->status, 8);
+          if (__any_sync(0xffffffffu, it > spin_limit || (ld_relaxed_int(&ks->status) & 8))) break;
+        }
         if (G > PAUSE_BLOCKS) __nanosleep(PAUSE_NEXT);
       }
 #pragma unroll
@@ -299,8 +300,7 @@ __global__ void __launch_bounds__(T, 1)
       for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
       if (lane == 0) {
         result = s;
-        gaveUp = stop;
-        if (blockIdx.x == 0 && !stop) {
+        if (blockIdx.x == 0) {
           if (j <= dir)
             ks->H[j * m + dir] = s;
           else if (dir >= 0)
@@ -309,10 +309,6 @@ __global__ void __launch_bounds__(T, 1)
       }
     }
     __syncthreads();
-    if (gaveUp) {
-      copy_wait<0>();
-      return;
-    }
     total = result;
     h = TV(total);
   }
