@@ -544,6 +544,7 @@ __global__ void __launch_bounds__(128) k_cellres(DevMesh m, CellResParams D, con
   if (c >= m.N) return;
   const int N = m.N, F = m.F, B = m.B;
   double dv[5] = {0, 0, 0, 0, 0};
+  double vt[4] = {0, 0, 0, 0};  // the viscous face terms' sums, apart: they may be a 1e-5th of the pressure forces
   double rmax = 0.0;
   const int e0 = m.cptr[c], e1 = m.cptr[c + 1];
   for (int e = e0; e < e1; ++e) {
@@ -554,7 +555,7 @@ __global__ void __launch_bounds__(128) k_cellres(DevMesh m, CellResParams D, con
     for (int k = 0; k < 5; ++k) v[k] = fflux[k * FB + f];
     if (fvisc)
 #pragma unroll
-      for (int k = 0; k < 4; ++k) v[1 + k] -= fvisc[k * FB + f];
+      for (int k = 0; k < 4; ++k) vt[k] += flip(fvisc[k * FB + f], code < 0);
 #pragma unroll
     for (int k = 0; k < 5; ++k) dv[k] += flip(v[k], code < 0);
     rmax = pmax(rmax, m.nodc[f] * flam[f]);
@@ -566,7 +567,7 @@ __global__ void __launch_bounds__(128) k_cellres(DevMesh m, CellResParams D, con
     for (int k = 0; k < 5; ++k) dv[k] += fflux[k * FB + F + b];
     if (fvisc)
 #pragma unroll
-      for (int k = 0; k < 4; ++k) dv[1 + k] -= fvisc[k * FB + F + b];
+      for (int k = 0; k < 4; ++k) vt[k] += fvisc[k * FB + F + b];
     if (m.bpartner && m.bpartner[b] >= 0) {
       // coupled face: nonOrthDeltaCoeffs lambda as for an internal face (setCoAndDeltaT.H:73-87)
       rmax = pmax(rmax, m.bnodc[b] * flam[F + b]);
@@ -585,6 +586,9 @@ __global__ void __launch_bounds__(128) k_cellres(DevMesh m, CellResParams D, con
   double r[5];
 #pragma unroll
   for (int k = 0; k < 5; ++k) r[k] = -dv[k];
+  if (fvisc)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) r[1 + k] += vt[k];
   l2cell[c] = dv[0] * dv[0];
   const double rpOld = rPDT[c];
   if (D.ddt != ICS_DDT_STEADY) {
@@ -845,17 +849,20 @@ __global__ void __launch_bounds__(128) k_src_tangent(DevMesh m, double dgPhys, c
 #pragma unroll
   for (int k = 0; k < 5; ++k) r[k] = -dv[k];
   if (fvisc) {
+    double vt[4] = {0, 0, 0, 0};
     for (int e = m.cptr[c]; e < m.cptr[c + 1]; ++e) {
       const int code = m.cface[e];
       const int f = code >= 0 ? code : ~code;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) r[1 + k] += flip(fvisc[k * FB + f].d, code < 0);
+      for (int k = 0; k < 4; ++k) vt[k] += flip(fvisc[k * FB + f].d, code < 0);
     }
     for (int e = m.bptr[c]; e < m.bptr[c + 1]; ++e) {
       const int b = m.bface[e];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) r[1 + k] += fvisc[k * FB + m.F + b].d;
+      for (int k = 0; k < 4; ++k) vt[k] += fvisc[k * FB + m.F + b].d;
     }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) r[1 + k] += vt[k];
   }
   const double Vc = m.V[c];
 #pragma unroll
