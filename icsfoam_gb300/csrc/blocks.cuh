@@ -151,6 +151,30 @@ struct SlotBlock<float> {
   };
 };
 
+// acc += B x (SIGN 1) or acc -= B x (SIGN -1) over the slots of a row.  FP64: the
+// products of two slots are summed in part (five zeros before the first slot)
+// and meet the row's sum together (flush, at every second slot and the last
+// one).  Accumulating them into acc term by term saves one operation of eleven
+// (a solve of 197k cells 7.7 against 8.3 ms), but rounds each of the 30 products
+// at the size of the row's diagonal part.  Error of the increments of three
+// cycles against the same solve in 80 bits: 5.0e-17 of the largest, 7.8e-17 term
+// by term, 5.3e-17 with a sum per slot (12 operations).
+template <int SIGN, typename TB, typename TV>
+__device__ __forceinline__ void add_slot(const SlotBlock<TB>& B, TV g, const TV* x, TV* acc, TV* part, bool flush) {
+  if constexpr (sizeof(TB) == 4) {
+    B.template mac<SIGN>(g, x, acc);
+  } else {
+    B.template mac<SIGN>(g, x, part);
+    if (flush) {
+#pragma unroll
+      for (int i = 0; i < 5; ++i) {
+        acc[i] += part[i];
+        part[i] = TV(0);
+      }
+    }
+  }
+}
+
 // y -= SIGN V x, V = the non-LF viscous laplacians at column cell col of slot
 // (only when m.vjslot is set; TB is the block storage type)
 template <typename TB, int SIGN = 1, typename TV>

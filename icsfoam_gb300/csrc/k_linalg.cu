@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(128) k_spmv(DevMesh m, const TB* __restrict__ 
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.N) return;
   const int s = c >> 5, lane = c & 31;
-  TV xc[5], acc[5];
+  TV xc[5], acc[5], part[5] = {0, 0, 0, 0, 0};
 #pragma unroll
   for (int k = 0; k < 5; ++k) xc[k] = x[5 * c + k];
   const TB* D = dg + (size_t)s * 25 * 32 + lane;
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(128) k_spmv(DevMesh m, const TB* __restrict__ 
     for (int k = 0; k < 5; ++k) xj[k] = x[5 * col + k];
     SlotBlock<TB> Bk;
     Bk.load(blk, base + t, lane);
-    Bk.template mac<1>(g, xj, acc);
+    add_slot<1>(Bk, g, xj, acc, part, (t & 1) || t == ns - 1);
     if (m.vjslot) vj_sub<TB>(m, base + t, lane, col, xj, acc);
   }
   if (m.nInst > 1 && hb_in_zone(m, c)) {
@@ -166,9 +166,9 @@ __global__ void __launch_bounds__(128) k_cyc_mv(DevMesh m, const TB* __restrict_
 //   pass 3 (level-0 rows): the reverse sweep, as k_lusgs_level MODE 1.
 // Same arithmetic as the separate kernels up to the order of the sums.  In
 // FP64 these passes are bound by the FP64 pipe, so their cost is their count
-// of operations: one product per slot in pass 2 (98k rows: 94 -> 45 us) and
-// products accumulated by multiply-adds (pass 1 52 -> 37, pass 3 45 -> 39 us);
-// the FP32 passes are bound by HBM and did not change.
+// of operations: one product per slot in pass 2 (98k rows: 94 -> 49 us) and
+// products accumulated by multiply-adds over two slots (add_slot; pass 1 52 ->
+// 40, pass 3 45 -> 43 us); the FP32 passes are bound by HBM and did not change.
 template <typename TB, typename TV, int MINB = 1, int UNR = 1>
 __global__ void __launch_bounds__(128, MINB) k_op_level0(DevMesh m, const TB* __restrict__ blk, const TB* __restrict__ dg,
                                                    const TV* __restrict__ x, TV* __restrict__ w,
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(128, MINB) k_op_level0(DevMesh m, const TB* __
   if (i >= count) return;
   const int c = cells ? cells[start + i] : start + i;
   const int s = c >> 5, lane = c & 31;
-  TV xc[5], acc[5];
+  TV xc[5], acc[5], part[5] = {0, 0, 0, 0, 0};
 #pragma unroll
   for (int k = 0; k < 5; ++k) xc[k] = x[5 * (size_t)c + k];
   const TB* D = dg + (size_t)s * 25 * 32 + lane;
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(128, MINB) k_op_level0(DevMesh m, const TB* __
       for (int k = 0; k < 5; ++k) xn[k] = x[5 * (size_t)colA + k];
     SlotBlock<TB> Bk;
     Bk.load(blk, base + t, lane);
-    Bk.template mac<1>(g, xj, acc);
+    add_slot<1>(Bk, g, xj, acc, part, (t & 1) || t == ns - 1);
     if (m.vjslot) vj_sub<TB>(m, base + t, lane, col, xj, acc);
   }
   if (m.nInst > 1 && hb_in_zone(m, c)) {
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(128, MINB) k_op_level1(DevMesh m, const TB* __
   if (i >= count) return;
   const int c = cells ? cells[start + i] : start + i;
   const int s = c >> 5, lane = c & 31;
-  TV xc[5], acc[5];
+  TV xc[5], acc[5], part[5] = {0, 0, 0, 0, 0};
 #pragma unroll
   for (int k = 0; k < 5; ++k) xc[k] = x[5 * (size_t)c + k];
   const TB* D = dg + (size_t)s * 25 * 32 + lane;
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(128, MINB) k_op_level1(DevMesh m, const TB* __
     for (int k = 0; k < 5; ++k) xj[k] = x[5 * (size_t)col + k] - rj * w[5 * col + k];
     SlotBlock<TB> Bk;
     Bk.load(blk, base + t, lane);
-    Bk.template mac<1>(g, xj, acc);
+    add_slot<1>(Bk, g, xj, acc, part, (t & 1) || t == ns - 1);
     if (m.vjslot) vj_sub<TB>(m, base + t, lane, col, xj, acc);
   }
   if (m.nInst > 1 && hb_in_zone(m, c)) {
@@ -291,7 +291,7 @@ __device__ __forceinline__ void lusgs_fwd_row(const DevMesh& m, const TB* __rest
   const int s = c >> 5, lane = c & 31;
   const int base = m.slot_base[s];
   const int nl = m.nlow[c];
-  TV acc[5];
+  TV acc[5], part[5] = {0, 0, 0, 0, 0};
 #pragma unroll
   for (int k = 0; k < 5; ++k) acc[k] = r[5 * c + k];
   const TV g = TV(m.gamma);
@@ -304,7 +304,7 @@ __device__ __forceinline__ void lusgs_fwd_row(const DevMesh& m, const TB* __rest
     for (int k = 0; k < 5; ++k) dj[k] = rj * r[5 * col + k];
     SlotBlock<TB> Bk;
     Bk.load(blk, base + t, lane);
-    Bk.template mac<-1>(g, dj, acc);
+    add_slot<-1>(Bk, g, dj, acc, part, (t & 1) || t == nl - 1);
     if (m.vjslot) vj_sub<TB, -1>(m, base + t, lane, col, dj, acc);
   }
   if (SCALE) {
@@ -323,23 +323,33 @@ __device__ __forceinline__ void lusgs_rev_row(const DevMesh& m, const TB* __rest
   const int s = c >> 5, lane = c & 31;
   const int base = m.slot_base[s];
   const int nl = m.nlow[c], ns = m.nslot[c];
-  TV acc[5];
+  TV acc[5], part[5] = {0, 0, 0, 0, 0};
 #pragma unroll
   for (int k = 0; k < 5; ++k) acc[k] = r[5 * c + k];
   // two slots in flight: their column loads and the dependent gathers overlap
   // (2% on the reverse sweep; a deeper software pipeline with the next slot's
   // column and deltas loaded ahead measured 11% slower)
   const TV g = TV(m.gamma);
-#pragma unroll 2
-  for (int t = ns - 1; t >= nl; --t) {
+  auto slot = [&](int t, bool flush) {
     const int col = m.scol[(base + t) * 32 + lane];
     TV dj[5];
 #pragma unroll
     for (int k = 0; k < 5; ++k) dj[k] = r[5 * col + k];
     SlotBlock<TB> Bk;
     Bk.load(blk, base + t, lane);
-    Bk.template mac<-1>(g, dj, acc);
+    add_slot<-1>(Bk, g, dj, acc, part, flush);
     if (m.vjslot) vj_sub<TB, -1>(m, base + t, lane, col, dj, acc);
+  };
+  if constexpr (sizeof(TB) == 8) {
+    int t = ns - 1;
+    for (; t > nl; t -= 2) {  // flushed at compile time: an addition costs its cycles where predicated off too
+      slot(t, false);
+      slot(t - 1, true);
+    }
+    if (t == nl) slot(t, true);
+  } else {
+#pragma unroll 2
+    for (int t = ns - 1; t >= nl; --t) slot(t, false);
   }
   const TV rc = TV(rD[c]);
 #pragma unroll
@@ -358,7 +368,8 @@ __device__ __forceinline__ void lusgs_rev_row2(const DevMesh& m, const TB* __res
   const int b0 = m.slot_base[c0 >> 5], b1 = m.slot_base[c1 >> 5];
   const int nl0 = m.nlow[c0], nl1 = m.nlow[c1];
   int t0 = m.nslot[c0] - 1, t1 = m.nslot[c1] - 1;
-  TV a0[5], a1[5];
+  TV a0[5], a1[5], p0[5] = {0, 0, 0, 0, 0}, p1[5] = {0, 0, 0, 0, 0};
+  bool odd = false;  // every second slot of the two rows
 #pragma unroll
   for (int k = 0; k < 5; ++k) {
     a0[k] = r[5 * c0 + k];
@@ -366,7 +377,7 @@ __device__ __forceinline__ void lusgs_rev_row2(const DevMesh& m, const TB* __res
   }
   const TV g = TV(m.gamma);
 #pragma unroll 1
-  for (; t0 >= nl0 || t1 >= nl1; --t0, --t1) {
+  for (; t0 >= nl0 || t1 >= nl1; --t0, --t1, odd = !odd) {
     const bool v0 = t0 >= nl0, v1 = t1 >= nl1;
     const int col0 = v0 ? m.scol[(b0 + t0) * 32 + l0] : c0;
     const int col1 = v1 ? m.scol[(b1 + t1) * 32 + l1] : c1;
@@ -380,11 +391,11 @@ __device__ __forceinline__ void lusgs_rev_row2(const DevMesh& m, const TB* __res
     if (v0) B0.load(blk, b0 + t0, l0);
     if (v1) B1.load(blk, b1 + t1, l1);
     if (v0) {
-      B0.template mac<-1>(g, d0, a0);
+      add_slot<-1>(B0, g, d0, a0, p0, odd || t0 == nl0);
       if (m.vjslot) vj_sub<TB, -1>(m, b0 + t0, l0, col0, d0, a0);
     }
     if (v1) {
-      B1.template mac<-1>(g, d1, a1);
+      add_slot<-1>(B1, g, d1, a1, p1, odd || t1 == nl1);
       if (m.vjslot) vj_sub<TB, -1>(m, b1 + t1, l1, col1, d1, a1);
     }
   }
@@ -431,15 +442,15 @@ __global__ void __launch_bounds__(128) k_lusgs_level(DevMesh m, const TB* __rest
 
 // ------------------------------------------------- FP64 rows on five lanes
 // The FP64 products of few rows.  A warp's FP64 instruction holds its scheduler
-// for 64 cycles, so a row per thread costs a warp 175 x 64 cycles for a product
+// for 64 cycles, so a row per thread costs a warp 190 x 64 cycles for a product
 // with six neighbours however few warps there are, while most of the 608
 // schedulers idle.  Here five lanes share a row, one component each, six rows
-// to a warp: 35 instructions per warp, in the same order per component.
+// to a warp: 38 instructions per warp, in the same order per component.
 // A row costs 7% more of the pipe in all, so the row-per-thread kernels stay for
 // many rows.  By events around a launch (5 us of them), a row per thread against
-// five lanes, product / second level / reverse: 5k rows 12.7 : 9.8 / 15.3 : 10.5
-// / 14.8 : 10.3 us, 23.5k 18.3 : 13.7 / 20.6 : 15.8 / 18.5 : 13.8, 32k 18.9 :
-// 17.1 / 22.2 : 20.2 / 20.3 : 16.7; from 39k rows (two full warps per scheduler)
+// five lanes, product / second level / reverse: 5k rows 13.6 : 10.1 / 16.3 : 10.6
+// / 16.3 : 10.5 us, 23.3k 19.0 : 14.9 / 21.4 : 16.7 / 20.8 : 14.9, 31.7k 20.2 :
+// 18.9 / 23.4 : 22.6 / 22.3 : 19.2; from 39k rows (two full warps per scheduler)
 // on neither way is ahead at every size, within 5% on average.
 // ROWS_PRODUCT: w = A x (k_spmv, k_op_level0); ROWS_LEVEL1: k_op_level1;
 // ROWS_REVERSE: the reverse sweep of a level, w in place (k_lusgs_level MODE 1).
@@ -459,7 +470,7 @@ __global__ void __launch_bounds__(ROWS5_THREADS) k_rows5(DevMesh m, const double
   const int c = on ? (cells ? cells[start + row] : start + row) : 0;
   const int lane = c & 31, base = m.slot_base[c >> 5];
   const int first = MODE == ROWS_REVERSE && on ? m.nlow[c] : 0, ns = on ? m.nslot[c] : 0;
-  double acc = 0.0;
+  double acc = 0.0, part = 0.0;
   if (MODE == ROWS_REVERSE) {
     if (on) acc = w[5 * (size_t)c + i];
   } else if (on) {
@@ -494,7 +505,7 @@ __global__ void __launch_bounds__(ROWS5_THREADS) k_rows5(DevMesh m, const double
 #pragma unroll
       for (int j = 0; j < 5; ++j) {
         if (MODE == ROWS_REVERSE) xj[j] = -xj[j];
-        acc += B[j] * xj[j];
+        part += B[j] * xj[j];
       }
       if (m.vjslot) {
         double y[5] = {0, 0, 0, 0, 0};
@@ -503,6 +514,10 @@ __global__ void __launch_bounds__(ROWS5_THREADS) k_rows5(DevMesh m, const double
         for (int j = 0; j < 5; ++j)
           if (j == i) acc += y[j];
       }
+    }
+    if ((q & 1) || q == trips - 1) {  // as add_slot
+      acc += part;
+      part = 0.0;
     }
   }
   if (!on) return;
@@ -1289,17 +1304,17 @@ __global__ void __launch_bounds__(128) k_jacobi_sweep(DevMesh m, const TB* __res
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.N) return;
   const int s = c >> 5, lane = c & 31;
-  TV acc[5] = {TV(0), TV(0), TV(0), TV(0), TV(0)};
-  const int base = m.slot_base[s];
+  TV acc[5] = {TV(0), TV(0), TV(0), TV(0), TV(0)}, part[5] = {0, 0, 0, 0, 0};
+  const int base = m.slot_base[s], ns = m.nslot[c];
   const TV g = TV(m.gamma);
-  for (int t = 0; t < m.nslot[c]; ++t) {
+  for (int t = 0; t < ns; ++t) {
     const int col = m.scol[(base + t) * 32 + lane];
     TV xj[5];
 #pragma unroll
     for (int k = 0; k < 5; ++k) xj[k] = xo[5 * col + k];
     SlotBlock<TB> Bk;
     Bk.load(blk, base + t, lane);
-    Bk.template mac<1>(g, xj, acc);
+    add_slot<1>(Bk, g, xj, acc, part, (t & 1) || t == ns - 1);
     if (m.vjslot) vj_sub<TB>(m, base + t, lane, col, xj, acc);
   }
   TV r[5];
