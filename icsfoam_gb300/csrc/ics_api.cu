@@ -1758,7 +1758,7 @@ int ics_autotune(ics_handle hh, ics_tuning* out) {
       autotune_linalg(h, log);
       t.face_block = h.tuneFaceBs;
       t.grad_block = h.tuneGradBs;
-      t.mgs_blocks = h.tuneMgsBlocks;
+      t.mgs_blocks = 608;  // no effect (ics_tuning)
       t.fused_operator = h.tuneFused;
       t.reverse_rows = h.tuneRevRows;
       std::lock_guard<std::mutex> lock(g_tune_mu);
@@ -1766,7 +1766,6 @@ int ics_autotune(ics_handle hh, ics_tuning* out) {
     }
     h.tuneFaceBs = t.face_block;
     h.tuneGradBs = t.grad_block;
-    h.tuneMgsBlocks = t.mgs_blocks;
     h.tuneFused = t.fused_operator;
     h.tuneRevRows = t.reverse_rows;
     drop_graphs(h);  // the captured cycle holds the old launch shapes
@@ -1792,7 +1791,6 @@ int ics_set_tuning(ics_handle hh, const ics_tuning* t) {
     }
     h.tuneFaceBs = t->face_block;
     h.tuneGradBs = t->grad_block;
-    h.tuneMgsBlocks = t->mgs_blocks;
     h.tuneFused = t->fused_operator;
     h.tuneRevRows = t->reverse_rows;
     drop_graphs(h);

@@ -1015,6 +1015,18 @@ static void rev_level(Handle& h, const TB* blk, const TB* rD, TV* r, const int* 
                                        h.m, blk, rD, r, cells, start, cnt));
 }
 
+// whether some reverse level runs the kernels that Handle::tuneRevRows chooses
+// between: not with the sync-free sweeps, the chain scan or another
+// preconditioner, nor where every level's rows are on five lanes each
+template <typename TB>
+static bool rev_rows_choice(const Handle& h) {
+  const DevMesh& m = h.m;
+  if (m.sw_fwd || h.cfg.c.preconditioner != ICS_PC_LUSGS) return false;
+  for (int l = m.fuse_last ? 1 : 0; l < m.nrl; ++l)
+    if (sizeof(TB) == 4 || m.rl_ptr[l + 1] - m.rl_ptr[l] > ROWS5_LIMIT) return true;
+  return false;
+}
+
 // Resident warps of a sync-free sweep: a few levels' worth, so that the loads
 // of the next levels' rows are in flight while a level is polled, and no more
 // pollers than that.  Measured on a 227k-cell RCM box (181 levels): two rows
@@ -1525,7 +1537,15 @@ static void autotune_linalg_t(Handle& h, std::vector<std::pair<std::string, doub
     log.emplace_back("operator_spmv_then_lusgs", split);
     h.tuneFused = fused <= split ? 1 : 0;
   }
-  // rows per thread of the reverse level sweeps, timed on the whole LU-SGS
+  // rows per thread of the reverse level sweeps, timed on the whole LU-SGS,
+  // where a level takes the kernels they choose between
+  h.tuneRevRows = 1;
+  if (!rev_rows_choice<TB>(h)) {
+    ICS_CUDA(cudaEventDestroy(e0));
+    ICS_CUDA(cudaEventDestroy(e1));
+    ICS_CUDA(cudaGetLastError());
+    return;
+  }
   double revMs[3] = {0, 0, 0};
   for (int rows : {1, 2}) {
     h.tuneRevRows = rows;

@@ -508,7 +508,8 @@ typedef struct {
   int32_t from_cache;      /* 1: taken from an earlier tuning of a case of the same shape */
   int32_t reverse_rows;    /* rows per thread of the reverse LU-SGS level sweep (1 / 2:
                               two rows' slot loads in flight together); no effect on an
-                              FP64 level of up to 36000 rows                             */
+                              FP64 level of up to 36000 rows or on a mesh of more than
+                              two levels, where the autotuner leaves it at 1             */
 } ics_tuning;
 /* Time each candidate launch choice on the handle's current state and
  * assembled Jacobian (CUDA events on its stream) and keep the fastest, for
