@@ -377,7 +377,9 @@ __global__ void __launch_bounds__(T, 1)
   if (dir + 1 < m) {
     const double beta = sqrt(total);
     if (dir < 0 && blockIdx.x == 0 && tid == 0) dev_beta0(ks, beta, m);
-    if (!(beta > 0.0)) return;
+    // a zero start of a cycle is a breakdown (dev_beta0); a zero vector later on
+    // is divided by its norm all the same, and the solve ends as not finite
+    if (dir < 0 && !(beta > 0.0)) return;
     const TV b = TV(beta), rb = TV(1) / b, rl = rb * fma(-b, rb, TV(1));
     VT* out = reinterpret_cast<VT*>(V + (size_t)(dir + 1) * vs);
 #pragma unroll
