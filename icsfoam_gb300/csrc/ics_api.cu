@@ -202,6 +202,9 @@ void ensure_workspace(Handle& h) {
   const int m = h.cfg.c.n_directions;
   const size_t eb = p == ICS_PREC_MIXED ? 4 : 8;
   const size_t n5 = 5ull * h.m.N;
+  // the basis also holds the scalar transport's FP64 vectors, which are longer
+  // than FP32 vectors of five equations on up to 12 cells
+  const size_t basis = std::max(kstride(h) * eb, ((size_t)h.m.N + 63) / 64 * 64 * sizeof(double));
   if (h.kvPrec != p || h.kvDirs < m) drop_graphs(h);  // captured pointers change
   if (h.kvPrec != p) {
     void* ptrs[] = {h.blk, h.dg, h.dginv, h.rD, h.kw, h.kx, h.kb, h.kt, h.kv};
@@ -215,13 +218,13 @@ void ensure_workspace(Handle& h) {
     h.kx = dalloc<char>(h, n5 * eb);
     h.kb = dalloc<char>(h, n5 * eb);
     h.kt = dalloc<char>(h, n5 * eb);
-    h.kv = dalloc<char>(h, kstride(h) * eb * m);
+    h.kv = dalloc<char>(h, basis * m);
     h.kvDirs = m;
     h.kvPrec = p;
     h.haveMatrix = false;
   } else if (h.kvDirs < m) {
     dfree(h.kv);
-    h.kv = dalloc<char>(h, kstride(h) * eb * m);
+    h.kv = dalloc<char>(h, basis * m);
     h.kvDirs = m;
   }
 }
