@@ -61,3 +61,49 @@ def test_products_and_sweeps_round_as_plain_sums(gpu_binding, shape):
         scale = np.sqrt((e ** 2).mean(axis=0))
         rms = [np.sqrt((((np.asarray(a, np.longdouble) - e) / scale) ** 2).mean()) for a in (device(v), plain[k](v))]
         assert rms[0] <= 1.1 * rms[1], rms
+
+
+def _cell_by_cell(m, J, dtype):
+    """Both sweeps row after row, in the order of the cells."""
+    diag, low, up = (np.asarray(a, dtype) for a in J)
+    rD = (1.0 / np.abs(np.einsum("nii->ni", J[0])).max(axis=1)).astype(dtype)
+    below, above = [[] for _ in range(m.n_cells)], [[] for _ in range(m.n_cells)]
+    for f, (o, n) in enumerate(zip(m.owner, m.neighbour)):
+        above[o].append((n, up[f]))
+        below[n].append((o, low[f]))
+
+    def sweeps(r):
+        x = r.copy()
+        for c in range(m.n_cells):
+            for j, B in below[c]:
+                x[c] = x[c] - (B * (rD[j] * x[j])).sum(axis=1)
+        for c in reversed(range(m.n_cells)):
+            for j, B in above[c]:
+                x[c] = x[c] - (B * x[j]).sum(axis=1)
+            x[c] = rD[c] * x[c]
+        return x
+
+    return sweeps
+
+
+# the scan of a chain of many levels and the sync-free sweeps; 1.2: a few
+# thousand rounding errors, correlated along the levels
+@pytest.mark.parametrize("shape", ["chain_129", "chain_1000", "levels"])
+def test_sweeps_of_many_levels_round_as_plain_ones(gpu_binding, shape):
+    w = {"chain_129": lambda: cases.shock_tube(129), "chain_1000": lambda: cases.shock_tube(1000),
+         "levels": lambda: cases.bump_channel(19, 9, 7, ordering_mode="natural")}[shape]()
+    w = perturb(w)
+    h = abi.CaseHandle(gpu_binding, w.mesh, cases.make_config(gpu_binding, w.settings))
+    h.set_primitive(w.p, w.U, w.T)
+    h.begin_time_step()
+    h.residual()
+    h.assemble_jacobian()
+    J = h.get_jacobian()
+    errors = np.zeros(2)
+    for seed in range(4):
+        r = np.random.default_rng(seed).standard_normal((w.mesh.n_cells, 5)) * np.abs(h.get_state()["W"]).max(axis=0)
+        e = _cell_by_cell(w.mesh, J, np.longdouble)(r.astype(np.longdouble))
+        scale = np.maximum(np.sqrt((e ** 2).mean(axis=0)), 1e-300)
+        for k, a in enumerate((h.precondition(r), _cell_by_cell(w.mesh, J, np.float64)(r))):
+            errors[k] += float((((np.asarray(a, np.longdouble) - e) / scale) ** 2).mean())
+    assert np.sqrt(errors[0]) <= 1.2 * np.sqrt(errors[1]), np.sqrt(errors)
