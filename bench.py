@@ -217,7 +217,7 @@ def kernel_bound(kind, mixed):
 # HLLC + MUSCL / cellLimited<Venkatakrishnan>: counted by ncu from the
 # executed DFMA (2 flops), DADD and DMUL instructions of one launch
 # (profiles/fp64_residual_bump_125x63x61.md), divided by the faces / cells
-FP64_FLOPS_PER_UNIT = {"face": 297.0, "grad": 876.1}
+FP64_FLOPS_PER_UNIT = {"face": 313.0, "grad": 907.4}
 
 
 def load_peaks():

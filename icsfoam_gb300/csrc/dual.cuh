@@ -119,8 +119,10 @@ __device__ __forceinline__ long long mag(const Dual& x) { return mag(x.v); }
 // -x without the FP64 pipe
 __device__ __forceinline__ double neg(double x) { return flip(x, true); }
 __device__ __forceinline__ Dual neg(const Dual& x) { return -x; }
-// x / b from the reciprocal r = fl(1/b): the product's remainder corrects it
-// to the rounding of a division, in 3 operations of the FP64 pipe against 10
+// x / b from the reciprocal r = fl(1/b) by Markstein's correction: the product's
+// remainder corrects it to the rounding of a division, in 3 operations of the
+// FP64 pipe against 10 (NaN where x is infinite or b zero, like the expressions
+// that use it)
 __device__ __forceinline__ double quot(double x, double b, double r) {
   const double q = x * r;
   return fma(fma(-q, b, x), r, q);

@@ -487,8 +487,8 @@ void build_mesh(Handle& h, const ics_mesh_desc* d) {
   m.fl_lptr = upload(h, m.fl_ptr);
   // the sync-free sweeps: every schedule of more than two levels.  Measured
   // against one CTA that walks the levels (us per forward sweep, FP64 / FP32):
-  // 12^3 RCM box 48 / 47 against 176 / 58, 24^3 97 / 96 against 556 / 131,
-  // 61^3 276 / 268 against 7069 / 1010.
+  // 12^3 RCM box 48 / 28 against 176 / 58, 24^3 97 / 57 against 556 / 131,
+  // 61^3 276 / 154 against 7069 / 1010.
   if (m.nfl > 2) {
     m.sweep_pad = dalloc<double>(h, 16ull * N);
     const std::vector<int> sf = ticket_order(fcells, m.fl_ptr), sr = ticket_order(rcells, m.rl_ptr);

@@ -11,11 +11,12 @@
 // matrix, the Givens rotations, the back substitution, the stop test
 // (coupledMatrixSolver.C:198-221) and the norm factors (gmres.C:812-850).
 // Here each of those is per case:
-//   * every reduction runs over segments of at most SEG_CELLS cells that
-//     never straddle two cases; the last segment of a case to finish folds
-//     the case's partial sums in segment order (a per-case last-block-done
-//     tree), so a case's sums depend only on its own cells and sizes, not on
-//     the other cases in the stack;
+//   * the Gram-Schmidt of a case of up to COLUMN_CELLS cells runs in a cluster
+//     of blocks of its own (k_ccolumn); every other reduction runs over
+//     segments of at most SEG_CELLS cells that never straddle two cases, and
+//     the last segment of a case to finish folds the case's partial sums in
+//     segment order.  Either way a case's sums depend only on its own cells
+//     and sizes, not on the other cases in the stack;
 //   * the Krylov scalars (H, c, s, bh, y, beta) live per case in device
 //     memory and the per-case kernels read them there, so one restart cycle
 //     is one launch sequence for all cases, captured once as a CUDA graph;

@@ -10,10 +10,13 @@
 //   jacobi    z = D^-1 r with precomputed 5x5 inverses (Jacobi.C:55-135)
 //   gmres     left-preconditioned restarted GMRES with modified Gram-Schmidt
 //             and Givens rotations (gmres.C:772-1107).  All vectors and the
-//             Hessenberg matrix stay on the device; dot products use a fixed
-//             grid and a last-block-done tree, so results are reproducible
-//             run to run.  One host synchronisation per restart cycle reads
-//             the L1 residuals for the stop test (coupledMatrixSolver.C:198-221).
+//             Hessenberg matrix stay on the device.  The Gram-Schmidt sums are
+//             exchanged through slots and added in slot order (k_column.cu),
+//             the norms and residuals by a grid of the size's choosing whose
+//             last block folds the partial sums in block order, so results are
+//             reproducible run to run.  One host synchronisation per restart
+//             cycle reads the L1 residuals for the stop test
+//             (coupledMatrixSolver.C:198-221).
 #include <algorithm>
 #include <cmath>
 
@@ -615,7 +618,7 @@ __device__ __forceinline__ bool sweep_ready(const TV* v) {
 // FP64 rows, 16 lanes each (two rows per warp): lane (p, i) = (lane / 5, lane
 // % 5) of a row handles component i of its p-th neighbour of three, so the
 // three neighbours are polled, scaled and multiplied at once.  GB300 issues a
-// warp's FP64 instruction over about 70 cycles of its scheduler whatever
+// warp's FP64 instruction over 64 cycles of its scheduler whatever
 // lanes are active, so a row costs its count of instructions: 10 here against
 // 105 with one row per lane.  The sums keep the order of lusgs_fwd_row /
 // lusgs_rev_row.

@@ -120,8 +120,9 @@ __global__ void __launch_bounds__(128) k_gauss_coefficients(DevMesh m) {
 // limiter's bounds want anyway, and three multiply-adds per field and face, where
 // interpolating to the face first takes five operations and the division by V
 // comes on top.  FP64 operations bound the kernel (656 a cell with six faces,
-// eight fields and Venkatakrishnan's limiter, 736 before: 708 -> 633 us on
-// 480k cells).  mask selects the fields, limited
+// eight fields and Venkatakrishnan's limiter with the compiler's contraction, 736
+// with face values: 708 -> 633 us on 480k cells; 610 with the roundings written
+// out, 591 us).  mask selects the fields, limited
 // selects cellLimited (1 = minmod, 2 = Venkatakrishnan).
 template <int LIMITED, typename Real = double>
 __global__ void __launch_bounds__(128) k_grad(DevMesh m, const Real* __restrict__ q, const double* __restrict__ bq,
@@ -582,7 +583,7 @@ __global__ void __launch_bounds__(128) k_cellres(DevMesh m, CellResParams D, con
   const double Vc = m.V[c];
   // R V directly: the divergences' division by V and the source's product with
   // it cancel (and every division saved is ten operations of the FP64 pipe
-  // that bounds this kernel: 166 -> 93 us on 480k cells, 90 operations a cell)
+  // that bounds this kernel: 166 -> 79 us on 480k cells, 66 operations a cell)
   double r[5];
 #pragma unroll
   for (int k = 0; k < 5; ++k) r[k] = -dv[k];

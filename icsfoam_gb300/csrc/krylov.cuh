@@ -72,7 +72,8 @@ __device__ __forceinline__ TD convert(double x) {
     return x;
 }
 
-// x / b from the reciprocal r = fl(1/b) and its error term rl = r (1 - b r):
+// x / b from the reciprocal r = fl(1/b) and its error term rl = r (1 - b r), after
+// Markstein:
 // two operations, within a half unit and 2^-50 of the quotient
 template <typename TV>
 __device__ __forceinline__ TV quotient(TV x, TV r, TV rl) {
